@@ -193,6 +193,16 @@ __host__ __device__ constexpr int ep_thread_bound(int kind) {
 // method evaluates every term (its FP32 exp is cheap and flushes far below).
 constexpr float kRadialCut = 46.0f;
 
+// ar = alpha r^2 above the cut, and x == 0, on the bit patterns for FP64 (an
+// FP64 comparison issues on the FP64 pipe; a NaN is neither)
+__device__ __forceinline__ bool above_cut(float ar) { return ar > kRadialCut; }
+__device__ __forceinline__ bool above_cut(double ar) {
+  return (unsigned)__double2hiint(ar) - 0x40470000u <= 0x7FF00000u - 0x40470000u;  // [46, inf]
+}
+__device__ __forceinline__ bool is_zero(double x) {
+  return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u;
+}
+
 template <typename R, bool DERIV, int NC, bool CUT = false>
 __device__ __forceinline__ void group_radial(const Tables<R>& t, int g, R r2, R (&G0)[NC],
                                              R (&G1)[NC], R (&G2)[NC]) {
@@ -202,9 +212,9 @@ __device__ __forceinline__ void group_radial(const Tables<R>& t, int g, R r2, R 
   for (int c = 0; c < NC; ++c) G0[c] = G1[c] = G2[c] = (R)0;
   if (!t.group_split[g]) {
     for (int p = 0; p < np; ++p) {
-      const R al = t.alpha[p0 + p];
-      if (CUT && al * r2 > (R)kRadialCut) continue;
-      const R e0 = rexp(-al * r2);
+      const R al = t.alpha[p0 + p], ar = al * r2;
+      if (CUT && above_cut(ar)) continue;
+      const R e0 = rexp(-ar);
       const R e1 = al * e0, e2 = al * e1;
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
@@ -222,9 +232,9 @@ __device__ __forceinline__ void group_radial(const Tables<R>& t, int g, R r2, R 
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         const int wi = wb + c * np + p;
-        const R al = t.walpha[wi];
-        if (CUT && al * r2 > (R)kRadialCut) continue;
-        const R e0 = rexp(-al * r2);
+        const R al = t.walpha[wi], ar = al * r2;
+        if (CUT && above_cut(ar)) continue;
+        const R e0 = rexp(-ar);
         const R w = t.wd[wi];
         G0[c] = fma(w, e0, G0[c]);
         if (DERIV) {
@@ -530,8 +540,8 @@ __device__ inline void ep_electron(const qmc_wf_desc& d, const Tables<R>& t, con
       // evaluate the same electron index of different walkers, so the branch
       // is mostly uniform)
       if constexpr (!kMixed<R>) {
-        if (o.v == (R)0 && (!KIN || (o.gx == (R)0 && o.gy == (R)0 && o.gz == (R)0 &&
-                                     o.lap == (R)0)))
+        if (is_zero(o.v) && (!KIN || (is_zero(o.gx) && is_zero(o.gy) && is_zero(o.gz) &&
+                                      is_zero(o.lap))))
           return;
       }
       R wv[JC];

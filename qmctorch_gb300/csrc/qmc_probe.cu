@@ -23,7 +23,7 @@ __global__ void __launch_bounds__(256) fma_probe(int64_t iters, double* out) {
   out[tid] = (double)s;
 }
 
-template <typename T, bool TANG = false>
+template <typename T, bool FIXED = false>
 __global__ void __launch_bounds__(256) exp_probe(int64_t iters, double* out) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   T a[8];
@@ -34,8 +34,8 @@ __global__ void __launch_bounds__(256) exp_probe(int64_t iters, double* out) {
     for (int k = 0; k < 8; ++k) {
       if constexpr (sizeof(T) == 4)
         a[k] = -__expf(a[k]) * (T)1e-3;
-      else if (TANG)
-        a[k] = -qmc::exp_tang(a[k]) * (T)1e-3;
+      else if (FIXED)
+        a[k] = -qmc::exp_fixed(a[k]) * (T)1e-3;
       else
         a[k] = -exp(a[k]) * (T)1e-3;
     }
@@ -58,15 +58,20 @@ extern "C" int qmc_probe_fma(int32_t kind, int32_t blocks, int64_t iters, double
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
-__global__ void __launch_bounds__(256) exp64_eval(const double* __restrict__ x, int64_t n,
-                                                  double* __restrict__ y) {
+__global__ void __launch_bounds__(256) fixed64_eval(int32_t kind, const double* __restrict__ x,
+                                                    int64_t n, double* __restrict__ y) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) y[i] = qmc::rexp(x[i]);
+  if (i < n) y[i] = kind == 0 ? qmc::rexp(x[i]) : (kind == 1 ? qmc::psqrt(x[i]) : qmc::prcp(x[i]));
+}
+
+extern "C" int qmc_probe_fixed64(int32_t kind, const double* x, int64_t n, double* y,
+                                 void* stream) {
+  if (kind < 0 || kind > 2 || n < 0 || (n > 0 && (!x || !y))) return 1;
+  if (n == 0) return 0;
+  fixed64_eval<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(kind, x, n, y);
+  return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
 extern "C" int qmc_probe_exp64(const double* x, int64_t n, double* y, void* stream) {
-  if (n < 0 || (n > 0 && (!x || !y))) return 1;
-  if (n == 0) return 0;
-  exp64_eval<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(x, n, y);
-  return cudaGetLastError() == cudaSuccess ? 0 : 4;
+  return qmc_probe_fixed64(0, x, n, y, stream);
 }
