@@ -315,23 +315,27 @@ __device__ __forceinline__ void group_s(const Tables<R>& t, int g, R dx, R dy, R
   }
 }
 
+// p shell: the components have the same weights (GK_P), so one radial sum
+// serves all three
 template <typename R, bool DERIV, typename F, bool CUT = false>
 __device__ __forceinline__ void group_p(const Tables<R>& t, int g, R dx, R dy, R dz, R r2, F& f) {
-  R G0[3], G1[3], G2[3];
-  group_radial<R, DERIV, 3, CUT>(t, g, r2, G0, G1, G2);
+  R G0[1], G1[1], G2[1];
+  group_radial<R, DERIV, 1, CUT>(t, g, r2, G0, G1, G2);
   const int a0 = t.group_ao[g];
   const R o = (R)0, i = (R)1;
   auto vs = [&](int c) { return t.vscale ? t.vscale[a0 + c] : (R)1; };
   f(a0, ao_from<R, DERIV>(dx, i, o, o, o, 1, dx, dy, dz, r2, G0[0], G1[0], G2[0], vs(0)));
-  f(a0 + 1, ao_from<R, DERIV>(dy, o, i, o, o, 1, dx, dy, dz, r2, G0[1], G1[1], G2[1], vs(1)));
-  f(a0 + 2, ao_from<R, DERIV>(dz, o, o, i, o, 1, dx, dy, dz, r2, G0[2], G1[2], G2[2], vs(2)));
+  f(a0 + 1, ao_from<R, DERIV>(dy, o, i, o, o, 1, dx, dy, dz, r2, G0[0], G1[0], G2[0], vs(1)));
+  f(a0 + 2, ao_from<R, DERIV>(dz, o, o, i, o, 1, dx, dy, dz, r2, G0[0], G1[0], G2[0], vs(2)));
 }
 
-// cartesian d shell, components xx, xy, xz, yy, yz, zz (pyscf.py:120-122)
+// cartesian d shell, components xx, xy, xz, yy, yz, zz (pyscf.py:120-122): the
+// squares share their weights and so do the mixed products (GK_D), so the
+// sums of xx and xy serve all six
 template <typename R, bool DERIV, typename F, bool CUT = false>
 __device__ __forceinline__ void group_d(const Tables<R>& t, int g, R dx, R dy, R dz, R r2, F& f) {
-  R G0[6], G1[6], G2[6];
-  group_radial<R, DERIV, 6, CUT>(t, g, r2, G0, G1, G2);
+  R G0[2], G1[2], G2[2];
+  group_radial<R, DERIV, 2, CUT>(t, g, r2, G0, G1, G2);
   const int a0 = t.group_ao[g];
   const R o = (R)0, two = (R)2;
   auto vs = [&](int c) { return t.vscale ? t.vscale[a0 + c] : (R)1; };
@@ -339,13 +343,13 @@ __device__ __forceinline__ void group_d(const Tables<R>& t, int g, R dx, R dy, R
                           vs(0)));
   f(a0 + 1, ao_from<R, DERIV>(dx * dy, dy, dx, o, o, 2, dx, dy, dz, r2, G0[1], G1[1], G2[1],
                               vs(1)));
-  f(a0 + 2, ao_from<R, DERIV>(dx * dz, dz, o, dx, o, 2, dx, dy, dz, r2, G0[2], G1[2], G2[2],
+  f(a0 + 2, ao_from<R, DERIV>(dx * dz, dz, o, dx, o, 2, dx, dy, dz, r2, G0[1], G1[1], G2[1],
                               vs(2)));
-  f(a0 + 3, ao_from<R, DERIV>(dy * dy, o, two * dy, o, two, 2, dx, dy, dz, r2, G0[3], G1[3], G2[3],
+  f(a0 + 3, ao_from<R, DERIV>(dy * dy, o, two * dy, o, two, 2, dx, dy, dz, r2, G0[0], G1[0], G2[0],
                               vs(3)));
-  f(a0 + 4, ao_from<R, DERIV>(dy * dz, o, dz, dy, o, 2, dx, dy, dz, r2, G0[4], G1[4], G2[4],
+  f(a0 + 4, ao_from<R, DERIV>(dy * dz, o, dz, dy, o, 2, dx, dy, dz, r2, G0[1], G1[1], G2[1],
                               vs(4)));
-  f(a0 + 5, ao_from<R, DERIV>(dz * dz, o, o, two * dz, two, 2, dx, dy, dz, r2, G0[5], G1[5], G2[5],
+  f(a0 + 5, ao_from<R, DERIV>(dz * dz, o, o, two * dz, two, 2, dx, dy, dz, r2, G0[0], G1[0], G2[0],
                               vs(5)));
 }
 
