@@ -20,6 +20,7 @@
 #pragma once
 
 #include "qmc_device.cuh"
+#include "qmc_fixdot.cuh"
 
 namespace qmc {
 
@@ -91,6 +92,9 @@ __host__ __device__ inline EPLayout ep_layout(const qmc_wf_desc& d, int kind) {
 // shared-memory and scratch layouts
 // ---------------------------------------------------------------------------
 constexpr int64_t kDetSmemBytes = 16384;
+// AOs per chunk of the FP64 local energy's contraction (two values per AO)
+constexpr int kFixElAOs = 8;
+static_assert(kFixElAOs >= QMC_MAX_COMP && kFixElAOs <= kFixAOs, "a chunk holds an AO group");
 
 struct EPShape {
   int nwb;       // walkers per block
@@ -104,6 +108,7 @@ struct EPShape {
   int64_t smem;  // dynamic shared memory bytes
   int64_t o_tab, o_pos, o_pnew, o_mo, o_bk, o_jrow, o_vrow, o_dref, o_psi, o_f, o_kin, o_v,
       o_iel, o_acc;
+  int64_t o_fix, o_ecol;  // FP64: the threads' AO values as limbs, W's column exponents
   int64_t o_det;  // determinant-phase work arrays of the block's walkers, or -1: HBM scratch
 };
 
@@ -151,6 +156,12 @@ __host__ __device__ inline EPShape ep_shape(const qmc_wf_desc& d, int kind, int 
   o += align8(nwb * 4);
   s.o_acc = o;
   o += align8(nwb * 4);
+  s.o_fix = s.o_ecol = o;
+  if (!kMixed<R>) {
+    o += (int64_t)s.nthreads * (kind == 1 ? 2 * kFixElAOs : kFixAOs) * 8;
+    s.o_ecol = o;
+    o += align8((int64_t)s.ncol * 4);
+  }
   // the determinant phase works in shared memory when the block's arrays are
   // small (the psi / Metropolis kernels of small molecules), else in HBM scratch
   const int64_t det_bytes = (int64_t)nwb * ep_layout(d, kind == 1 ? 1 : 0).bytes_per_slot;
@@ -199,6 +210,11 @@ __device__ __forceinline__ bool above_cut(float ar) { return ar > kRadialCut; }
 __device__ __forceinline__ bool above_cut(double ar) {
   return (unsigned)__double2hiint(ar) - 0x40470000u <= 0x7FF00000u - 0x40470000u;  // [46, inf]
 }
+// ar beyond which exp(-ar) is zero in FP64 (below half the smallest subnormal)
+__device__ __forceinline__ bool above_zero(float) { return false; }
+__device__ __forceinline__ bool above_zero(double ar) {
+  return (unsigned)__double2hiint(ar) - 0x40875000u <= 0x7FF00000u - 0x40875000u;  // [746, inf]
+}
 __device__ __forceinline__ bool is_zero(double x) {
   return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u;
 }
@@ -213,7 +229,7 @@ __device__ __forceinline__ void group_radial(const Tables<R>& t, int g, R r2, R 
   if (!t.group_split[g]) {
     for (int p = 0; p < np; ++p) {
       const R al = t.alpha[p0 + p], ar = al * r2;
-      if (CUT && above_cut(ar)) continue;
+      if (CUT ? above_cut(ar) : above_zero(ar)) continue;
       const R e0 = rexp(-ar);
       const R e1 = al * e0, e2 = al * e1;
 #pragma unroll
@@ -233,7 +249,7 @@ __device__ __forceinline__ void group_radial(const Tables<R>& t, int g, R r2, R 
       for (int c = 0; c < NC; ++c) {
         const int wi = wb + c * np + p;
         const R al = t.walpha[wi], ar = al * r2;
-        if (CUT && above_cut(ar)) continue;
+        if (CUT ? above_cut(ar) : above_zero(ar)) continue;
         const R e0 = rexp(-ar);
         const R w = t.wd[wi];
         G0[c] = fma(w, e0, G0[c]);
@@ -413,13 +429,13 @@ __device__ __forceinline__ void group_sto(const Tables<R>& t, int g, R dx, R dy,
 
 // All AOs of one electron (split coordinates ex, ey, ez); the electron-atom
 // difference is formed once per atom (groups are stored atom by atom).
-template <typename R, bool DERIV, typename F>
+template <typename R, bool DERIV, typename F, bool CUT = !kMixed<R>>
 __device__ __forceinline__ void for_each_ao_ep(const Tables<R>& t, XP<R> ex, XP<R> ey, XP<R> ez,
-                                               F& f) {
+                                               F& f, int g0, int g1) {
   int last = -1;
   R dx = 0, dy = 0, dz = 0, r2 = 0;
   const bool sto = t.radial != QMC_RADIAL_GTO;
-  for (int g = 0; g < t.ngroup; ++g) {
+  for (int g = g0; g < g1; ++g) {
     const int A = t.group_atom[g];
     if (A != last) {
       dx = dif(ex, t.atom_p[3 * A]);
@@ -434,8 +450,63 @@ __device__ __forceinline__ void for_each_ao_ep(const Tables<R>& t, XP<R> ex, XP<
     if (sto)
       group_sto<R, DERIV>(t, g, dx, dy, dz, r2, f);
     else
-      ao_group<R, DERIV, F, !kMixed<R>>(t, g, dx, dy, dz, r2, f);
+      ao_group<R, DERIV, F, CUT>(t, g, dx, dy, dz, r2, f);
   }
+}
+
+template <typename R, bool DERIV, typename F, bool CUT = !kMixed<R>>
+__device__ __forceinline__ void for_each_ao_ep(const Tables<R>& t, XP<R> ex, XP<R> ey, XP<R> ez,
+                                               F& f) {
+  for_each_ao_ep<R, DERIV, F, CUT>(t, ex, ey, ez, f, 0, t.ngroup);
+}
+
+// FP64 MO row of an electron at (x, y, z) by the fixed-point contraction: element j
+// to mo[j * rs] (over the AO groups gb .. ge - 1) and, with KIN, -1/2 (sum_a (lap AO_a + 2 g . grad AO_a) W_aj + jl mo_j)
+// to bk[j * rs]. v: the thread's limb slots (stride vs): kFixAOs, or with KIN 2 kFixElAOs.
+template <bool KIN, bool CUT>
+__device__ inline void ep_fixed_rows(const Tables<double>& t, const int* ecol, int nmu, double x,
+                                     double y, double z, double gx, double gy, double gz,
+                                     double jl, int2* v, int vs, double* mo, double* bk,
+                                     int64_t rs, int gb, int ge) {
+  constexpr int kCap = KIN ? kFixElAOs : kFixAOs;
+  const int2* W = reinterpret_cast<const int2*>(t.W);
+  if (gb >= ge)
+    for (int j = 0; j < nmu; ++j) mo[j * rs] = 0.0;
+  for (int g0 = gb; g0 < ge;) {
+    const int a0 = t.group_ao[g0];
+    int g1 = g0 + 1;
+    while (g1 < ge && t.group_ao[g1 + 1] - a0 <= kCap) ++g1;
+    const int na = t.group_ao[g1] - a0;
+    // values first, then limbs relative to the chunk's largest exponent
+    int Ev = 0, Eb = 0;
+    auto put = [&](int i, double val, int& E) {
+      const int e = (__double2hiint(val) >> 20) & 0x7FF;
+      E = e > E ? e : E;
+      v[i * vs] = make_int2(__double2hiint(val), __double2loint(val));
+    };
+    auto acc = [&](int a, const AOVal<double>& o) {
+      put(a - a0, o.v, Ev);
+      if (KIN) put(kCap + a - a0, o.lap + 2.0 * (gx * o.gx + gy * o.gy + gz * o.gz), Eb);
+    };
+    for_each_ao_ep<double, KIN, decltype(acc), CUT>(t, XP<double>{x, 0.0}, XP<double>{y, 0.0},
+                                                    XP<double>{z, 0.0}, acc, g0, g1);
+    auto limbs = [&](int i, int E) {
+      const int2 q = v[i * vs];
+      v[i * vs] = fix_limbs(__hiloint2double(q.x, q.y), E);
+    };
+    if (Ev > 0 || g0 == gb) {  // a chunk of zeros (cut primitives) adds nothing
+      for (int i = 0; i < na; ++i) limbs(i, Ev);
+      fix_rows(v, vs, na, Ev, W + (int64_t)a0 * t.ncol, t.ncol, ecol, nmu, mo, rs, g0 == gb);
+    }
+    if (KIN && (Eb > 0 || g0 == gb)) {
+      for (int i = 0; i < na; ++i) limbs(kCap + i, Eb);
+      fix_rows(v + kCap * vs, vs, na, Eb, W + (int64_t)a0 * t.ncol, t.ncol, ecol, nmu, bk, rs,
+               g0 == gb);
+    }
+    g0 = g1;
+  }
+  if (KIN)
+    for (int j = 0; j < nmu; ++j) bk[j * rs] = -0.5 * fma(jl, mo[j * rs], bk[j * rs]);
 }
 
 // JC consecutive W values with vector loads (rows are 16-byte aligned and
@@ -469,7 +540,8 @@ __device__ __forceinline__ void load_w(const double* p, double (&w)[JC]) {
 // electron; vrow (E_L): its V_en plus half its V_ee row.
 template <typename R, int JC, bool KIN>
 __device__ inline void ep_electron(const qmc_wf_desc& d, const Tables<R>& t, const XP<R>* pw,
-                                   int e, R* mo, R* bk, int nwb, double* jrow, double* vrow) {
+                                   int e, R* mo, R* bk, int nwb, double* jrow, double* vrow,
+                                   int2* fix, int fix_stride, const int* ecol) {
   const int ne = d.nelec, nmu = d.nmo_used;
   const XP<R> ex = pw[3 * e], ey = pw[3 * e + 1], ez = pw[3 * e + 2];
   R gx = (R)0, gy = (R)0, gz = (R)0, jl = (R)0;
@@ -534,39 +606,32 @@ __device__ inline void ep_electron(const qmc_wf_desc& d, const Tables<R>& t, con
   const int64_t cs = nwb;
   R* mrow = mo + (int64_t)e * nmu * cs;
   R* brow = KIN ? bk + (int64_t)e * nmu * cs : nullptr;
-  for (int j0 = 0; j0 < nmu; j0 += JC) {
-    R a0[JC], ad[JC], al[JC];
+  if constexpr (!kMixed<R>) {
+    ep_fixed_rows<KIN, true>(t, ecol, nmu, ex.h, ey.h, ez.h, gx, gy, gz, jl, fix, fix_stride, mrow,
+                             brow, cs, 0, t.ngroup);
+  } else {
+    for (int j0 = 0; j0 < nmu; j0 += JC) {
+      R a0[JC], ab[JC];
 #pragma unroll
-    for (int jj = 0; jj < JC; ++jj) a0[jj] = ad[jj] = al[jj] = (R)0;
-    auto acc = [&](int a, const AOVal<R>& o) {
-      // FP64: an AO whose primitives were all cut (far atom) is zero with its
-      // derivatives, and its FMAs would add zeros: skipped (the lanes of a warp
-      // evaluate the same electron index of different walkers, so the branch
-      // is mostly uniform)
-      if constexpr (!kMixed<R>) {
-        if (is_zero(o.v) && (!KIN || (is_zero(o.gx) && is_zero(o.gy) && is_zero(o.gz) &&
-                                      is_zero(o.lap))))
-          return;
-      }
-      R wv[JC];
-      load_w<JC>(t.W + (int64_t)a * t.ncol + j0, wv);
-      R gdot = (R)0;
-      if (KIN) gdot = (R)2 * (gx * o.gx + gy * o.gy + gz * o.gz);
+      for (int jj = 0; jj < JC; ++jj) a0[jj] = ab[jj] = (R)0;
+      auto acc = [&](int a, const AOVal<R>& o) {
+        R wv[JC];
+        load_w<JC>(t.W + (int64_t)a * t.ncol + j0, wv);
+        R b = (R)0;
+        if (KIN) b = o.lap + (R)2 * (gx * o.gx + gy * o.gy + gz * o.gz);
+#pragma unroll
+        for (int jj = 0; jj < JC; ++jj) {
+          a0[jj] = fma(o.v, wv[jj], a0[jj]);
+          if (KIN) ab[jj] = fma(b, wv[jj], ab[jj]);
+        }
+      };
+      for_each_ao_ep<R, KIN>(t, ex, ey, ez, acc);
 #pragma unroll
       for (int jj = 0; jj < JC; ++jj) {
-        a0[jj] = fma(o.v, wv[jj], a0[jj]);
-        if (KIN) {
-          ad[jj] = fma(gdot, wv[jj], ad[jj]);
-          al[jj] = fma(o.lap, wv[jj], al[jj]);
+        if (j0 + jj < nmu) {
+          mrow[(j0 + jj) * cs] = a0[jj];
+          if (KIN) brow[(j0 + jj) * cs] = (R)(-0.5) * (ab[jj] + jl * a0[jj]);
         }
-      }
-    };
-    for_each_ao_ep<R, KIN>(t, ex, ey, ez, acc);
-#pragma unroll
-    for (int jj = 0; jj < JC; ++jj) {
-      if (j0 + jj < nmu) {
-        mrow[(j0 + jj) * cs] = a0[jj];
-        if (KIN) brow[(j0 + jj) * cs] = (R)(-0.5) * (al[jj] + ad[jj] + jl * a0[jj]);
       }
     }
   }
@@ -1023,7 +1088,7 @@ __device__ inline double coop_lu_steps(R* A, int64_t rs, int64_t cs, int n, int 
       piv[k] = p;
       if (p != k) det = -det;
       det *= to_f64(akk);
-      inv = akk != (R)0 ? (R)1 / akk : (R)0;
+      inv = akk != (R)0 ? prcp(akk) : (R)0;
       for (int i = k + 1 + r; i < n; i += nt) {
         const R l = A[i * rs + k * cs] * inv;
         A[i * rs + k * cs] = l;
@@ -1170,6 +1235,15 @@ struct EPPtrs {
   EPShape S;
 };
 
+// The block's tables for the electron-parallel kernels (FP64: W as limbs).
+template <typename R>
+__device__ inline Tables<R> ep_tables(const qmc_wf_desc& d, const EPShape& S, unsigned char* smem) {
+  const Tables<R> t = load_tables<R>(d, d.nmo_used, S.ncol, smem + S.o_tab);
+  if constexpr (!kMixed<R>)
+    fix_table(const_cast<R*>(t.W), t.nao, t.ncol, reinterpret_cast<int*>(smem + S.o_ecol));
+  return t;
+}
+
 // Evaluate psi (and, with KIN, the kinetic energy and potentials) for the
 // block's walkers at split positions `pbuf` (shared memory, [nwb][3 nelec]).
 // Results in shared memory: psi[wl], and with KIN kin[wl], v[wl] (V_en + V_ee),
@@ -1207,7 +1281,9 @@ __device__ inline void ep_eval(const qmc_wf_desc& d, const Tables<R>& t, const E
       const int e = ((b / ns) & 1) ? b + ns - 1 - slot : b + slot;
       if (e < ne)
         ep_electron<R, JC, KIN>(d, t, pbuf + wl * S.pstride, e, MO + wl, BK + wl, nwb,
-                                &JR[e * nwb + wl], &VR[e * nwb + wl]);
+                                &JR[e * nwb + wl], &VR[e * nwb + wl],
+                                reinterpret_cast<int2*>(p.smem + S.o_fix) + tid, S.nthreads,
+                                reinterpret_cast<const int*>(p.smem + S.o_ecol));
     }
   }
   __syncthreads();
@@ -1244,7 +1320,7 @@ __device__ inline void ep_eval(const qmc_wf_desc& d, const Tables<R>& t, const E
     double jf = 1.0;
     if (d.use_jastrow || d.use_jastrow_en) {
       if constexpr (kMixed<R> && !KIN) jf = exp_mixed(logj);
-      else jf = exp(logj);
+      else jf = jexp(logj);
     }
     PSI[wl] = psid * jf;
     if (KIN) {

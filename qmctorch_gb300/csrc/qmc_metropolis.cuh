@@ -27,7 +27,7 @@ __device__ __forceinline__ void metropolis_block(const qmc_wf_desc& d, const qmc
                                                  unsigned char* __restrict__ scr, int64_t ss,
                                                  const EPShape& S, int64_t block,
                                                  unsigned char* smem) {
-  const Tables<R> t = load_tables<R>(d, d.nmo_used, S.ncol, smem + S.o_tab);
+  const Tables<R> t = ep_tables<R>(d, S, smem);
   const int64_t nw = a.nwalkers;
   const int nwb = S.nwb, ne = d.nelec, nc = 3 * ne, ps = S.pstride;
   const int64_t w0 = block * nwb;
@@ -135,7 +135,7 @@ __device__ __forceinline__ void metropolis_block(const qmc_wf_desc& d, const qmc
           // same decision up to the rounding of the ratio
           acc = fxn >= u * F[tid] ? 1 : 0;
         } else {
-          double df = fxn / F[tid];
+          double df = pdiv(fxn, F[tid]);
           if (df > 1.0) df = 1.0;
           acc = (df - u >= 0.0) ? 1 : 0;
         }

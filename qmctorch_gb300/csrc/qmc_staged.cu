@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(128) jastrow_kernel(const qmc_wf_desc d, const
   const int ne = d.nelec;
   PosView P{pos + w * 3 * ne, 1};
   const double wj = __ldg(d.jastrow_w);
-  const double J = exp(jastrow_log<double>(d, P, wj));
+  const double J = jexp(jastrow_log<double>(d, P, wj));
   if (jast) jast[w] = J;
   if (!djast && !d2jast) return;
   for (int i = 0; i < ne; ++i) {
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(128) jastrow_en_kernel(const qmc_wf_desc d,
   PosView P{pos + w * 3 * ne, 1};
   double u = 0.0;
   for (int i = 0; i < ne; ++i) u += en_terms(d, P(3 * i), P(3 * i + 1), P(3 * i + 2)).u;
-  const double J = exp(u);
+  const double J = jexp(u);
   if (jast) jast[w] = J;
   if (!djast && !d2jast) return;
   for (int i = 0; i < ne; ++i) {

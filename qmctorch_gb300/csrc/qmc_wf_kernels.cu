@@ -18,7 +18,7 @@ __global__ void __launch_bounds__(EPBound<R>::kThreads) ep_psi_kernel(const qmc_
                                                       unsigned char* __restrict__ scr, int64_t ss,
                                                       const EPShape S) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const Tables<R> t = load_tables<R>(d, d.nmo_used, S.ncol, smem + S.o_tab);
+  const Tables<R> t = ep_tables<R>(d, S, smem);
   const int64_t w0 = (int64_t)blockIdx.x * S.nwb;
   XP<R>* P = reinterpret_cast<XP<R>*>(smem + S.o_pos);
   ep_stage_positions<R>(pos, w0, nw, S.nwb, 3 * d.nelec, S.pstride, P);
@@ -36,7 +36,7 @@ __global__ void __launch_bounds__(EPElBound<R>::kThreads) ep_eloc_kernel(const q
                                                        unsigned char* __restrict__ scr, int64_t ss,
                                                        const EPShape S) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const Tables<R> t = load_tables<R>(d, d.nmo_used, S.ncol, smem + S.o_tab);
+  const Tables<R> t = ep_tables<R>(d, S, smem);
   const int64_t w0 = (int64_t)blockIdx.x * S.nwb;
   XP<R>* P = reinterpret_cast<XP<R>*>(smem + S.o_pos);
   ep_stage_positions<R>(pos, w0, nw, S.nwb, 3 * d.nelec, S.pstride, P);
