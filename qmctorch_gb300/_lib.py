@@ -23,12 +23,14 @@ BUILD = os.path.join(ROOT, "_build")
 INCLUDE = os.path.join(ROOT, "include")
 
 SOURCES = ["qmc_wf_kernels.cu", "qmc_staged.cu", "qmc_metropolis.cu", "qmc_capi_common.cu",
-           "qmc_probe.cu", "qmc_adjoint.cu", "qmc_drift.cu", "qmc_sweep.cu", "qmc_reduce.cu",
+           "qmc_probe.cu", "qmc_adjoint.cu", "qmc_gradients.cu", "qmc_drift.cu", "qmc_sweep.cu", "qmc_reduce.cu",
            "qmc_mo_tc.cu", "qmc_scf.cpp"]
 # translation units compiled more than once, with defines: (source, object, flags)
 INSTANCES = [("qmc_metropolis_inst.cu", "qmc_metropolis_%s_%d" % (r, jc),
               ["-DQMC_INST_R=%s" % r, "-DQMC_INST_JC=%d" % jc])
              for r in ("float", "double") for jc in (8, 16, 24)]
+INSTANCES += [("qmc_hmc_inst.cu", "qmc_hmc_%d" % jc, ["-DQMC_INST_JC=%d" % jc])
+              for jc in (8, 16, 24)]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I" + INCLUDE]
 

@@ -1,7 +1,5 @@
-// Drift-diffusion (generalized) Metropolis and Hamiltonian Monte Carlo on the
-// device, FP64, one thread per walker for all steps of a call
-// (generalized_metropolis.py:46-219, hamiltonian.py:75-201); the HMC kernel is
-// at the end of the file.
+// Drift-diffusion (generalized) Metropolis on the device, FP64, one thread per
+// walker for all steps of a call (generalized_metropolis.py:46-219).
 //
 // The reference's chain, kept as it is so that replayed draws give its chains:
 // every proposal starts from the walkers' positions at the start of the call
@@ -365,98 +363,6 @@ __global__ void __launch_bounds__(kDriftTPB) drift_kernel(const qmc_wf_desc d,
   if (a.accepted) a.accepted[w] += nacc;
 }
 
-// ---------------------------------------------------------------------------
-// Hamiltonian Monte Carlo (hamiltonian.py:75-201)
-// ---------------------------------------------------------------------------
-// Per step and walker: momenta p ~ N(0, I) over all 3 Ne coordinates,
-// H_start = U(q) + |p|^2 / 2 with U = -log psi^2, a leapfrog trajectory of L
-// steps of size eps (half momentum step, L - 1 full position + momentum steps,
-// a last position step and half momentum step) with the force
-// -grad U = 2 grad psi / psi from the full Jacobi evaluation at each point,
-// p negated, and the end point rejected when exp(H_start - H_end) < u. The
-// trajectory's positions, momenta and forces live in the walker's work
-// arrays (xi, dri, drf); pos holds the chain's current positions.
-__global__ void __launch_bounds__(kDriftTPB) hmc_kernel(const qmc_wf_desc d,
-                                                        const qmc_hmc_args a,
-                                                        double* __restrict__ scr, int64_t ss) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int ncol = round_up(d.nmo_used, 8);
-  const Tables<double> t = load_tables<double>(d, d.nmo_used, ncol, smem);
-  const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= a.nwalkers) return;
-  const int nc = 3 * d.nelec;
-  const DriftLayout L = drift_layout(d);
-  double* sw = scr + w;
-  auto S = [&](int64_t item) -> double& { return sw[item * ss]; };
-  double* x0 = a.pos + w * nc;  // the chain's current positions
-  const double eps = a.step_size, heps = 0.5 * a.step_size;
-  const bool replay = a.momenta != nullptr;
-  Rng rng{(uint32_t)a.seed, (uint32_t)(a.seed >> 32), (uint32_t)w, 0, 0};
-  int nacc = 0, idecor = 0;
-  int64_t isnap = 0;
-  double* q = sw + L.xi * ss;  // trajectory positions, stride ss
-  for (int istep = 0; istep < a.nstep; ++istep) {
-    // momenta (replayed, or Box-Muller pairs of the step's Philox stream)
-    rng.step = a.step_offset + istep;
-    rng.call = 0;
-    double psq = 0.0;
-    for (int c = 0; c < nc; c += 4) {
-      double z[4];
-      if (replay) {
-        for (int k = 0; k < 4 && c + k < nc; ++k)
-          z[k] = a.momenta[((int64_t)istep * a.nwalkers + w) * nc + c + k];
-      } else {
-        const U4 r = rng.next();
-        rng.normal2(r.x, r.y, z[0], z[1]);
-        rng.normal2(r.z, r.w, z[2], z[3]);
-      }
-      for (int k = 0; k < 4 && c + k < nc; ++k) {
-        S(L.dri + c + k) = z[k];
-        psq = fma(z[k], z[k], psq);
-      }
-    }
-    for (int c = 0; c < nc; ++c) S(L.xi + c) = x0[c];
-    double logj;
-    double sigma = drift_full_eval(d, t, L, sw, ss, x0, 1, L.drf, &logj);
-    const double h0 = -2.0 * (logj + log(fabs(sigma))) + 0.5 * psq;
-    // half step in momentum: p -= (eps / 2) grad U, grad U = -2 grad log psi
-    for (int c = 0; c < nc; ++c)
-      S(L.dri + c) = __dsub_rn(S(L.dri + c), __dmul_rn(heps, -2.0 * S(L.drf + c)));
-    for (int l = 0; l < a.traj_length; ++l) {
-      for (int c = 0; c < nc; ++c) q[c * ss] = __dadd_rn(q[c * ss], __dmul_rn(eps, S(L.dri + c)));
-      sigma = drift_full_eval(d, t, L, sw, ss, q, ss, L.drf, &logj);
-      const double f = l + 1 < a.traj_length ? eps : heps;  // the last momentum step is a half step
-      for (int c = 0; c < nc; ++c)
-        S(L.dri + c) = __dsub_rn(S(L.dri + c), __dmul_rn(f, -2.0 * S(L.drf + c)));
-    }
-    // p is negated before the kinetic energy, which its sign does not change
-    psq = 0.0;
-    for (int c = 0; c < nc; ++c) psq = fma(S(L.dri + c), S(L.dri + c), psq);
-    const double h1 = -2.0 * (logj + log(fabs(sigma))) + 0.5 * psq;
-    double u;
-    if (replay) {
-      u = a.uniforms[(int64_t)istep * a.nwalkers + w];
-    } else {
-      rng.call = (uint32_t)((nc + 3) / 4);
-      const U4 r = rng.next();
-      u = rng.uniform53(r.x, r.y);
-    }
-    if (!(exp(h0 - h1) < u)) {
-      ++nacc;
-      for (int c = 0; c < nc; ++c) x0[c] = q[c * ss];
-    }
-    if (istep >= a.ntherm) {
-      if (idecor % a.ndecor == 0 && a.samples && isnap < a.nsnap) {
-        double* o = a.samples + (isnap * a.nwalkers + w) * nc;
-        for (int c = 0; c < nc; ++c) o[c] = x0[c];
-        ++isnap;
-      }
-      ++idecor;
-    }
-  }
-  if (a.accepted) a.accepted[w] += nacc;
-}
-
 }  // namespace qmc
 
 using namespace qmc;
@@ -493,35 +399,6 @@ int qmc_drift_run(const qmc_wf_desc* d0, const qmc_drift_args* a, void* scratch,
   const double sd = sqrt(sqrt(a->step_size));  // covariance sqrt(step) I
   drift_kernel<<<grid, kDriftTPB, smem, (cudaStream_t)stream>>>(
       dd, *a, (double*)scratch, pad_walkers(a->nwalkers), sd);
-  return launch_status();
-}
-
-int64_t qmc_hmc_scratch_bytes(const qmc_wf_desc* d, int64_t nw) {
-  return qmc_drift_scratch_bytes(d, nw);
-}
-
-int qmc_hmc_run(const qmc_wf_desc* d0, const qmc_hmc_args* a, void* scratch,
-                int64_t scratch_bytes, void* stream) {
-  int st = check_desc(d0);
-  if (st) return st;
-  if (!a) return QMC_ERR_ARG;
-  qmc_wf_desc dd = *d0;
-  dd.precision = QMC_PREC_FP64;  // the HMC sampler is FP64
-  const qmc_wf_desc* d = &dd;
-  if (a->nwalkers < 0 || a->nstep < 0 || a->ntherm < 0 || a->ndecor < 1 || a->nsnap < 0 ||
-      a->traj_length < 1 || !(a->step_size > 0.0))
-    return QMC_ERR_ARG;
-  if ((a->momenta != nullptr) != (a->uniforms != nullptr)) return QMC_ERR_ARG;
-  if (a->nwalkers == 0 || a->nstep == 0) return QMC_OK;
-  if (!a->pos || !scratch) return QMC_ERR_ARG;
-  if (a->nsnap > 0 && !a->samples) return QMC_ERR_ARG;
-  if (scratch_bytes < qmc_hmc_scratch_bytes(d, a->nwalkers)) return QMC_ERR_SCRATCH;
-  const int ncol = round_up(d->nmo_used, 8);
-  const int64_t smem = tables_smem_bytes<double>(*d, ncol);
-  if ((st = prepare_smem(hmc_kernel, smem))) return st;
-  const dim3 grid((unsigned)((a->nwalkers + kDriftTPB - 1) / kDriftTPB));
-  hmc_kernel<<<grid, kDriftTPB, smem, (cudaStream_t)stream>>>(dd, *a, (double*)scratch,
-                                                               pad_walkers(a->nwalkers));
   return launch_status();
 }
 
