@@ -1,5 +1,5 @@
-// Drift-diffusion (generalized) Metropolis on the device, FP64, one thread per
-// walker for all steps of a call (generalized_metropolis.py:46-219).
+// Drift-diffusion (generalized) Metropolis on the device, FP64, all steps of a
+// call in one launch (generalized_metropolis.py:46-219).
 //
 // The reference's chain, kept as it is so that replayed draws give its chains:
 // every proposal starts from the walkers' positions at the start of the call
@@ -12,258 +12,446 @@
 // min(1, T_if rho_f / (T_fi rho_i)) - u >= 0.
 //
 // Because each proposal differs from the start positions in one electron only,
-// the start positions' MO rows (values and gradients), spin determinants,
-// determinant gradients and Jastrow gradient are computed once per call; a
-// step evaluates the moved electron's MO row, refactors the determinants of
-// its spin with that row replaced, and updates the Jastrow terms of its pairs.
-// psi and its electron gradient at the proposal are therefore the full
-// Jacobi-formula values (slater_jastrow.py:346-447), not an approximation.
+// what the gradients need of the start positions is computed once per call; a
+// step evaluates the moved electron's MO row, the determinants of its spin with
+// that row replaced, and the Jastrow terms of its pairs. psi and its electron
+// gradient at the proposal are the full Jacobi-formula values
+// (slater_jastrow.py:346-447), not an approximation.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "qmc_grad.cuh"
 #include "qmc_host.cuh"
 #include "qmc_rng.cuh"
 
 namespace qmc {
 
-constexpr int kDriftTPB = 64;
-
-struct DriftLayout {  // per-walker doubles, item-major
-  int64_t xi, ma, mx, my, mz, ao, nr, lu, x, dv0, gd0, dvf, gdf, jg0, dri, drf, total;
+// A walker's nslot threads share its work: the AO groups of the moved electron
+// (partial MO rows, partial gradients), the electrons' pairs and gradients.
+// FP64 pipe bound, so counted in FP64 instructions (H2O cc-pVDZ
+// single_double(4,4), about 1,700 per step instead of 14,000 of per-determinant
+// factorisations and component-wise AO gradients). Excitation mode: with A^-1
+// and X = A^-1 V of the start, a proposal of electron l is a rank-one change,
+//   r = phi'^T A^-1 (det' / det = r_l),  X' = X + A^-1 e_l (phi'_virt - phi' X) / r_l,
+// from the start each time, so nothing accumulates over the steps; and with
+//   Z_i[l] = sum_k A^-1(k, l) grad MO_k(r_i),
+//   m_i[v] = grad MO_virt,v(r_i) - sum_j X(j, v) grad MO_j(r_i)
+// of the start the determinant gradient of every electron that did not move is
+//   Sigma (Z_i[i] - q r_i Z_i[l]) + sum_v (m_i[v] - q t_v Z_i[l]) f_v(i),  q = 1 / r_l
+// (without the l terms for the other spin), f_v(i) = sum_k A'^-1(k, i) F(k, v),
+// F = d Sigma / d X (qmc_grad.cuh); the moved electron's comes from one pass over
+// its AOs. Explicit mode (CAS), and a proposal with a large excitation ratio
+// (kGradRatio), refactor the moved spin's determinants.
+struct DriftShape {
+  int nwb, nslot, nthreads, ncol;
+  int64_t o_wl, o_ecol, o_fix;  // W as limbs, its column exponents, the threads' AO limbs
+  int64_t smem, o_hot;  // o_hot < 0: the hot arrays too are in the scratch
+  // per walker, in doubles. Hot (shared memory): start positions, the two drifts
+  // (accepted and proposed), Jastrow gradient, the moved electron's MO row, its
+  // partial rows, r, t, X', F of both spins, the proposal's determinants, G of
+  // the moved electron, partial sums, scalars
+  int xs, dr, gj, phi, part, r, t, xp, f, dvf, g, red, val, hot;
+  // cold (scratch): MO values and gradients, LU | X, Z | m, A^-1 by columns,
+  // determinants, Jastrow of the start, pivots, work of the explicit sums
+  int ma, mg, lx, zm, inv, dv0, jg0, ju, jen, piv, lu, ginv, gx, cold;
 };
+enum { DV_SIGMA = 0, DV_Q = 1, DV_DET = 2, DV_FLAG = 4, DV_CUR = 5, DV_EACC = 6, DV_XACC = 7,
+       DV_N = 10 };
+constexpr int kDriftRed = 6;  // partial sums per slot: du, a1, a2, the moved electron's grad U
 
-__host__ __device__ inline DriftLayout drift_layout(const qmc_wf_desc& d) {
-  DriftLayout L;
-  const int64_t ne = d.nelec, nmu = d.nmo_used, nao = d.nao;
-  const int64_t nmax = d.nup > d.ndown ? d.nup : d.ndown, nd = d.ndet[0] + d.ndet[1];
-  int64_t o = 0;
-  auto take = [&](int64_t n) {
-    const int64_t r = o;
+static DriftShape drift_shape(const qmc_wf_desc& d, int nwb, int nslot, bool in_smem) {
+  DriftShape s;
+  s.nwb = nwb;
+  s.nslot = nslot;
+  s.nthreads = ((nwb * nslot + 31) / 32) * 32;
+  s.ncol = round_up(d.nmo_used, 8);
+  const int ne = d.nelec, nmu = d.nmo_used, nmax = d.nup > d.ndown ? d.nup : d.ndown;
+  const bool ex = d.det_mode == QMC_DET_EXPLICIT;
+  const int v0 = ex ? 0 : d.max_orb[0] - d.nup, v1 = ex ? 0 : d.max_orb[1] - d.ndown;
+  const int nv = v0 > v1 ? v0 : v1, nd = d.ndet[0] + d.ndet[1];
+  int o = 0;
+  auto take = [&](int n) {
+    const int r = o;
     o += n;
     return r;
   };
-  L.xi = take(3 * ne);        // current (accepted) positions
-  L.ma = take(ne * nmu);      // start positions: MO values
-  L.mx = take(ne * nmu);      // and their gradients
-  L.my = take(ne * nmu);
-  L.mz = take(ne * nmu);
-  L.ao = take(4 * nao);       // AO values and gradients of one electron
-  L.nr = take(4 * nmu);       // the moved electron's MO row (value, gradient)
-  L.lu = take(nmax * nmax);
-  L.x = take(nmax * nmax);    // inverse of one spin determinant
-  L.dv0 = take(nd);           // spin determinants at the start positions
-  L.gd0 = take(nd * nmax * 3);  // their d log D / d r_i
-  L.dvf = take(nd);           // the moved spin's determinants at the proposal
-  L.gdf = take(nd * nmax * 3);
-  L.jg0 = take(3 * ne);       // grad log J at the start positions
-  L.dri = take(3 * ne);       // drift at x_i
-  L.drf = take(3 * ne);       // drift at the proposal
-  L.total = o;
-  return L;
-}
-
-// MO values and gradients of one electron at (x, y, z): AO values and
-// gradients through the scratch, then the contraction with W; row element j
-// of quantity q (0 value, 1..3 gradient) goes to sw[(dst[q] + j) * ss].
-__device__ inline void drift_rows(const Tables<double>& t, int nmu, double* sw, int64_t ss,
-                                  int64_t ao, double x, double y, double z, const int64_t (&dst)[4]) {
-  const int nao = t.nao;
-  for_each_ao<double, true>(t, x, y, z, [&](int a, const AOVal<double>& v) {
-    sw[(ao + a) * ss] = v.v;
-    sw[(ao + nao + a) * ss] = v.gx;
-    sw[(ao + 2 * nao + a) * ss] = v.gy;
-    sw[(ao + 3 * nao + a) * ss] = v.gz;
-  });
-  for (int j = 0; j < nmu; ++j) {
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int a = 0; a < nao; ++a) {
-      const double w = t.W[(int64_t)a * t.ncol + j];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) s[q] = fma(sw[(ao + q * nao + a) * ss], w, s[q]);
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) sw[(dst[q] + j) * ss] = s[q];
+  s.xs = take(3 * ne);
+  s.dr = take(6 * ne);
+  s.gj = take(3 * ne);
+  s.phi = take(nmu);
+  s.part = take(nslot * (nmu > 3 ? nmu : 3));
+  s.r = take(nmax);
+  s.t = take(nv);
+  s.xp = take(nmax * nv);
+  s.f = take(2 * nmax * nv);
+  s.dvf = take(d.ndet[0] > d.ndet[1] ? d.ndet[0] : d.ndet[1]);
+  s.g = take(nmu);
+  s.red = take(nslot * kDriftRed);
+  s.val = take(DV_N);
+  s.hot = o;
+  o = 0;
+  s.ma = take(ne * nmu);
+  s.mg = take(3 * ne * nmu);
+  s.lx = take(ex ? 0 : ne * nmu);
+  s.zm = take(ex ? 0 : 3 * ne * nmu);
+  s.inv = take(ex ? 0 : ne * nmax);
+  s.dv0 = take(nd);
+  s.jg0 = take(3 * ne);
+  s.ju = take(ne);
+  s.jen = take(ne);
+  s.piv = take(ne);
+  s.lu = take(2 * nmax * nmax);
+  s.ginv = take(2 * nmax * nmax);
+  s.gx = take(ne * nmu);
+  s.cold = o;
+  s.o_wl = (tables_smem_bytes<double>(d, s.ncol) + 15) & ~int64_t(15);
+  s.o_ecol = s.o_wl + (int64_t)d.nao * s.ncol * 8;
+  s.o_fix = s.o_ecol + align8((int64_t)s.ncol * 4);
+  s.smem = (s.o_fix + (int64_t)s.nthreads * kFixAOs * 8 + 15) & ~int64_t(15);
+  s.o_hot = -1;
+  if (in_smem) {
+    s.o_hot = s.smem;
+    s.smem += (int64_t)s.hot * nwb * 8;
   }
+  return s;
 }
 
-// Spin determinant u of spin s from the start rows, with electron er's row
-// taken from the moved row (er < 0: none); writes d log D / d r_i of the
-// spin's electrons to sw[(gd + i * 3 + q) * ss] and returns D.
-__device__ inline double drift_det(const qmc_wf_desc& d, const DriftLayout& L, double* sw,
-                                   int64_t ss, int s, int u, int er, int64_t gd) {
+struct DriftWork {  // one thread's walker: hot and cold arrays
+  double* hp;
+  int64_t hs;
+  double* cp;
+  int64_t cs;
+  __device__ __forceinline__ double& H(int i) const { return hp[(int64_t)i * hs]; }
+  __device__ __forceinline__ double& C(int i) const { return cp[(int64_t)i * cs]; }
+};
+
+// Electron-electron Pade pair at the difference dx: u = w0 r / (1 + w r), and
+// returns the factor c of its gradient, c dx = w0 / (1 + w r)^2 dx / r.
+__device__ __forceinline__ double pade_pair(double w0, double w, double dx, double dy, double dz,
+                                            double& u) {
+  const double r = psqrt(dx * dx + dy * dy + dz * dz);
+  const double iu = prcp(fma(w, r, 1.0)), q = w0 * iu;
+  u = q * r;
+  return q * iu * prcp(r);
+}
+
+// One thread per (walker, spin): the explicit determinants of spin s from
+// the start rows (electron er's row from `phi`; er < 0: none) to dst, and
+// G(i, j) = sum_u coef_u det_u A_u^-T into the spin's rows of gx with coef_u
+// from the other spin's determinants at oth (oth < 0: determinants only).
+__device__ __noinline__ void drift_explicit(const qmc_wf_desc& d, const DriftShape& S,
+                                      const DriftWork& k, int s, int er, double* dst, int64_t ds,
+                                      const double* oth, int64_t os) {
   const int n = s ? d.ndown : d.nup, r0 = s ? d.nup : 0, nmu = d.nmo_used;
   const int nmax = d.nup > d.ndown ? d.nup : d.ndown;
-  if (n == 0) return 1.0;
-  int cols[QMC_MAX_NSPIN], piv[QMC_MAX_NSPIN];
-  det_columns(d, s, u, cols);
-  auto row = [&](int q, int i, int c) -> double {
-    if (r0 + i == er) return sw[(L.nr + (int64_t)q * nmu + c) * ss];
-    const int64_t base = q == 0 ? L.ma : (q == 1 ? L.mx : (q == 2 ? L.my : L.mz));
-    return sw[(base + (int64_t)(r0 + i) * nmu + c) * ss];
-  };
-  MView<double> LU{sw + L.lu * ss, (int64_t)nmax * ss, ss};
-  MView<double> X{sw + L.x * ss, (int64_t)nmax * ss, ss};
-  for (int i = 0; i < n; ++i)
-    for (int j = 0; j < n; ++j) LU(i, j) = row(0, i, cols[j]);
-  const double det = lu_factor<double>(LU, n, piv);
-  for (int i = 0; i < n; ++i)
-    for (int j = 0; j < n; ++j) X(i, j) = i == j ? 1.0 : 0.0;
-  lu_solve<double>(LU, n, piv, X.c(), X, n);
-  for (int i = 0; i < n; ++i) {
-    double g[3] = {0.0, 0.0, 0.0};
+  const MView<double> LU{k.cp + (int64_t)(S.lu + s * nmax * nmax) * k.cs, (int64_t)nmax * k.cs, k.cs};
+  const MView<double> V{k.cp + (int64_t)(S.ginv + s * nmax * nmax) * k.cs, (int64_t)nmax * k.cs, k.cs};
+  int piv[QMC_MAX_NSPIN], cols[QMC_MAX_NSPIN];
+  if (oth)
+    for (int i = 0; i < n * nmu; ++i) k.C(S.gx + r0 * nmu + i) = 0.0;
+  for (int u = 0; u < d.ndet[s]; ++u) {
+    if (n == 0) {
+      dst[u * ds] = 1.0;
+      continue;
+    }
+    det_columns(d, s, u, cols);
+    for (int i = 0; i < n; ++i)
+      for (int j = 0; j < n; ++j) {
+        const int c = cols[j];
+        LU(i, j) = r0 + i == er ? k.H(S.phi + c) : k.C(S.ma + (r0 + i) * nmu + c);
+      }
+    const double det = lu_factor<double>(LU, n, piv);
+    dst[u * ds] = det;
+    if (!oth) continue;
+    double coef = 0.0;
+    for (int c = 0; c < d.ncfg; ++c)
+      if (__ldg(d.cfg_det[s] + c) == u)
+        coef = fma(__ldg(d.ci_weight + c), oth[__ldg(d.cfg_det[1 - s] + c) * os], coef);
+    if (coef == 0.0) continue;
+    for (int i = 0; i < n; ++i)
+      for (int j = 0; j < n; ++j) V(i, j) = i == j ? 1.0 : 0.0;
+    lu_solve<double>(LU, n, piv, V.c(), V, n);
     for (int j = 0; j < n; ++j) {
-      const double xv = X(j, i);
-#pragma unroll
-      for (int q = 0; q < 3; ++q) g[q] = fma(xv, row(q + 1, i, cols[j]), g[q]);
-    }
-#pragma unroll
-    for (int q = 0; q < 3; ++q) sw[(gd + (int64_t)i * 3 + q) * ss] = g[q];
-  }
-  return det;
-}
-
-// Electron-electron Pade pair of electrons i and j at the given coordinates:
-// adds w0 r / (1 + w r) to *u and w0 / (1 + w r)^2 (x_i - x_j) / r to g.
-__device__ __forceinline__ void pade_pair(double w0, double w, const double (&xi)[3],
-                                          const double (&xj)[3], double* u, double (&g)[3]) {
-  const double dx[3] = {xi[0] - xj[0], xi[1] - xj[1], xi[2] - xj[2]};
-  const double r = sqrt(dx[0] * dx[0] + dx[1] * dx[1] + dx[2] * dx[2]);
-  const double iu = 1.0 / (1.0 + w * r);
-  *u += w0 * r * iu;
-#pragma unroll
-  for (int q = 0; q < 3; ++q) g[q] += w0 * iu * iu * dx[q] / r;
-}
-
-// Sum over the CI configurations: returns Sigma = sum_k c_k D_k^up D_k^dn and
-// writes grad Sigma (the Jacobi traces weighted by each configuration) to
-// sw[(out + c) * ss]; the moved spin sm's determinants come from dvf / gdf
-// (sm < 0: none moved), the others from dv0 / gd0.
-__device__ inline double drift_slater(const qmc_wf_desc& d, const DriftLayout& L, double* sw,
-                                      int64_t ss, int sm, int64_t out) {
-  const int nc = 3 * d.nelec, nmax = d.nup > d.ndown ? d.nup : d.ndown;
-  auto S = [&](int64_t item) -> double& { return sw[item * ss]; };
-  for (int c = 0; c < nc; ++c) S(out + c) = 0.0;
-  double sigma = 0.0;
-  for (int k = 0; k < d.ncfg; ++k) {
-    const int uu = __ldg(d.cfg_det[0] + k), ud = __ldg(d.cfg_det[1] + k);
-    const int k0 = uu, k1 = d.ndet[0] + ud;
-    const double dv0 = S((sm == 0 ? L.dvf : L.dv0) + k0);
-    const double dv1 = S((sm == 1 ? L.dvf : L.dv0) + k1);
-    const double cd = __ldg(d.ci_weight + k) * dv0 * dv1;
-    sigma += cd;
-    for (int s = 0; s < 2; ++s) {
-      const int n = s ? d.ndown : d.nup, r0 = s ? d.nup : 0, kk = s ? k1 : k0;
-      const int64_t gd = (s == sm ? L.gdf : L.gd0) + (int64_t)kk * nmax * 3;
-      for (int i = 0; i < n; ++i)
-        for (int q = 0; q < 3; ++q)
-          S(out + 3 * (r0 + i) + q) = fma(cd, S(gd + i * 3 + q), S(out + 3 * (r0 + i) + q));
-    }
-  }
-  return sigma;
-}
-
-// Full evaluation at positions P (coordinate c at P[c * ps]): the MO rows and
-// their gradients into ma..mz, the spin determinants and their electron
-// gradients into dv0 / gd0, the Jastrow gradient into jg0, and
-// grad log psi = grad Sigma / Sigma + grad log J into sw[(out + c) * ss].
-// Returns Sigma; *logj = log J.
-__device__ inline double drift_full_eval(const qmc_wf_desc& d, const Tables<double>& t,
-                                         const DriftLayout& L, double* sw, int64_t ss,
-                                         const double* P, int64_t ps, int64_t out,
-                                         double* logj) {
-  const int ne = d.nelec, nmu = d.nmo_used, nc = 3 * ne;
-  const int nmax = d.nup > d.ndown ? d.nup : d.ndown;
-  auto S = [&](int64_t item) -> double& { return sw[item * ss]; };
-  auto xyz = [&](int e, double (&p)[3]) {
-    for (int q = 0; q < 3; ++q) p[q] = P[(3 * e + q) * ps];
-  };
-  for (int e = 0; e < ne; ++e) {
-    const int64_t dst[4] = {L.ma + (int64_t)e * nmu, L.mx + (int64_t)e * nmu,
-                            L.my + (int64_t)e * nmu, L.mz + (int64_t)e * nmu};
-    drift_rows(t, nmu, sw, ss, L.ao, P[3 * e * ps], P[(3 * e + 1) * ps], P[(3 * e + 2) * ps],
-               dst);
-  }
-  for (int s = 0; s < 2; ++s)
-    for (int u = 0; u < d.ndet[s]; ++u) {
-      const int k = (s ? d.ndet[0] : 0) + u;
-      S(L.dv0 + k) = drift_det(d, L, sw, ss, s, u, -1, L.gd0 + (int64_t)k * nmax * 3);
-    }
-  const double wj = d.use_jastrow ? __ldg(d.jastrow_w) : 0.0;
-  double lj = 0.0;
-  for (int i = 0; i < ne; ++i) {
-    double g[3] = {0.0, 0.0, 0.0}, pi[3];
-    xyz(i, pi);
-    double ui = 0.0;
-    if (d.use_jastrow_en) {
-      const EnTerms en = en_terms(d, pi[0], pi[1], pi[2]);
-      lj += en.u;
-      for (int q = 0; q < 3; ++q) g[q] += en.g[q];
-    }
-    if (d.use_jastrow) {
-      for (int j = 0; j < ne; ++j) {
-        if (j == i) continue;
-        double pj[3], uj = 0.0;
-        xyz(j, pj);
-        pade_pair(same_spin(d, i, j) ? 0.25 : 0.5, wj, pi, pj, &uj, g);
-        if (j > i) ui += uj;
+      const int c = cols[j];
+      for (int i = 0; i < n; ++i) {
+        double& g = k.C(S.gx + (r0 + i) * nmu + c);
+        g = fma(coef * det, V(j, i), g);
       }
     }
-    lj += ui;
-    for (int q = 0; q < 3; ++q) S(L.jg0 + 3 * i + q) = g[q];
   }
-  const double sigma = drift_slater(d, L, sw, ss, -1, out);
-  for (int c = 0; c < nc; ++c) S(out + c) = S(out + c) / sigma + S(L.jg0 + c);
-  *logj = lj;
-  return sigma;
 }
 
-__global__ void __launch_bounds__(kDriftTPB) drift_kernel(const qmc_wf_desc d,
-                                                          const qmc_drift_args a,
-                                                          double* __restrict__ scr, int64_t ss,
-                                                          double sd) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int ncol = round_up(d.nmo_used, 8);
-  const Tables<double> t = load_tables<double>(d, d.nmo_used, ncol, smem);
-  const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= a.nwalkers) return;
-  const int ne = d.nelec, nmu = d.nmo_used, nc = 3 * ne;
-  const DriftLayout L = drift_layout(d);
-  double* sw = scr + w;
-  auto S = [&](int64_t item) -> double& { return sw[item * ss]; };
-  double* xs = a.pos + w * nc;  // start positions (read-only until the end)
-  const double wj = d.use_jastrow ? __ldg(d.jastrow_w) : 0.0;
-  const double step = a.step_size;
-  auto xyz = [&](int e, double (&p)[3]) {
-    for (int q = 0; q < 3; ++q) p[q] = xs[3 * e + q];
-  };
-
+// Excitation mode: F(i, v) = d Sigma / d X of spin s at H(S.f + s nmax nv + i nv + v)
+// from X and the other spin's relative determinants.
+__device__ inline void drift_adjoint(const qmc_wf_desc& d, const DriftShape& S,
+                                     const DriftWork& k, int s, CView<double> X, const double* oth,
+                                     int64_t os) {
+  const int n = s ? d.ndown : d.nup, nv = d.max_orb[s] - n;
+  if (nv <= 0) return;
   const int nmax = d.nup > d.ndown ? d.nup : d.ndown;
-  // ---- start positions: MO rows, spin determinants, Jastrow, drift ----
-  double logj0, rhoi;
-  {
-    const double sigma = drift_full_eval(d, t, L, sw, ss, xs, 1, L.dri, &logj0);
-    const double psi = exp(logj0) * sigma;
-    rhoi = psi * psi;
-    if (rhoi == 0.0) {
-      // the reference's drift grad(rho) / (2 rho) is undefined where rho is
-      // zero (underflow included): every later transition kernel is NaN and
-      // every move of this walker is rejected
-      rhoi = 1e-16;
-      for (int c = 0; c < nc; ++c) S(L.dri + c) = nan("");
+  const int f0 = S.f + s * (S.dvf - S.f) / 2;
+  (void)nmax;
+  for (int i = 0; i < n * nv; ++i) k.H(f0 + i) = 0.0;
+  for (int c = 0; c < d.ncfg; ++c) {
+    const int* e = d.det_table[s] + 5 * __ldg(d.cfg_det[s] + c);
+    const int ord = __ldg(e);
+    if (ord == 0) continue;
+    const double cd = __ldg(d.ci_weight + c) * oth[__ldg(d.cfg_det[1 - s] + c) * os];
+    const int i0 = __ldg(e + 1);
+    if (ord == 1) {
+      k.H(f0 + i0) += cd;
+    } else {  // x = X0 X3 - X1 X2
+      const int i1 = __ldg(e + 2), i2 = __ldg(e + 3), i3 = __ldg(e + 4);
+      const double x0 = X(i0 / nv, i0 % nv), x1 = X(i1 / nv, i1 % nv), x2 = X(i2 / nv, i2 % nv),
+                   x3 = X(i3 / nv, i3 % nv);
+      k.H(f0 + i0) = fma(cd, x3, k.H(f0 + i0));
+      k.H(f0 + i3) = fma(cd, x0, k.H(f0 + i3));
+      k.H(f0 + i1) = fma(-cd, x2, k.H(f0 + i1));
+      k.H(f0 + i2) = fma(-cd, x1, k.H(f0 + i2));
     }
-    for (int c = 0; c < nc; ++c) S(L.xi + c) = xs[c];
   }
+}
+
+// MO values and gradients of electron e at the start positions (eight columns
+// at a time), and its Jastrow terms.
+__device__ inline void drift_start_rows(const qmc_wf_desc& d, const Tables<double>& t,
+                                        const DriftShape& S, const DriftWork& k, int e) {
+  const int nmu = d.nmo_used, ne = d.nelec;
+  const double x = k.H(S.xs + 3 * e), y = k.H(S.xs + 3 * e + 1), z = k.H(S.xs + 3 * e + 2);
+  for (int j0 = 0; j0 < nmu; j0 += 8) {
+    double m[4][8];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int jj = 0; jj < 8; ++jj) m[q][jj] = 0.0;
+    auto acc = [&](int a, const AOVal<double>& o) {
+      double wv[8];
+      load_w<8>(t.W + (int64_t)a * t.ncol + j0, wv);
+#pragma unroll
+      for (int jj = 0; jj < 8; ++jj) {
+        m[0][jj] = fma(o.v, wv[jj], m[0][jj]);
+        m[1][jj] = fma(o.gx, wv[jj], m[1][jj]);
+        m[2][jj] = fma(o.gy, wv[jj], m[2][jj]);
+        m[3][jj] = fma(o.gz, wv[jj], m[3][jj]);
+      }
+    };
+    for_each_ao_ep<double, true, decltype(acc), false>(t, XP<double>{x, 0.0}, XP<double>{y, 0.0},
+                                                       XP<double>{z, 0.0}, acc);
+#pragma unroll
+    for (int jj = 0; jj < 8; ++jj)
+      if (j0 + jj < nmu) {
+        k.C(S.ma + e * nmu + j0 + jj) = m[0][jj];
+        for (int q = 0; q < 3; ++q) k.C(S.mg + (3 * e + q) * nmu + j0 + jj) = m[q + 1][jj];
+      }
+  }
+  double u = 0.0, g[3] = {0.0, 0.0, 0.0}, uen = 0.0;
+  if (d.use_jastrow_en) {
+    const EnTerms en = en_terms(d, x, y, z);
+    u = uen = en.u;
+    for (int q = 0; q < 3; ++q) g[q] = en.g[q];
+  }
+  if (d.use_jastrow) {
+    const double w = __ldg(d.jastrow_w);
+    for (int j = 0; j < ne; ++j) {
+      if (j == e) continue;
+      const double dx = x - k.H(S.xs + 3 * j), dy = y - k.H(S.xs + 3 * j + 1),
+                   dz = z - k.H(S.xs + 3 * j + 2);
+      double uj;
+      const double c = pade_pair(same_spin(d, e, j) ? 0.25 : 0.5, w, dx, dy, dz, uj);
+      if (j > e) u += uj;
+      g[0] = fma(c, dx, g[0]);
+      g[1] = fma(c, dy, g[1]);
+      g[2] = fma(c, dz, g[2]);
+    }
+  }
+  k.C(S.ju + e) = u;
+  k.C(S.jen + e) = uen;
+  for (int q = 0; q < 3; ++q) k.C(S.jg0 + 3 * e + q) = g[q];
+}
+
+__global__ void __launch_bounds__(kGradThreads)
+    drift_kernel(const __grid_constant__ qmc_wf_desc d, const __grid_constant__ qmc_drift_args a,
+                 double* __restrict__ scr, int64_t ss, double sd,
+                 const __grid_constant__ DriftShape S) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const Tables<double> t = load_tables<double>(d, d.nmo_used, S.ncol, smem);
+  Tables<double> tl = t;  // W as limbs
+  int* const ecol = reinterpret_cast<int*>(smem + S.o_ecol);
+  {
+    double* const wl = reinterpret_cast<double*>(smem + S.o_wl);
+    for (int i = threadIdx.x; i < d.nao * S.ncol; i += blockDim.x) wl[i] = t.W[i];
+    __syncthreads();
+    fix_table(wl, d.nao, S.ncol, ecol);
+    tl.W = wl;
+  }
+  int2* const fix = reinterpret_cast<int2*>(smem + S.o_fix) + threadIdx.x;
+  const int tid = threadIdx.x, slot = tid / S.nwb, wl = tid - slot * S.nwb, ns = S.nslot;
+  const int64_t nw = a.nwalkers, w = (int64_t)blockIdx.x * S.nwb + wl;
+  const bool on = slot < ns, live = on && w < nw;
+  const int64_t ws = w < nw ? w : nw - 1;  // walkers past the last repeat it, storing nothing
+  DriftWork k;
+  if (S.o_hot >= 0) {
+    k.hp = reinterpret_cast<double*>(smem + S.o_hot) + wl;
+    k.hs = S.nwb;
+  } else {
+    k.hp = scr + (int64_t)S.cold * ss + w;
+    k.hs = ss;
+  }
+  k.cp = scr + w;
+  k.cs = ss;
+  const int ne = d.nelec, nmu = d.nmo_used, nc = 3 * ne;
+  const int nmax = d.nup > d.ndown ? d.nup : d.ndown;
+  const bool ex = d.det_mode == QMC_DET_EXPLICIT;
+  const double wj = d.use_jastrow ? __ldg(d.jastrow_w) : 0.0, step = a.step_size;
+  const int spin = slot & 1;  // of the determinant phases (slots 0 and 1)
+  auto nof = [&](int s) { return s ? d.ndown : d.nup; };
+  auto r0of = [&](int s) { return s ? d.nup : 0; };
+  auto nvof = [&](int s) { return ex ? 0 : d.max_orb[s] - nof(s); };
+  auto f0of = [&](int s) { return S.f + s * (S.dvf - S.f) / 2; };
+  auto dv0 = [&](int s) { return k.cp + (int64_t)(S.dv0 + (s ? d.ndet[0] : 0)) * k.cs; };
+  // X of the start: the virtual columns beside the LU
+  auto x0 = [&](int s) {
+    return CView<double>{k.cp + ((int64_t)S.lx + r0of(s) * nmu + nof(s)) * k.cs,
+                         (int64_t)nmu * k.cs, k.cs};
+  };
+  double* const pos = a.pos + ws * nc;
+  // this thread's AO groups of the moved electron: an even share of the AOs
+  int glo = 0, ghi = 0;
+  while (glo < t.ngroup && t.group_ao[glo] * ns < t.nao * slot) ++glo;
+  ghi = glo;
+  while (ghi < t.ngroup && t.group_ao[ghi] * ns < t.nao * (slot + 1)) ++ghi;
+
+  // ---- start positions ----
+  if (on)
+    for (int e = slot; e < ne; e += ns)
+      for (int q = 0; q < 3; ++q) k.H(S.xs + 3 * e + q) = pos[3 * e + q];
+  __syncthreads();
+  if (on)
+    for (int e = slot; e < ne; e += ns) drift_start_rows(d, t, S, k, e);
+  __syncthreads();
+  if (slot < 2) {
+    const int s = spin, n = nof(s);
+    double det = 1.0;
+    if (ex) {
+      drift_explicit(d, S, k, s, -1, dv0(s), k.cs, nullptr, 0);
+    } else if (n == 0) {
+      for (int u = 0; u < d.ndet[s]; ++u) dv0(s)[u * k.cs] = 1.0;
+    } else {
+      int piv[QMC_MAX_NSPIN];
+      const MView<double> M{k.cp + ((int64_t)S.lx + r0of(s) * nmu) * k.cs, (int64_t)nmu * k.cs, k.cs};
+      for (int i = 0; i < n; ++i)
+        for (int j = 0; j < d.max_orb[s]; ++j) M(i, j) = k.C(S.ma + (r0of(s) + i) * nmu + j);
+      det = lu_factor<double>(M, n, piv);
+      for (int i = 0; i < n; ++i) k.C(S.piv + r0of(s) + i) = (double)piv[i];
+      const int nv = nvof(s);
+      const MView<double> X{M.p + n * M.cs, M.rs, M.cs};
+      if (nv > 0) lu_solve<double>(M, n, piv, X.c(), X, nv);
+      excitation_values<double, double>(d, d.det_table[s], s, X.c(), nv > 0 ? nv : 1, dv0(s), k.cs);
+    }
+    k.H(S.val + DV_DET + s) = det;
+  }
+  __syncthreads();
+  // A^-1 by columns; F, or G in explicit mode
+  if (!ex && on)
+    for (int e = slot; e < ne; e += ns) {
+      const int s = e < d.nup ? 0 : 1, n = nof(s), r0 = r0of(s);
+      const MView<double> LU{k.cp + ((int64_t)S.lx + r0 * nmu) * k.cs, (int64_t)nmu * k.cs, k.cs};
+      const int y = S.inv + e * nmax;
+      int at = e - r0;  // where the row interchanges move the one
+      for (int r = 0; r < n; ++r) {
+        const int p = (int)k.C(S.piv + r0 + r);
+        at = at == r ? p : (at == p ? r : at);
+      }
+      for (int r = 0; r < n; ++r) {
+        double v = r == at ? 1.0 : 0.0;
+        for (int c = at; c < r; ++c) v = fma(-LU(r, c), k.C(y + c), v);
+        k.C(y + r) = v;
+      }
+      for (int r = n - 1; r >= 0; --r) {
+        double v = k.C(y + r);
+        for (int c = r + 1; c < n; ++c) v = fma(-LU(r, c), k.C(y + c), v);
+        k.C(y + r) = v * LU(r, r);
+      }
+    }
+  if (slot < 2) {
+    if (ex)
+      drift_explicit(d, S, k, spin, -1, dv0(spin), k.cs, dv0(1 - spin), k.cs);
+    else
+      drift_adjoint(d, S, k, spin, x0(spin), dv0(1 - spin), k.cs);
+    if (slot == 0) {
+      double sigma = 0.0;
+      for (int c = 0; c < d.ncfg; ++c)
+        sigma = fma(__ldg(d.ci_weight + c), dv0(0)[__ldg(d.cfg_det[0] + c) * k.cs] *
+                                                dv0(1)[__ldg(d.cfg_det[1] + c) * k.cs], sigma);
+      k.H(S.val + DV_SIGMA) = sigma;
+      k.H(S.val + DV_CUR) = 0.0;
+      k.H(S.val + DV_EACC) = -1.0;
+      k.H(S.val + DV_FLAG) = 0.0;
+    }
+  }
+  __syncthreads();
+  double rhoi = 0.0, logj0 = 0.0;
+  const double dd0 = k.H(S.val + DV_DET) * k.H(S.val + DV_DET + 1);
+  if (on) {
+    // the walker's threads all hold the start's density and log J
+    const double sigma = k.H(S.val + DV_SIGMA);
+    for (int e = 0; e < ne; ++e) logj0 += k.C(S.ju + e);
+    const double psi = jexp(logj0) * (dd0 * sigma);
+    rhoi = psi * psi;
+    // where rho is zero (underflow included) the reference's drift
+    // grad(rho) / (2 rho) is undefined: every later transition kernel is NaN and
+    // every move of this walker is rejected
+    const bool zero = rhoi == 0.0;
+    if (zero) rhoi = 1e-16;
+    const double is = zero ? nan("") : 1.0 / sigma;
+    for (int e = slot; e < ne; e += ns) {
+      const int s = e < d.nup ? 0 : 1, n = nof(s), nv = nvof(s), i = e - r0of(s);
+      double g[3] = {0.0, 0.0, 0.0};
+      const int mg = S.mg + 3 * e * nmu;
+      if (ex) {
+        for (int j = 0; j < nmu; ++j)
+          for (int q = 0; q < 3; ++q)
+            g[q] = fma(k.C(S.gx + e * nmu + j), k.C(mg + q * nmu + j), g[q]);
+      } else {
+        for (int q = 0; q < 3; ++q) {
+          const int row = mg + q * nmu, zr = S.zm + (3 * e + q) * nmu;
+          for (int v = 0; v < nv; ++v) {
+            double m = k.C(row + n + v);
+            for (int j = 0; j < n; ++j) m = fma(-x0(s)(j, v), k.C(row + j), m);
+            k.C(zr + n + v) = m;
+          }
+          for (int l = 0; l < n; ++l) {
+            double v = 0.0;
+            for (int j = 0; j < n; ++j)
+              v = fma(k.C(S.inv + (r0of(s) + l) * nmax + j), k.C(row + j), v);
+            k.C(zr + l) = v;
+          }
+          g[q] = sigma * k.C(zr + i);
+        }
+        for (int v = 0; v < nv; ++v) {
+          double f = 0.0;
+          for (int j = 0; j < n; ++j)
+            f = fma(k.C(S.inv + e * nmax + j), k.H(f0of(s) + j * nv + v), f);
+          for (int q = 0; q < 3; ++q) g[q] = fma(f, k.C(S.zm + (3 * e + q) * nmu + n + v), g[q]);
+        }
+      }
+      for (int q = 0; q < 3; ++q)
+        k.H(S.dr + 3 * e + q) = fma(g[q], is, k.C(S.jg0 + 3 * e + q));
+    }
+  }
+  __syncthreads();
 
   Rng rng{(uint32_t)a.seed, (uint32_t)(a.seed >> 32), (uint32_t)w, 0, 0};
   const bool replay = a.electron_index != nullptr;
   int nacc = 0, idecor = 0;
   int64_t isnap = 0;
   for (int istep = 0; istep < a.nstep; ++istep) {
-    // ---- draws: the moved electron, its noise, the acceptance uniform ----
+    // ---- draws, by every thread of the walker: the moved electron, its noise, the
+    // acceptance uniform ----
     int e;
     double eta[3], uacc;
     if (replay) {
-      const int64_t o = (int64_t)istep * a.nwalkers + w;
+      const int64_t o = (int64_t)istep * nw + ws;
       e = a.electron_index[o];
       for (int q = 0; q < 3; ++q) eta[q] = a.normals[o * 3 + q];
       uacc = a.uniforms[o];
@@ -280,87 +468,316 @@ __global__ void __launch_bounds__(kDriftTPB) drift_kernel(const qmc_wf_desc d,
       for (int q = 0; q < 3; ++q) eta[q] *= sd;
     }
     if (e < 0 || e >= ne) e = 0;  // replayed indices are checked by the host
+    const int cur = k.H(S.val + DV_CUR) != 0.0 ? 3 * ne : 0;
+    const int dri = S.dr + cur, drf = S.dr + 3 * ne - cur;
     // proposal: start positions with electron e at xs_e + (step drift_i(e) + eta)
     double pe[3], pe0[3];
-    xyz(e, pe0);
-    for (int q = 0; q < 3; ++q)
-      pe[q] = __dadd_rn(pe0[q], __dadd_rn(__dmul_rn(step, S(L.dri + 3 * e + q)), eta[q]));
+    for (int q = 0; q < 3; ++q) {
+      pe0[q] = k.H(S.xs + 3 * e + q);
+      pe[q] = __dadd_rn(pe0[q], __dadd_rn(__dmul_rn(step, k.H(dri + 3 * e + q)), eta[q]));
+    }
+    const int sm = e < d.nup ? 0 : 1, n = nof(sm), r0 = r0of(sm), l = e - r0, nv = nvof(sm);
 
-    // ---- psi and drift at the proposal ----
-    const int64_t nrd[4] = {L.nr, L.nr + nmu, L.nr + 2 * nmu, L.nr + 3 * nmu};
-    drift_rows(t, nmu, sw, ss, L.ao, pe[0], pe[1], pe[2], nrd);
-    const int sm = e < d.nup ? 0 : 1;
-    for (int u = 0; u < d.ndet[sm]; ++u) {
-      const int k = (sm ? d.ndet[0] : 0) + u;
-      S(L.dvf + k) = drift_det(d, L, sw, ss, sm, u, e, L.gdf + (int64_t)k * nmax * 3);
+    // ---- this thread's AO groups of the moved electron (partial MO row) and its
+    // electrons' pairs with it ----
+    double du = 0.0, ge[3] = {0.0, 0.0, 0.0};
+    if (on) {
+      ep_fixed_rows<false, false>(tl, ecol, nmu, pe[0], pe[1], pe[2], 0.0, 0.0, 0.0, 0.0, fix,
+                                  S.nthreads, &k.H(S.part + slot * nmu), nullptr, k.hs, glo, ghi);
+      if (d.use_jastrow_en && slot == e % ns) {
+        const EnTerms en = en_terms(d, pe[0], pe[1], pe[2]);
+        du = en.u - k.C(S.jen + e);
+        for (int q = 0; q < 3; ++q) ge[q] = en.g[q];
+      }
+      for (int j = slot; j < ne; j += ns) {
+        if (j == e) continue;
+        double gj[3];
+        for (int q = 0; q < 3; ++q) gj[q] = k.C(S.jg0 + 3 * j + q);
+        if (d.use_jastrow) {
+          // pair (j, e) at the proposal and at the start
+          const double w0 = same_spin(d, e, j) ? 0.25 : 0.5;
+          double d1[3], d0[3], u1, u0;
+          for (int q = 0; q < 3; ++q) {
+            const double xj = k.H(S.xs + 3 * j + q);
+            d1[q] = xj - pe[q];
+            d0[q] = xj - pe0[q];
+          }
+          const double c1 = pade_pair(w0, wj, d1[0], d1[1], d1[2], u1);
+          const double c0 = pade_pair(w0, wj, d0[0], d0[1], d0[2], u0);
+          du += u1 - u0;
+          for (int q = 0; q < 3; ++q) {
+            const double g1 = c1 * d1[q];
+            gj[q] += fma(-c0, d0[q], g1);
+            ge[q] -= g1;  // grad_e of the pair is minus grad_j
+          }
+        }
+        for (int q = 0; q < 3; ++q) k.H(S.gj + 3 * j + q) = gj[q];
+      }
     }
-    const double sigma = drift_slater(d, L, sw, ss, sm, L.drf);
-    // Jastrow: the pairs of e and its electron-nucleus terms change
-    double logj = logj0, ge[3] = {0.0, 0.0, 0.0};
-    if (d.use_jastrow_en) {
-      const EnTerms en1 = en_terms(d, pe[0], pe[1], pe[2]);
-      const EnTerms en0 = en_terms(d, pe0[0], pe0[1], pe0[2]);
-      logj += en1.u - en0.u;
-      for (int q = 0; q < 3; ++q) ge[q] += en1.g[q];
+    __syncthreads();
+    if (on)
+      for (int j = slot; j < nmu; j += ns) {
+        double v = 0.0;
+        for (int p = 0; p < ns; ++p) v += k.H(S.part + p * nmu + j);
+        k.H(S.phi + j) = v;
+      }
+    __syncthreads();
+    // ---- determinants at the proposal ----
+    if (!ex) {
+      if (on)
+        for (int i = slot; i < n + nv; i += ns) {
+          if (i < n) {  // r_i = phi' A^-1 e_i
+            double v = 0.0;
+            for (int j = 0; j < n; ++j) v = fma(k.H(S.phi + j), k.C(S.inv + (r0 + i) * nmax + j), v);
+            k.H(S.r + i) = v;
+          } else {  // t_v = phi'_virt - phi' X
+            double v = k.H(S.phi + i);
+            for (int j = 0; j < n; ++j) v = fma(-k.H(S.phi + j), x0(sm)(j, i - n), v);
+            k.H(S.t + i - n) = v;
+          }
+        }
+      __syncthreads();
+      if (slot == 0) {
+        const double q = 1.0 / k.H(S.r + l);
+        for (int v = 0; v < nv; ++v) {
+          const double tq = k.H(S.t + v) * q;
+          k.H(S.t + v) = tq;
+          for (int j = 0; j < n; ++j)
+            k.H(S.xp + j * nv + v) = fma(k.C(S.inv + e * nmax + j), tq, x0(sm)(j, v));
+        }
+        k.H(S.val + DV_Q) = q;
+        const CView<double> X{k.hp + (int64_t)S.xp * k.hs, (int64_t)nv * k.hs, k.hs};
+        excitation_values<double, double>(d, d.det_table[sm], sm, X, nv > 0 ? nv : 1,
+                                          k.hp + (int64_t)S.dvf * k.hs, k.hs);
+        bool sum = false;
+        for (int u = 0; u < d.ndet[sm]; ++u)
+          sum |= __double2hiint(fabs(k.H(S.dvf + u))) > __double2hiint(kGradRatio);
+        k.H(S.val + DV_FLAG) = sum ? 1.0 : 0.0;
+        if (sum)
+          drift_explicit(d, S, k, sm, e, k.hp + (int64_t)S.dvf * k.hs, k.hs, dv0(1 - sm), k.cs);
+      }
+    } else if (slot == 0) {
+      drift_explicit(d, S, k, sm, e, k.hp + (int64_t)S.dvf * k.hs, k.hs, dv0(1 - sm), k.cs);
     }
-    for (int j = 0; j < ne; ++j) {
-      double gj[3];
-      for (int q = 0; q < 3; ++q) gj[q] = S(L.jg0 + 3 * j + q);
-      if (j != e && d.use_jastrow) {
-        double pj[3], u1 = 0.0, u0 = 0.0, g1[3] = {0.0, 0.0, 0.0}, g0[3] = {0.0, 0.0, 0.0};
-        xyz(j, pj);
-        const double w0 = same_spin(d, e, j) ? 0.25 : 0.5;
-        pade_pair(w0, wj, pj, pe, &u1, g1);   // pair (j, e) at the proposal
-        pade_pair(w0, wj, pj, pe0, &u0, g0);  // and at the start
-        logj += u1 - u0;
-        for (int q = 0; q < 3; ++q) {
-          gj[q] += g1[q] - g0[q];
-          ge[q] -= g1[q];  // grad_e of the pair is minus grad_j
+    __syncthreads();
+    const double* const dvf = k.hp + (int64_t)S.dvf * k.hs;
+    if (slot < 2) {
+      const CView<double> X{k.hp + (int64_t)S.xp * k.hs, (int64_t)nv * k.hs, k.hs};
+      if (!ex) {
+        // slot 0: the moved spin (unless it has G already), slot 1: the other
+        const int s = slot == 0 ? sm : 1 - sm;
+        if (s == sm) {
+          if (k.H(S.val + DV_FLAG) == 0.0) drift_adjoint(d, S, k, s, X, dv0(1 - s), k.cs);
+        } else
+          drift_adjoint(d, S, k, s, x0(s), dvf, k.hs);
+      } else if (slot == 1) {
+        // the moved spin's G from the determinants phase; the other's now
+        drift_explicit(d, S, k, 1 - sm, -1, k.hp + (int64_t)S.part * k.hs, 0, dvf, k.hs);
+      }
+      if (slot == (ex ? 0 : 1)) {
+        double sigma = 0.0;
+        for (int c = 0; c < d.ncfg; ++c)
+          sigma = fma(__ldg(d.ci_weight + c), dvf[__ldg(d.cfg_det[sm] + c) * k.hs] *
+                                                  dv0(1 - sm)[__ldg(d.cfg_det[1 - sm] + c) * k.cs],
+                      sigma);
+        k.H(S.val + DV_SIGMA) = sigma;
+      }
+    }
+    __syncthreads();
+    // ---- gradients: the moved electron's G row, this thread's electrons, then this
+    // thread's AO groups of the moved electron ----
+    const double sigma = k.H(S.val + DV_SIGMA), is = 1.0 / sigma;
+    if (on) {
+      const bool sum = ex || k.H(S.val + DV_FLAG) != 0.0;  // the moved spin's G is in gx
+      const double q0 = ex ? 0.0 : k.H(S.val + DV_Q);
+      double a1 = 0.0, a2 = 0.0;
+      const int eacc = (int)k.H(S.val + DV_EACC);
+      for (int i = slot; i < ne; i += ns) {
+        if (i != e) {
+          const int s = i < d.nup ? 0 : 1, mg = S.mg + 3 * i * nmu, ns_ = nof(s), nvs = nvof(s);
+          double g[3] = {0.0, 0.0, 0.0};
+          const bool moved = s == sm;
+          if (ex || (sum && moved)) {
+            for (int j = 0; j < nmu; ++j)
+              for (int q = 0; q < 3; ++q)
+                g[q] = fma(k.C(S.gx + i * nmu + j), k.C(mg + q * nmu + j), g[q]);
+          } else {
+            const double ri = moved ? q0 * k.H(S.r + i - r0) : 0.0;
+            const int zr = S.zm + 3 * i * nmu;
+            double z[3];
+            for (int q = 0; q < 3; ++q) {
+              z[q] = moved ? k.C(zr + q * nmu + l) : 0.0;
+              g[q] = sigma * fma(-ri, z[q], k.C(zr + q * nmu + i - r0of(s)));
+            }
+            for (int v = 0; v < nvs; ++v) {
+              double f = 0.0;
+              for (int j = 0; j < ns_; ++j) {
+                const double yi = k.C(S.inv + i * nmax + j);
+                f = fma(moved ? fma(-ri, k.C(S.inv + e * nmax + j), yi) : yi,
+                        k.H(f0of(s) + j * nvs + v), f);
+              }
+              const double tv = moved ? k.H(S.t + v) : 0.0;
+              for (int q = 0; q < 3; ++q)
+                g[q] = fma(fma(-tv, z[q], k.C(zr + q * nmu + ns_ + v)), f, g[q]);
+            }
+          }
+          for (int q = 0; q < 3; ++q) {
+            const int c = 3 * i + q;
+            const double df = fma(g[q], is, k.H(S.gj + c));
+            k.H(drf + c) = df;
+            // the proposal has the start's position here; the accepted one unless i moved
+            double dx = 0.0;
+            if (i == eacc) dx = __dsub_rn(k.H(S.val + DV_XACC + q), k.H(S.xs + c));
+            const double t1 = __dsub_rn(dx, __dmul_rn(df, step));
+            const double t2 = __dsub_rn(-dx, __dmul_rn(k.H(dri + c), step));
+            a1 = fma(t1, t1, a1);
+            a2 = fma(t2, t2, a2);
+          }
         }
       }
-      if (j != e)
-        for (int q = 0; q < 3; ++q) S(L.drf + 3 * j + q) = S(L.drf + 3 * j + q) / sigma + gj[q];
-    }
-    for (int q = 0; q < 3; ++q) S(L.drf + 3 * e + q) = S(L.drf + 3 * e + q) / sigma + ge[q];
-    const double psif = exp(logj) * sigma;
-    double rhof = psif * psif;
-    const bool defined = rhof != 0.0;  // else the reference's drift is NaN: rejected
-    if (rhof == 0.0) rhof = 1e-16;
-
-    // ---- transition kernels and the decision ----
-    double a1 = 0.0, a2 = 0.0;
-    for (int c = 0; c < nc; ++c) {
-      const int ec = c / 3;
-      const double xf = ec == e ? pe[c - 3 * e] : xs[c];
-      const double xi = S(L.xi + c);
-      const double t1 = __dsub_rn(__dsub_rn(xi, xf), __dmul_rn(S(L.drf + c), step));
-      const double t2 = __dsub_rn(__dsub_rn(xf, xi), __dmul_rn(S(L.dri + c), step));
-      a1 = fma(t1, t1, a1);
-      a2 = fma(t2, t2, a2);
-    }
-    const double tif = exp(-0.5 * sqrt(a1) / step), tfi = exp(-0.5 * sqrt(a2) / step);
-    double p = (tif * rhof) / (tfi * rhoi);
-    if (p > 1.0) p = 1.0;
-    if (defined && p - uacc >= 0.0) {
-      ++nacc;
-      for (int c = 0; c < nc; ++c) {
-        const int ec = c / 3;
-        S(L.xi + c) = ec == e ? pe[c - 3 * e] : xs[c];
-        S(L.dri + c) = S(L.drf + c);
+      const int red = S.red + slot * kDriftRed;
+      k.H(red) = du;
+      k.H(red + 1) = a1;
+      k.H(red + 2) = a2;
+      for (int q = 0; q < 3; ++q) k.H(red + 3 + q) = ge[q];
+      double ga[3] = {0.0, 0.0, 0.0};
+      const int norb = ex ? nmu : d.max_orb[sm];
+      for (int j0 = 0; j0 < norb; j0 += 8) {
+        double G[8];
+        if (sum) {
+#pragma unroll
+          for (int jj = 0; jj < 8; ++jj)
+            G[jj] = j0 + jj < norb ? k.C(S.gx + e * nmu + j0 + jj) : 0.0;
+        } else {
+          // y' = A^-1 e_l / r_l; G_virt = y' F, G_occ = Sigma y' - G_virt X'^T
+#pragma unroll
+          for (int jj = 0; jj < 8; ++jj)
+            G[jj] = j0 + jj < n ? sigma * (k.C(S.inv + e * nmax + j0 + jj) * q0) : 0.0;
+          for (int v = 0; v < nv; ++v) {
+            double f = 0.0;
+            for (int j = 0; j < n; ++j)
+              f = fma(k.C(S.inv + e * nmax + j) * q0, k.H(f0of(sm) + j * nv + v), f);
+#pragma unroll
+            for (int jj = 0; jj < 8; ++jj) {
+              if (j0 + jj < n) G[jj] = fma(-f, k.H(S.xp + (j0 + jj) * nv + v), G[jj]);
+              if (j0 + jj == n + v) G[jj] = f;
+            }
+          }
+        }
+        FixG<8> fg;
+        fg.set(G, ecol + j0);
+        auto h = [&](int ao) {
+          return fg.dot(reinterpret_cast<const int2*>(tl.W) + (int64_t)ao * t.ncol + j0);
+        };
+        grad_ao_backward(t, pe[0], pe[1], pe[2], h, ga, glo, ghi);
       }
-      rhoi = rhof;
+      for (int q = 0; q < 3; ++q) k.H(S.part + slot * 3 + q) = ga[q];
     }
+    __syncthreads();
+    // ---- transition kernels and the decision ----
+    if (slot == 0) {
+      double logj = logj0, a1 = 0.0, a2 = 0.0, g[3] = {0.0, 0.0, 0.0}, gu[3] = {0.0, 0.0, 0.0};
+      for (int p = 0; p < ns; ++p) {
+        const int red = S.red + p * kDriftRed;
+        logj += k.H(red);
+        a1 += k.H(red + 1);
+        a2 += k.H(red + 2);
+        for (int q = 0; q < 3; ++q) {
+          gu[q] += k.H(red + 3 + q);
+          g[q] += k.H(S.part + p * 3 + q);
+        }
+      }
+      const int eacc = (int)k.H(S.val + DV_EACC);
+      for (int q = 0; q < 3; ++q) {
+        const int c = 3 * e + q;
+        const double df = fma(g[q], is, gu[q]);
+        k.H(drf + c) = df;
+        const double xi = e == eacc ? k.H(S.val + DV_XACC + q) : pe0[q];
+        const double t1 = __dsub_rn(__dsub_rn(xi, pe[q]), __dmul_rn(df, step));
+        const double t2 = __dsub_rn(__dsub_rn(pe[q], xi), __dmul_rn(k.H(dri + c), step));
+        a1 = fma(t1, t1, a1);
+        a2 = fma(t2, t2, a2);
+      }
+      // the determinants that Sigma is relative to
+      const double det = ex ? 1.0
+                            : (k.H(S.val + DV_FLAG) != 0.0 ? k.H(S.val + DV_DET + 1 - sm)
+                                                           : dd0 * k.H(S.r + l));
+      const double psif = jexp(logj) * (det * sigma);
+      double rhof = psif * psif;
+      const bool defined = rhof != 0.0;  // else the reference's drift is NaN: rejected
+      if (rhof == 0.0) rhof = 1e-16;
+      const double hs = 0.5 / step;
+      const double tif = rexp(-hs * psqrt(a1)), tfi = rexp(-hs * psqrt(a2));
+      double p = (tif * rhof) / (tfi * rhoi);
+      if (p > 1.0) p = 1.0;
+      if (defined && p - uacc >= 0.0) {
+        ++nacc;
+        rhoi = rhof;
+        k.H(S.val + DV_CUR) = cur ? 0.0 : 1.0;
+        k.H(S.val + DV_EACC) = (double)e;
+        for (int q = 0; q < 3; ++q) k.H(S.val + DV_XACC + q) = pe[q];
+      }
+    }
+    __syncthreads();
     if (istep >= a.ntherm) {
       if (idecor % a.ndecor == 0 && a.samples && isnap < a.nsnap) {
-        double* o = a.samples + (isnap * a.nwalkers + w) * nc;
-        for (int c = 0; c < nc; ++c) o[c] = S(L.xi + c);
+        if (live) {
+          const int eacc = (int)k.H(S.val + DV_EACC);
+          double* o = a.samples + (isnap * nw + w) * nc;
+          for (int i = slot; i < ne; i += ns)
+            for (int q = 0; q < 3; ++q)
+              o[3 * i + q] = i == eacc ? k.H(S.val + DV_XACC + q) : k.H(S.xs + 3 * i + q);
+        }
         ++isnap;
       }
       ++idecor;
     }
   }
-  for (int c = 0; c < nc; ++c) xs[c] = S(L.xi + c);
-  if (a.accepted) a.accepted[w] += nacc;
+  if (live && slot == 0) {
+    const int eacc = (int)k.H(S.val + DV_EACC);
+    if (eacc >= 0)
+      for (int q = 0; q < 3; ++q) pos[3 * eacc + q] = k.H(S.val + DV_XACC + q);
+    if (a.accepted) a.accepted[w] += nacc;
+  }
+}
+
+// Launch plan, by the rule of grad_plan: the least warp work on the busiest SM
+// (a walker's work is shared evenly by its threads, up to one per electron).
+static DriftShape drift_plan(const qmc_wf_desc& d, int64_t nw) {
+  int dev = 0, nsm = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  DriftShape best = drift_shape(d, 1, 2, true);
+  best.smem = -1;
+  double best_cost = 0.0;
+  const int most = d.nelec > 16 ? 16 : (d.nelec < 2 ? 2 : d.nelec);
+  for (int in_smem = 1; in_smem >= 0 && best.smem < 0; --in_smem)
+    for (int nwb = 32; nwb >= 4; nwb /= 2)
+      for (int nslot = 2; nslot <= most; ++nslot) {
+        const DriftShape s = drift_shape(d, nwb, nslot, in_smem == 1);
+        if (s.nthreads > kGradThreads || s.smem > 227 * 1024) continue;
+        if (prepare_smem(drift_kernel, s.smem) != QMC_OK) continue;
+        int occ = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, drift_kernel, s.nthreads, s.smem) !=
+                cudaSuccess ||
+            occ < 1) {
+          cudaGetLastError();
+          continue;
+        }
+        const int64_t blocks = (nw + nwb - 1) / nwb, on_sm = (blocks + nsm - 1) / nsm;
+        const int64_t rounds = (on_sm + occ - 1) / occ;
+        const int64_t walkers = (rounds == 1 ? on_sm : rounds * occ) * nwb;
+        const double warps = (double)(on_sm < occ ? on_sm : occ) * s.nthreads / 32.0;
+        const int per = (d.nelec + nslot - 1) / nslot;
+        double cost = (double)walkers * per * s.nthreads / ((double)nwb * d.nelec);
+        if (warps < 12.0) cost *= sqrt(12.0 / warps);
+        cost *= 1.0 + 0.1 * (nwb < 32 ? 32.0 / nwb : 1.0);
+        if (best.smem < 0 || cost < 0.999 * best_cost) {
+          best = s;
+          best_cost = cost;
+        }
+      }
+  return best;
 }
 
 }  // namespace qmc
@@ -371,7 +788,8 @@ extern "C" {
 
 int64_t qmc_drift_scratch_bytes(const qmc_wf_desc* d, int64_t nw) {
   if (check_desc(d) != QMC_OK || nw < 0) return -1;
-  return drift_layout(*d).total * pad_walkers(nw) * (int64_t)sizeof(double);
+  const DriftShape s = drift_shape(*d, 1, 16, false);  // the most threads per walker
+  return (int64_t)(s.cold + s.hot) * pad_walkers(nw) * (int64_t)sizeof(double);
 }
 
 int qmc_drift_run(const qmc_wf_desc* d0, const qmc_drift_args* a, void* scratch,
@@ -392,13 +810,12 @@ int qmc_drift_run(const qmc_wf_desc* d0, const qmc_drift_args* a, void* scratch,
   if (!a->pos || !scratch) return QMC_ERR_ARG;
   if (a->nsnap > 0 && !a->samples) return QMC_ERR_ARG;
   if (scratch_bytes < qmc_drift_scratch_bytes(d, a->nwalkers)) return QMC_ERR_SCRATCH;
-  const int ncol = round_up(d->nmo_used, 8);
-  const int64_t smem = tables_smem_bytes<double>(*d, ncol);
-  if ((st = prepare_smem(drift_kernel, smem))) return st;
-  const dim3 grid((unsigned)((a->nwalkers + kDriftTPB - 1) / kDriftTPB));
+  const DriftShape S = drift_plan(*d, a->nwalkers);
+  if (S.smem < 0) return QMC_ERR_SHAPE;
+  if ((st = prepare_smem(drift_kernel, S.smem))) return st;
   const double sd = sqrt(sqrt(a->step_size));  // covariance sqrt(step) I
-  drift_kernel<<<grid, kDriftTPB, smem, (cudaStream_t)stream>>>(
-      dd, *a, (double*)scratch, pad_walkers(a->nwalkers), sd);
+  drift_kernel<<<(unsigned)((a->nwalkers + S.nwb - 1) / S.nwb), S.nthreads, S.smem,
+                 (cudaStream_t)stream>>>(dd, *a, (double*)scratch, pad_walkers(a->nwalkers), sd, S);
   return launch_status();
 }
 
