@@ -46,10 +46,14 @@ class Loss(nn.Module):
         """Returns (loss, local energies) of the batch ``pos``."""
         with self.get_grad_mode(no_grad):
             eloc = self.wf.local_energy(pos)
-            keep = self.get_clipping_mask(eloc)
-            factor = self.get_sampling_weights(pos, deactivate_weight)
-            weighted = factor * eloc
-            return self.loss_fn(weighted[keep]), eloc
+            weighted = eloc
+            if self.use_weight and not deactivate_weight:
+                weighted = self.get_sampling_weights(pos, deactivate_weight) * eloc
+            # without clipping every entry is kept: no mask is indexed (its gather, and
+            # the sort and scatter of the gather's gradient, cost more than the kernels of
+            # a small molecule: LiH, 8192 walkers, a gradient step)
+            kept = weighted[self.get_clipping_mask(eloc)] if self.clip else weighted.reshape(-1)
+            return self.loss_fn(kept), eloc
 
     @staticmethod
     def get_grad_mode(no_grad):

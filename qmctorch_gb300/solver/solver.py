@@ -148,8 +148,9 @@ class SolverBase:
                 eloc = torch.cat(chunks)
             # mean, variance and sampling error: compensated device reduction
             e, s, err = rt.walker_stats(eloc)
-        log.info("  Energy   : %f +/- %f", e.item(), err.item())
-        log.info("  Variance : %f", s.item())
+        if log.isEnabledFor(logging.INFO):  # each value read waits for the GPU
+            log.info("  Energy   : %f +/- %f", e.item(), err.item())
+            log.info("  Variance : %f", s.item())
         log.info("  Size     : %d", len(eloc))
         obs = SimpleNamespace(pos=pos, local_energy=eloc, energy=e, variance=s, error=err)
         self._dump(obs, hdf5_group, "single_point")
@@ -338,13 +339,12 @@ class Solver(SolverBase):
         with torch.no_grad():
             eloc = self.wf.local_energy(lpos)
         psi = self.wf(lpos)
-        norm = 1.0 / len(psi)
-        weight = eloc.clone()
-        weight -= torch.mean(eloc)
-        weight /= psi.clone()
-        weight *= 2.0 * norm
-        clip_mask = self.loss.get_clipping_mask(eloc)
-        psi = psi[clip_mask]
-        weight = weight[clip_mask]
+        mean = torch.mean(eloc)
+        weight = (eloc - mean) / psi.detach()
+        weight *= 2.0 * (1.0 / len(psi))
+        if self.loss.clip:
+            clip_mask = self.loss.get_clipping_mask(eloc)
+            psi = psi[clip_mask]
+            weight = weight[clip_mask]
         psi.backward(weight)
-        return torch.mean(eloc), eloc
+        return mean, eloc

@@ -274,18 +274,18 @@ class SlaterJastrow(WaveFunction):
         nmu = self.highest_occ_mo
         lib = _lib.lib()
         g = rt.dev64(gout, device)
-        g_exp = torch.zeros(bt.nentries, dtype=rt.F64, device=device)
-        g_W = torch.zeros((self.ao.norb, nmu), dtype=rt.F64, device=device)
-        g_w = torch.zeros(2, dtype=rt.F64, device=device)  # e-e and e-n Pade weights
-        g_ci = torch.zeros(self.nci, dtype=rt.F64, device=device)
+        # one zeroed buffer: exponents, W, the e-e and e-n Pade weights, CI weights
+        sizes = (bt.nentries, self.ao.norb * nmu, 2, self.nci)
+        g_exp, g_W, g_w, g_ci = torch.zeros(sum(sizes), dtype=rt.F64, device=device).split(sizes)
         scr = rt.scratch(getattr(lib, scratch_fn)(call.ref, nb), device)
         _lib.check(getattr(lib, fn)(call.ref, rt.ptr(x), nb, rt.ptr(g), rt.ptr(bt.t["w_entry"]),
                                     bt.nentries, rt.ptr(g_exp), rt.ptr(g_W), nmu, rt.ptr(g_w),
                                     rt.ptr(g_ci), rt.ptr(scr), scr.numel(), rt.stream_handle()),
                    fn)
         mod = self.mo.mo_modifier
-        g_mod = torch.zeros(mod.shape, dtype=rt.F64, device=device)
-        g_mod[:, :nmu] = g_W * rt.dev64(self.mo.mo_scf, device)[:, :nmu]
+        g_mod = g_W.view(self.ao.norb, nmu) * rt.dev64(self.mo.mo_scf, device)[:, :nmu]
+        if nmu < mod.shape[1]:  # the unused orbitals' gradient is zero
+            g_mod = torch.nn.functional.pad(g_mod, (0, mod.shape[1] - nmu))
         cast = lambda t, p: t.to(device=p.device, dtype=p.dtype).reshape(p.shape)  # noqa: E731
         jw, jwn = self._jastrow_weights()
         return (cast(g_exp, self.ao.bas_exp), cast(g_mod, mod), cast(g_w[:1], jw),
