@@ -72,8 +72,9 @@ inline SweepShape sweep_shape(const qmc_wf_desc& d, int nww, int jc) {
     s.o_v[k] = q;
     q += align16((int64_t)s.n[k] * s.ld[k] * rs);
   }
+  // the rebuild's work matrix and a move's rows are never in use together: one place
   s.o_m = q;
-  q += align16((int64_t)s.nmax * s.ldm * rs);
+  const int64_t q_m = q + align16((int64_t)s.nmax * s.ldm * rs);
   s.o_ao = q;
   q += align16((int64_t)pad4(d.nao) * rs);
   s.o_phi = q;
@@ -86,6 +87,7 @@ inline SweepShape sweep_shape(const qmc_wf_desc& d, int nww, int jc) {
   q += align16((int64_t)d.ngprim * rs);
   s.o_d = q;
   q += align16((int64_t)d.natom * 4 * rs);
+  if (q < q_m) q = q_m;
   s.warp_bytes = q;
   s.smem = s.o_warp + (int64_t)nww * q;
   return s;
@@ -314,9 +316,15 @@ __device__ __forceinline__ R warp_sum(R v) {
 }
 
 // One block = nww walker chains, one warp each; the warps share only the
-// basis / MO tables and never wait for one another after loading them.
+// basis / MO tables and never wait for one another after loading them. Bound by
+// latency (a chain of short warp-wide phases), so the warps resident on an SM
+// decide, and those by shared memory: one block with one copy of the tables and as
+// many warps as its registers allow (80 and 128 a thread). C6H6 mixed: 22 warps per
+// SM, 7.4 KB each, against 2 x 8; 16384 walkers, two sweeps: 6.21 -> 6.05 ms.
+template <typename R>
+constexpr int kSweepWarps = kMixed<R> ? 24 : 16;
 template <typename R, int JC>
-__global__ void __launch_bounds__(256, kMixed<R> ? 3 : 2)
+__global__ void __launch_bounds__(32 * kSweepWarps<R>, 1)
     sweep_kernel(const qmc_wf_desc d, const qmc_metropolis_args a, const SweepShape S) {
   extern __shared__ __align__(16) unsigned char smem[];
   const Tables<R> t = load_tables<R>(d, S.nmax, S.ncol, smem + S.o_tab);
@@ -342,7 +350,6 @@ __global__ void __launch_bounds__(256, kMixed<R> ? 3 : 2)
   R* D = reinterpret_cast<R*>(base + S.o_d);
   const int ne = d.nelec, nc = 3 * ne, nup = d.nup;
   for (int i = lane; i < nc; i += 32) P[i] = split_xp<R>(a.pos[w * nc + i]);
-  for (int i = d.nao + lane; i < pad4(d.nao); i += 32) AO[i] = (R)0;
   __syncwarp();
 
   auto rebuild = [&]() {
@@ -352,6 +359,8 @@ __global__ void __launch_bounds__(256, kMixed<R> ? 3 : 2)
       lane_slater_rows<R, JC>(t, P, s * nup, n, M, S.ldm, lane);
       warp_inverse<R>(M, S.ldm, s ? V1 : V0, s ? S.ld[1] : S.ld[0], n, lane);
     }
+    for (int i = d.nao + lane; i < pad4(d.nao); i += 32) AO[i] = (R)0;  // M lay over it
+    __syncwarp();
   };
   rebuild();
 
@@ -489,24 +498,33 @@ __global__ void __launch_bounds__(256, kMixed<R> ? 3 : 2)
   if (lane == 0 && a.accepted) a.accepted[w] += nacc;
 }
 
-// Walkers per block: the count that keeps the most warps resident per SM
-// (CUDA occupancy calculator), preferring larger blocks on ties.
+// Walkers per block: the fewest rounds of resident warps over the walkers that fall
+// to an SM, then the fewest walkers on the busiest SM, then the larger block (one
+// copy of the tables for more warps).
 template <typename R, int JC>
 static int launch_sweep(const qmc_wf_desc* d, const qmc_metropolis_args* a, cudaStream_t st) {
   SweepShape best = sweep_shape<R>(*d, 1, JC);
-  int best_warps = 0;
-  for (int nww = 8; nww >= 1; nww /= 2) {
+  int best_warps = 0, dev = 0, nsm = 1;
+  int64_t best_rounds = 0, best_load = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  for (int nww = kSweepWarps<R>; nww >= 1; --nww) {
     const SweepShape s = sweep_shape<R>(*d, nww, JC);
-    if (s.smem > 200 * 1024) continue;
+    if (s.smem > 227 * 1024) continue;
     if (prepare_smem(sweep_kernel<R, JC>, s.smem) != QMC_OK) continue;
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sweep_kernel<R, JC>, s.nthreads, s.smem) !=
-        cudaSuccess) {
+            cudaSuccess ||
+        occ < 1) {
       cudaGetLastError();
       continue;
     }
-    if (occ * nww > best_warps) {
+    const int64_t blocks = (a->nwalkers + nww - 1) / nww, on_sm = (blocks + nsm - 1) / nsm;
+    const int64_t rounds = (on_sm + occ - 1) / occ, load = on_sm * nww;
+    if (best_warps == 0 || rounds < best_rounds || (rounds == best_rounds && load < best_load)) {
       best_warps = occ * nww;
+      best_rounds = rounds;
+      best_load = load;
       best = s;
     }
   }
