@@ -69,40 +69,48 @@ __device__ inline void fix_table(double* W, int nao, int ncol, int* ecol) {
   __syncthreads();
 }
 
-// Adds the chunk's products to row[j * rs], j < n (first: sets). v: the thread's
-// AO values as limbs at v[i * vs], i < na, their biased exponent bound E; Wl: limbs of
-// the first AO's row of W.
+// The chunk's products of eight columns. v: the thread's AO values as limbs at
+// v[i * vs], i < na; Wl: limbs of the first AO's row of W at the first column (rows of
+// ncol).
+__device__ __forceinline__ void fix_products(const int2* v, int vs, int na, const int2* Wl,
+                                             int ncol, int64_t (&hh)[8], int64_t (&mid)[8],
+                                             int64_t (&ll)[8]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) hh[j] = mid[j] = ll[j] = 0;
+  for (int i = 0; i < na; ++i) {
+    const int2 a = v[i * vs];
+    if ((a.x | a.y) == 0) continue;
+    const int4* w = reinterpret_cast<const int4*>(Wl + i * ncol);
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      const int4 q = w[j >> 1];
+      hh[j] += (int64_t)a.x * q.x;
+      mid[j] += (int64_t)a.x * q.y;
+      mid[j] += (int64_t)a.y * q.x;
+      ll[j] += (int64_t)a.y * q.y;
+      hh[j + 1] += (int64_t)a.x * q.z;
+      mid[j + 1] += (int64_t)a.x * q.w;
+      mid[j + 1] += (int64_t)a.y * q.z;
+      ll[j + 1] += (int64_t)a.y * q.w;
+    }
+  }
+}
+// An entry's value from its products; E: biased exponent bound of the AO values, e:
+// the column's exponent. An AO or a coefficient that is not finite makes it NaN.
+__device__ __forceinline__ double fix_entry(int64_t hh, int64_t mid, int64_t ll, int E, int e) {
+  return (E >= 0x7FF || e == kFixNaN) ? nan("") : fix_value(hh, mid, ll, E - 1022 + e);
+}
+// Adds the chunk's products of n columns to row[j * rs] (first: sets).
 __device__ __forceinline__ void fix_rows(const int2* v, int vs, int na, int E, const int2* Wl,
                                          int ncol, const int* ecol, int n, double* row,
                                          int64_t rs, bool first) {
   for (int j0 = 0; j0 < n; j0 += 8) {
     int64_t hh[8], mid[8], ll[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) hh[j] = mid[j] = ll[j] = 0;
-    for (int i = 0; i < na; ++i) {
-      const int2 a = v[i * vs];
-      if ((a.x | a.y) == 0) continue;
-      const int4* w = reinterpret_cast<const int4*>(Wl + i * ncol + j0);
-#pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        const int4 q = w[j >> 1];
-        hh[j] += (int64_t)a.x * q.x;
-        mid[j] += (int64_t)a.x * q.y;
-        mid[j] += (int64_t)a.y * q.x;
-        ll[j] += (int64_t)a.y * q.y;
-        hh[j + 1] += (int64_t)a.x * q.z;
-        mid[j + 1] += (int64_t)a.x * q.w;
-        mid[j + 1] += (int64_t)a.y * q.z;
-        ll[j + 1] += (int64_t)a.y * q.w;
-      }
-    }
+    fix_products(v, vs, na, Wl + j0, ncol, hh, mid, ll);
 #pragma unroll
     for (int j = 0; j < 8; ++j)
       if (j0 + j < n) {
-        const int e = ecol[j0 + j];
-        // an AO or a coefficient that is not finite makes the entry NaN
-        const double x = (E >= 0x7FF || e == kFixNaN) ? nan("")
-                                                      : fix_value(hh[j], mid[j], ll[j], E - 1022 + e);
+        const double x = fix_entry(hh[j], mid[j], ll[j], E, ecol[j0 + j]);
         double& r = row[(j0 + j) * rs];
         r = first ? x : r + x;
       }

@@ -66,7 +66,7 @@ static inline int64_t scratch_slot_bytes(const qmc_wf_desc* d, int kind) {
   if (kind == 1) {
     qmc_wf_desc dd = *d;
     dd.precision = QMC_PREC_FP64;
-    const int64_t t = scratch_layout(dd, 1).bytes_per_slot;
+    const int64_t t = scratch_layout(dd).bytes_per_slot;
     if (t > b) b = t;
   }
   return b;
