@@ -46,6 +46,16 @@ __host__ __device__ inline bool el_regs(const qmc_wf_desc& d) {
   return true;
 }
 
+// The local energy of one ground-state determinant per spin beyond the register
+// path: only the diagonal of A^-1 B is needed, and the cooperative phase
+// (ep_det_el_coop) keeps the factors in shared memory.
+constexpr int kCoopMinN = 6;
+__host__ __device__ inline bool el_diagonal(const qmc_wf_desc& d) {
+  return d.det_mode == QMC_DET_EXCITATION && d.ndet[0] == 1 && d.ndet[1] == 1 &&
+         d.max_orb[0] == d.nup && d.max_orb[1] == d.ndown && !el_regs(d) &&
+         (d.nup > d.ndown ? d.nup : d.ndown) >= kCoopMinN;
+}
+
 __host__ __device__ inline EPLayout ep_layout(const qmc_wf_desc& d, int kind) {
   EPLayout L;
   const bool mixed = d.precision == QMC_PREC_MIXED;
@@ -108,7 +118,9 @@ struct EPShape {
   int64_t smem;  // dynamic shared memory bytes
   int64_t o_tab, o_pos, o_pnew, o_mo, o_bk, o_jrow, o_vrow, o_dref, o_psi, o_f, o_kin, o_v,
       o_iel, o_acc;
-  int64_t o_fix, o_ecol;  // FP64: the threads' AO values as limbs, W's column exponents
+  int64_t o_bd;         // FP32 local energy: gradient part of the kinetic rows
+  int64_t o_lu;         // the factors of el_diagonal's cooperative phase, or -1: work arrays
+  int64_t o_fix, o_ecol;  // the threads' AO values (FP64: as limbs); FP64: W's column exponents
   int64_t o_det;  // determinant-phase work arrays of the block's walkers, or -1: HBM scratch
 };
 
@@ -138,6 +150,8 @@ __host__ __device__ inline EPShape ep_shape(const qmc_wf_desc& d, int kind, int 
   o += align8(d.nelec * nmu * nwb * (int64_t)sizeof(R));
   s.o_bk = o;
   if (kind == 1) o += align8(d.nelec * nmu * nwb * (int64_t)sizeof(R));
+  s.o_bd = o;
+  if (kind == 1 && kMixed<R>) o += align8(d.nelec * nmu * nwb * (int64_t)sizeof(R));
   s.o_jrow = o;
   o += align8((int64_t)d.nelec * nwb * 8);
   s.o_vrow = o;
@@ -156,12 +170,18 @@ __host__ __device__ inline EPShape ep_shape(const qmc_wf_desc& d, int kind, int 
   o += align8(nwb * 4);
   s.o_acc = o;
   o += align8(nwb * 4);
-  s.o_fix = s.o_ecol = o;
-  if (!kMixed<R>) {
-    o += (int64_t)s.nthreads * (kind == 1 ? 2 * kFixElAOs : kFixAOs) * 8;
-    s.o_ecol = o;
-    o += align8((int64_t)s.ncol * 4);
+  s.o_lu = -1;
+  if (kind == 1 && el_diagonal(d) && nslot >= 4) {
+    const int64_t nmax = d.nup > d.ndown ? d.nup : d.ndown;
+    s.o_lu = o;
+    o += align8(2 * nmax * nmax * nwb * (int64_t)sizeof(R));
   }
+  s.o_fix = o;
+  if (kind == 1 || !kMixed<R>)
+    o += align8((int64_t)s.nthreads * (kind == 1 ? (kMixed<R> ? 3 : 2) * kFixElAOs : kFixAOs) *
+                (int64_t)sizeof(R));
+  s.o_ecol = o;
+  if (!kMixed<R>) o += align8((int64_t)s.ncol * 4);
   // the determinant phase works in shared memory when the block's arrays are
   // small (the psi / Metropolis kernels of small molecules), else in HBM scratch
   const int64_t det_bytes = (int64_t)nwb * ep_layout(d, kind == 1 ? 1 : 0).bytes_per_slot;
@@ -509,6 +529,90 @@ __device__ inline void ep_fixed_rows(const Tables<double>& t, const int* ecol, i
     for (int j = 0; j < nmu; ++j) bk[j * rs] = -0.5 * fma(jl, mo[j * rs], bk[j * rs]);
 }
 
+// Two FP32 multiply-adds in one instruction, each rounded as fmaf.
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  return ((uint64_t)__float_as_uint(hi) << 32) | __float_as_uint(lo);
+}
+__device__ __forceinline__ float unpack2(uint64_t v, int i) {
+  return __uint_as_float((unsigned)(v >> (32 * i)));
+}
+
+// FP32 MO and kinetic rows of an electron (as ep_fixed_rows<true>): the AO values
+// of a chunk of groups go to the thread's slots in shared memory, and one loop over
+// them multiplies with W, two columns per instruction, eight columns at a time; with
+// the accumulators in registers instead, every eight columns took a pass over all
+// AOs and their derivatives. Every entry sums its AOs in their order. With the
+// factors in shared memory (el_diagonal), C6H6, 16384 walkers: 4.57 -> 2.84 ms. (The
+// psi kernels keep their columns in registers: through the slots the H2O Metropolis
+// kernel took 3.64 instead of 3.15 ms.)
+__device__ inline void ep_float_rows(const Tables<float>& t, int nmu, XP<float> ex, XP<float> ey,
+                                     XP<float> ez, float gx, float gy, float gz, float jl, float* v,
+                                     int vs, float* mo, float* bk, float* bd, int64_t rs) {
+  constexpr int kCap = kFixElAOs;
+  for (int g0 = 0; g0 < t.ngroup;) {
+    const int a0 = t.group_ao[g0];
+    int g1 = g0 + 1;
+    while (g1 < t.ngroup && t.group_ao[g1 + 1] - a0 <= kCap) ++g1;
+    const int na = t.group_ao[g1] - a0;
+    auto acc = [&](int a, const AOVal<float>& o) {
+      v[(a - a0) * vs] = o.v;
+      v[(kCap + a - a0) * vs] = 2.0f * (gx * o.gx + gy * o.gy + gz * o.gz);
+      v[(2 * kCap + a - a0) * vs] = o.lap;
+    };
+    for_each_ao_ep<float, true>(t, ex, ey, ez, acc, g0, g1);
+    for (int j0 = 0; j0 < nmu; j0 += 8) {
+      uint64_t m[4], b[4], l[4];  // value, gradient and Laplacian sums
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int j = j0 + 2 * q;
+        const bool lo = g0 > 0 && j < nmu, hi = g0 > 0 && j + 1 < nmu;
+        m[q] = pack2(lo ? mo[j * rs] : 0.0f, hi ? mo[(j + 1) * rs] : 0.0f);
+        b[q] = pack2(lo ? bd[j * rs] : 0.0f, hi ? bd[(j + 1) * rs] : 0.0f);
+        l[q] = pack2(lo ? bk[j * rs] : 0.0f, hi ? bk[(j + 1) * rs] : 0.0f);
+      }
+      const float* W = t.W + (int64_t)a0 * t.ncol + j0;
+#pragma unroll 2
+      for (int i = 0; i < na; ++i) {
+        const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(W + i * t.ncol);
+        const ulonglong2 w1 = *reinterpret_cast<const ulonglong2*>(W + i * t.ncol + 4);
+        const float x = v[i * vs], y = v[(kCap + i) * vs], z = v[(2 * kCap + i) * vs];
+        const uint64_t xx = pack2(x, x), yy = pack2(y, y), zz = pack2(z, z);
+        m[0] = fma2(xx, w0.x, m[0]);
+        m[1] = fma2(xx, w0.y, m[1]);
+        m[2] = fma2(xx, w1.x, m[2]);
+        m[3] = fma2(xx, w1.y, m[3]);
+        b[0] = fma2(yy, w0.x, b[0]);
+        b[1] = fma2(yy, w0.y, b[1]);
+        b[2] = fma2(yy, w1.x, b[2]);
+        b[3] = fma2(yy, w1.y, b[3]);
+        l[0] = fma2(zz, w0.x, l[0]);
+        l[1] = fma2(zz, w0.y, l[1]);
+        l[2] = fma2(zz, w1.x, l[2]);
+        l[3] = fma2(zz, w1.y, l[3]);
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (j0 + q < nmu) {
+          const float x = unpack2(m[q / 2], q % 2), y = unpack2(b[q / 2], q % 2),
+                      z = unpack2(l[q / 2], q % 2);
+          mo[(j0 + q) * rs] = x;
+          if (g1 == t.ngroup) {
+            bk[(j0 + q) * rs] = -0.5f * (z + y + jl * x);
+          } else {
+            bd[(j0 + q) * rs] = y;
+            bk[(j0 + q) * rs] = z;
+          }
+        }
+    }
+    g0 = g1;
+  }
+}
+
 // JC consecutive W values with vector loads (rows are 16-byte aligned and
 // padded to a multiple of JC).
 template <int JC>
@@ -541,7 +645,7 @@ __device__ __forceinline__ void load_w(const double* p, double (&w)[JC]) {
 template <typename R, int JC, bool KIN>
 __device__ inline void ep_electron(const qmc_wf_desc& d, const Tables<R>& t, const XP<R>* pw,
                                    int e, R* mo, R* bk, int nwb, double* jrow, double* vrow,
-                                   int2* fix, int fix_stride, const int* ecol) {
+                                   R* fix, int fix_stride, const int* ecol, R* bd) {
   const int ne = d.nelec, nmu = d.nmo_used;
   const XP<R> ex = pw[3 * e], ey = pw[3 * e + 1], ez = pw[3 * e + 2];
   R gx = (R)0, gy = (R)0, gz = (R)0, jl = (R)0;
@@ -607,32 +711,31 @@ __device__ inline void ep_electron(const qmc_wf_desc& d, const Tables<R>& t, con
   R* mrow = mo + (int64_t)e * nmu * cs;
   R* brow = KIN ? bk + (int64_t)e * nmu * cs : nullptr;
   if constexpr (!kMixed<R>) {
-    ep_fixed_rows<KIN, true>(t, ecol, nmu, ex.h, ey.h, ez.h, gx, gy, gz, jl, fix, fix_stride, mrow,
+    ep_fixed_rows<KIN, true>(t, ecol, nmu, ex.h, ey.h, ez.h, gx, gy, gz, jl,
+                             reinterpret_cast<int2*>(fix), fix_stride, mrow,
                              brow, cs, 0, t.ngroup);
+  } else if constexpr (KIN) {
+    ep_float_rows(t, nmu, ex, ey, ez, gx, gy, gz, jl, fix, fix_stride, mrow, brow,
+                  bd + (int64_t)e * nmu * cs, cs);
   } else {
     for (int j0 = 0; j0 < nmu; j0 += JC) {
-      R a0[JC], ab[JC];
+      uint64_t m[JC / 2];
 #pragma unroll
-      for (int jj = 0; jj < JC; ++jj) a0[jj] = ab[jj] = (R)0;
+      for (int q = 0; q < JC / 2; ++q) m[q] = 0;
       auto acc = [&](int a, const AOVal<R>& o) {
-        R wv[JC];
-        load_w<JC>(t.W + (int64_t)a * t.ncol + j0, wv);
-        R b = (R)0;
-        if (KIN) b = o.lap + (R)2 * (gx * o.gx + gy * o.gy + gz * o.gz);
+        const ulonglong2* w = reinterpret_cast<const ulonglong2*>(t.W + (int64_t)a * t.ncol + j0);
+        const uint64_t v = pack2(o.v, o.v);
 #pragma unroll
-        for (int jj = 0; jj < JC; ++jj) {
-          a0[jj] = fma(o.v, wv[jj], a0[jj]);
-          if (KIN) ab[jj] = fma(b, wv[jj], ab[jj]);
+        for (int q = 0; q < JC / 4; ++q) {
+          const ulonglong2 x = w[q];
+          m[2 * q] = fma2(v, x.x, m[2 * q]);
+          m[2 * q + 1] = fma2(v, x.y, m[2 * q + 1]);
         }
       };
       for_each_ao_ep<R, KIN>(t, ex, ey, ez, acc);
 #pragma unroll
-      for (int jj = 0; jj < JC; ++jj) {
-        if (j0 + jj < nmu) {
-          mrow[(j0 + jj) * cs] = a0[jj];
-          if (KIN) brow[(j0 + jj) * cs] = (R)(-0.5) * (ab[jj] + jl * a0[jj]);
-        }
-      }
+      for (int jj = 0; jj < JC; ++jj)
+        if (j0 + jj < nmu) mrow[(j0 + jj) * cs] = unpack2(m[jj / 2], jj % 2);
     }
   }
 }
@@ -648,12 +751,10 @@ __device__ inline void ep_electron(const qmc_wf_desc& d, const Tables<R>& t, con
 // A^-1 A_virt is written back (in place over the virtual columns) for the
 // excitation determinants. Returns det(A) in FP64 (product of the pivots).
 constexpr int kRegNV = 2;
-// largest n of the register path: 5 under the 64-register bound of the FP32
-// kernels (more spills); the FP64 kernel keeps the shared-memory LU (its
-// register file is full with the FP64 electron phase: the register path
-// measured 17 % slower there)
+// Largest n of the register path (5: the FP32 kernels' 64-register bound spills more
+// beyond; FP64: 2.85 -> 1.50 ms against 1.67 ms through shared memory).
 template <typename R>
-constexpr int kRegMaxN = kMixed<R> ? 5 : 0;
+constexpr int kRegMaxN = 5;
 
 template <typename R, int N>
 __device__ inline double lu_solve_regs(R* rows, int64_t rs, int64_t cs, int nv) {
@@ -692,7 +793,7 @@ __device__ inline double lu_solve_regs(R* rows, int64_t rs, int64_t cs, int nv) 
     if (p != k) det = -det;
     const R akk = a[k][k];
     det *= to_f64(akk);
-    const R inv = akk != (R)0 ? (R)1 / akk : (R)0;
+    const R inv = akk != (R)0 ? prcp(akk) : (R)0;
     a[k][k] = inv;
 #pragma unroll
     for (int i = k + 1; i < N; ++i) {
@@ -848,7 +949,7 @@ __device__ inline void el_channel_regs(const qmc_wf_desc& d, int spin, CView<R> 
     if (p != k) det = -det;
     const R akk = a[k][k];
     det *= to_f64(akk);
-    const R inv = akk != (R)0 ? (R)1 / akk : (R)0;
+    const R inv = akk != (R)0 ? prcp(akk) : (R)0;
     a[k][k] = inv;
 #pragma unroll
     for (int i = k + 1; i < N; ++i) {
@@ -974,7 +1075,7 @@ __device__ inline bool el_channel_regs_n(const qmc_wf_desc& d, int spin, CView<R
   }
 }
 
-template <typename R, bool OP>
+template <typename R, bool OP, bool PLAIN = false>
 __device__ inline void ep_det(const qmc_wf_desc& d, const EPLayout& L, unsigned char* scr,
                               int64_t ss, int64_t w, int spin, R* mo_s, const R* bk_s, int wl,
                               int nwb, double* dref, const int* dtab) {
@@ -1020,7 +1121,7 @@ __device__ inline void ep_det(const qmc_wf_desc& d, const EPLayout& L, unsigned 
     wk.X = MView<R>{rows + n * cs, rs, cs};
   }
   double* ov = OP ? rptr<double>(scr, L.ov, ss, w) + (spin ? d.ndet[0] * ss : 0) : nullptr;
-  spin_channel<R, OP, T>(d, spin, mo, bk, wk, SpinOut<T>{dv, ov, ss, &dref[spin * nwb + wl]});
+  spin_channel<R, OP, T, PLAIN>(d, spin, mo, bk, wk, SpinOut<T>{dv, ov, ss, &dref[spin * nwb + wl]});
 }
 
 // Block-cooperative LU of the psi / Metropolis determinant phase for spin
@@ -1035,8 +1136,6 @@ __device__ inline void ep_det(const qmc_wf_desc& d, const EPLayout& L, unsigned 
 // thread the one-thread path runs on (slot = spin, tid < 2 nwb): it keeps the
 // pivots and det, and then solves the virtual columns and forms the
 // excitation values as ep_det does. Three block barriers per elimination step.
-constexpr int kCoopMinN = 6;
-
 template <typename R>
 __host__ __device__ inline bool coop_lu_applies(const qmc_wf_desc& d, int nslot) {
   if (d.det_mode != QMC_DET_EXCITATION || nslot < 4) return false;
@@ -1166,10 +1265,36 @@ __device__ inline void ep_det_coop(const qmc_wf_desc& d, const EPLayout& L, unsi
 // solves are independent, so the values are spin_channel's bitwise); the
 // channel's first thread then forms the determinant ratios and traces
 // (excitation_tail). Two more block barriers.
+// x = A^-1 b for one right-hand side b(i) (b may read x: it is copied first), by
+// lu_solve's operations; only the elements from `last` on are final.
+template <typename R, typename B>
+__device__ inline void column_solve(MView<R> LU, int n, const int* piv, const B& b, R* x, int last) {
+  for (int i = 0; i < n; ++i) x[i] = b(i);
+  for (int k = 0; k < n; ++k) {
+    const int p = piv[k];
+    if (p != k) {
+      const R t = x[k];
+      x[k] = x[p];
+      x[p] = t;
+    }
+  }
+  for (int i = 1; i < n; ++i) {
+    R s = x[i];
+    for (int k = 0; k < i; ++k) s = fma(-LU(i, k), x[k], s);
+    x[i] = s;
+  }
+  for (int i = n - 1; i >= last; --i) {
+    R s = x[i];
+    for (int k = i + 1; k < n; ++k) s = fma(-LU(i, k), x[k], s);
+    x[i] = s * LU(i, i);
+  }
+}
+
 template <typename R>
 __device__ inline void ep_det_el_coop(const qmc_wf_desc& d, const EPLayout& L,
                                       unsigned char* dbase, int64_t dss, int64_t w0, int64_t nw,
-                                      bool dsm, R* MO, R* BK, int nwb, int nslot, double* DREF) {
+                                      bool dsm, R* MO, R* BK, R* LUS, int nwb, int nslot,
+                                      double* DREF) {
   constexpr bool REFINE = kMixed<R>;
   const CoopRole c(nwb, nslot);
   const int spin = c.spin, wl = c.wl, r = c.r, nt = c.nt;
@@ -1190,12 +1315,48 @@ __device__ inline void ep_det_el_coop(const qmc_wf_desc& d, const EPLayout& L,
   wk.rc = MView<R>{rptr<R>(dbase, L.rc[spin], dss, w), dss, dss};
   wk.X64 = MView<double>{rptr<double>(dbase, L.x64[spin], dss, w), vm * dss, dss};
   wk.Y64 = MView<double>{rptr<double>(dbase, L.y64[spin], dss, w), (int64_t)L.omax * dss, dss};
+  if (LUS)  // el_diagonal
+    wk.LU = MView<R>{LUS + (int64_t)spin * L.nmax * L.nmax * nwb + wl, (int64_t)L.nmax * nwb, nwb};
   if (c.on)
     for (int i = r; i < n; i += nt)
       for (int j = 0; j < n; ++j) wk.LU(i, j) = mo(i, j);
   __syncthreads();  // the occupied block copied
   int piv[QMC_MAX_NSPIN];
   const double det = coop_lu_steps<R>(wk.LU.p, wk.LU.rs, wk.LU.cs, n, nmax, c.on, r, nt, piv);
+  if (LUS) {
+    // one determinant: column j's solution and residual stay with its thread, and
+    // only element j of the refined solution, its term of the trace, is kept (the
+    // last substitution ends there)
+    if (c.on && n > 0) {
+      R xl[QMC_MAX_NSPIN], rl[QMC_MAX_NSPIN];
+      for (int j = r; j < n; j += nt) {
+        column_solve<R>(wk.LU, n, piv, [&](int i) { return bk(i, j); }, xl, REFINE ? 0 : j);
+        double y = (double)xl[j];
+        if (REFINE) {
+          for (int i = 0; i < n; ++i)
+            rl[i] = residual_ds<R>(bk(i, j), n, [&](int k, R& a, R& x) {
+              a = mo(i, k);
+              x = xl[k];
+            });
+          column_solve<R>(wk.LU, n, piv, [&](int i) { return rl[i]; }, rl, j);
+          y = (double)xl[j] + (double)rl[j];
+        }
+        if (REFINE)
+          wk.Y64(j, 0) = y;
+        else
+          wk.Y(j, 0) = (R)y;
+      }
+    }
+    __syncthreads();  // every trace term written
+    if (threadIdx.x < 2 * nwb && w0 + wl < nw) {
+      double base = 0.0;
+      for (int j = 0; j < n; ++j) base += REFINE ? wk.Y64(j, 0) : (double)wk.Y(j, 0);
+      rptr<double>(dbase, L.dv, dss, w)[(spin ? d.ndet[0] : 0) * dss] = 1.0;
+      rptr<double>(dbase, L.ov, dss, w)[(spin ? d.ndet[0] : 0) * dss] = base;
+      DREF[spin * nwb + wl] = n == 0 ? 1.0 : det;
+    }
+    return;
+  }
   if (c.on && n > 0) {
     // this thread's columns; a private residual column for the refinements
     R rcl[QMC_MAX_NSPIN];
@@ -1244,6 +1405,40 @@ __device__ inline Tables<R> ep_tables(const qmc_wf_desc& d, const EPShape& S, un
   return t;
 }
 
+// Combine phase of walker wl: CI sum, Jastrow factor, energies.
+template <typename R, bool KIN>
+__device__ inline void ep_combine(const qmc_wf_desc& d, const Tables<R>& t, const EPPtrs& p,
+                                  unsigned char* dbase, int64_t dss, bool dsm, int64_t w0, int wl) {
+  using T = typename std::conditional<KIN, double, R>::type;
+  const EPShape& S = p.S;
+  const int nwb = S.nwb;
+  const double* JR = reinterpret_cast<const double*>(p.smem + S.o_jrow);
+  const double* VR = reinterpret_cast<const double*>(p.smem + S.o_vrow);
+  const double* DREF = reinterpret_cast<const double*>(p.smem + S.o_dref);
+  const EPLayout L = ep_layout(d, KIN ? 1 : 0);
+  double kin = 0.0;
+  const int64_t slot = dsm ? wl : w0 + wl;
+  const T* dv = rptr<T>(dbase, L.dv, dss, slot);
+  const double* ov = KIN ? rptr<double>(dbase, L.ov, dss, slot) : nullptr;
+  const double psid = ci_combine<T, KIN, T>(d, dv, ov, dss, DREF[wl], DREF[nwb + wl], &kin,
+                                             (!KIN && kMixed<R>) ? (const T*)t.ciw : nullptr);
+  double logj = 0.0, v = 0.0;
+  for (int e = 0; e < d.nelec; ++e) {
+    logj += JR[e * nwb + wl];
+    if (KIN) v += VR[e * nwb + wl];
+  }
+  double jf = 1.0;
+  if (d.use_jastrow || d.use_jastrow_en) {
+    if constexpr (kMixed<R> && !KIN) jf = exp_mixed(logj);
+    else jf = jexp(logj);
+  }
+  reinterpret_cast<double*>(p.smem + S.o_psi)[wl] = psid * jf;
+  if (KIN) {
+    reinterpret_cast<double*>(p.smem + S.o_kin)[wl] = kin;
+    reinterpret_cast<double*>(p.smem + S.o_v)[wl] = v;
+  }
+}
+
 // Evaluate psi (and, with KIN, the kinetic energy and potentials) for the
 // block's walkers at split positions `pbuf` (shared memory, [nwb][3 nelec]).
 // Results in shared memory: psi[wl], and with KIN kin[wl], v[wl] (V_en + V_ee),
@@ -1282,8 +1477,9 @@ __device__ inline void ep_eval(const qmc_wf_desc& d, const Tables<R>& t, const E
       if (e < ne)
         ep_electron<R, JC, KIN>(d, t, pbuf + wl * S.pstride, e, MO + wl, BK + wl, nwb,
                                 &JR[e * nwb + wl], &VR[e * nwb + wl],
-                                reinterpret_cast<int2*>(p.smem + S.o_fix) + tid, S.nthreads,
-                                reinterpret_cast<const int*>(p.smem + S.o_ecol));
+                                reinterpret_cast<R*>(p.smem + S.o_fix) + tid, S.nthreads,
+                                reinterpret_cast<const int*>(p.smem + S.o_ecol),
+                                reinterpret_cast<R*>(p.smem + S.o_bd) + wl);
     }
   }
   __syncthreads();
@@ -1294,7 +1490,7 @@ __device__ inline void ep_eval(const qmc_wf_desc& d, const Tables<R>& t, const E
   if (!KIN && coop_lu_applies<R>(d, S.nslot)) {
     ep_det_coop<R, R>(d, L, dbase, dss, w0, nw, dsm, MO, nwb, S.nslot, DREF);
   } else if (KIN && ELCOOP && coop_el_applies<R>(d, S.nslot)) {
-    if constexpr (KIN && ELCOOP) ep_det_el_coop<R>(d, L, dbase, dss, w0, nw, dsm, MO, BK, nwb, S.nslot, DREF);
+    if constexpr (KIN && ELCOOP) ep_det_el_coop<R>(d, L, dbase, dss, w0, nw, dsm, MO, BK, S.o_lu >= 0 ? reinterpret_cast<R*>(p.smem + S.o_lu) : nullptr, nwb, S.nslot, DREF);
   } else if (tid < 2 * nwb) {
     const int spin = tid / nwb, wl = tid - spin * nwb;
     if (w0 + wl < nw)
@@ -1302,32 +1498,173 @@ __device__ inline void ep_eval(const qmc_wf_desc& d, const Tables<R>& t, const E
                      d.det_table[spin]);
   }
   __syncthreads();
-  if (tid < nwb && w0 + tid < nw) {
-    using T = typename std::conditional<KIN, double, R>::type;
-    const int wl = tid;
-    const int64_t w = w0 + wl;
-    double kin = 0.0;
-    const int64_t slot = dsm ? wl : w;
-    const T* dv = rptr<T>(dbase, L.dv, dss, slot);
-    const double* ov = KIN ? rptr<double>(dbase, L.ov, dss, slot) : nullptr;
-    const double psid = ci_combine<T, KIN, T>(d, dv, ov, dss, DREF[wl], DREF[nwb + wl], &kin,
-                                               (!KIN && kMixed<R>) ? (const T*)t.ciw : nullptr);
-    double logj = 0.0, v = 0.0;
-    for (int e = 0; e < ne; ++e) {
-      logj += JR[e * nwb + wl];
-      if (KIN) v += VR[e * nwb + wl];
+  if (tid < nwb && w0 + tid < nw) ep_combine<R, KIN>(d, t, p, dbase, dss, dsm, w0, tid);
+}
+
+// ---------------------------------------------------------------------------
+// FP64 local energy: walkers next to a node of the ground determinant
+// ---------------------------------------------------------------------------
+// Where an excitation ratio (a determinant relative to the ground one) exceeds
+// kPlainRatio, the 2 x 2 minors of the double excitations cancel, and the local
+// energy amplifies the last bits of everything before it by about the ratio's
+// square (H2O: up to 1e-4 Ha, one walker in some 1e5). Such a walker is evaluated
+// again with the plain sequence of FP64 instructions (FP64-pipe exp, square root,
+// reciprocal, multiply-adds in AO order, IEEE pivots), whatever the other walkers of
+// its block do: its energy does not depend on the fixed-point functions' last bits.
+// H2O: about one block of 16 walkers in 100 does the second evaluation.
+constexpr double kPlainRatio = 4096.0;
+
+// All AOs of one electron with derivatives.
+template <typename F>
+__device__ inline void plain_aos(const Tables<double>& t, double x, double y, double z, F& f) {
+  for (int g = 0; g < t.ngroup; ++g) {
+    const int A = t.group_atom[g];
+    const double dx = x - t.atom_p[3 * A].h, dy = y - t.atom_p[3 * A + 1].h,
+                 dz = z - t.atom_p[3 * A + 2].h;
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    if (t.radial != QMC_RADIAL_GTO) {
+      group_sto<double, true>(t, g, dx, dy, dz, r2, f);
+      continue;
     }
-    double jf = 1.0;
-    if (d.use_jastrow || d.use_jastrow_en) {
-      if constexpr (kMixed<R> && !KIN) jf = exp_mixed(logj);
-      else jf = jexp(logj);
-    }
-    PSI[wl] = psid * jf;
-    if (KIN) {
-      KINV[wl] = kin;
-      V[wl] = v;
+    const int np = t.group_prim[g + 1] - t.group_prim[g];
+    for (int a = t.group_ao[g]; a < t.group_ao[g + 1]; ++a) {
+      double G0 = 0.0, G1 = 0.0, G2 = 0.0;
+      for (int p = 0; p < np; ++p) {
+        const int wi = t.ao_wofs[a] + p;
+        const double al = t.walpha[wi];
+        if (al * r2 > (double)kRadialCut) continue;
+        const double e0 = exp_tang(-al * r2), e1 = al * e0, e2 = al * e1, w = t.wd[wi];
+        G0 = fma(w, e0, G0);
+        G1 = fma(w, e1, G1);
+        G2 = fma(w, e2, G2);
+      }
+      const int kx = t.ao_k[3 * a], ky = t.ao_k[3 * a + 1], kz = t.ao_k[3 * a + 2];
+      const double px = pk0(dx, kx), py = pk0(dy, ky), pz = pk0(dz, kz);
+      const double qx = pk1(dx, kx) * py * pz, qy = px * pk1(dy, ky) * pz,
+                   qz = px * py * pk1(dz, kz);
+      const double lapP = pk2(dx, kx) * py * pz + px * pk2(dy, ky) * pz + px * py * pk2(dz, kz);
+      f(a, ao_from<double, true>(px * py * pz, qx, qy, qz, lapP, kx + ky + kz, dx, dy, dz, r2, G0,
+                                 G1, G2, t.vscale ? t.vscale[a] : 1.0));
     }
   }
+}
+
+// The electron phase of one electron.
+__device__ inline void plain_electron(const qmc_wf_desc& d, const Tables<double>& t,
+                                      const XP<double>* pw, int e, double* mo, double* bk, int nwb,
+                                      double* jrow, double* vrow) {
+  const int ne = d.nelec, nmu = d.nmo_used;
+  const double x = pw[3 * e].h, y = pw[3 * e + 1].h, z = pw[3 * e + 2].h;
+  double gx = 0.0, gy = 0.0, gz = 0.0, ks = 0.0, vs = 0.0, lp = 0.0, kn = 0.0;
+  const double w = d.use_jastrow ? __ldg(d.jastrow_w) : 0.0;
+  for (int j = 0; j < ne; ++j) {
+    if (j == e) continue;
+    const double dx = x - pw[3 * j].h, dy = y - pw[3 * j + 1].h, dz = z - pw[3 * j + 2].h;
+    const double r = sqrt_nr(dx * dx + dy * dy + dz * dz);
+    vs += rcp_nr(r);
+    if (d.use_jastrow) {
+      const double w0 = same_spin(d, e, j) ? 0.25 : 0.5;
+      const double iu = rcp_nr(1.0 + w * r);
+      ks += w0 * r * iu;
+      const double ir = rcp_nr(r);
+      const double k1 = w0 * iu * iu;
+      gx += k1 * dx * ir;
+      gy += k1 * dy * ir;
+      gz += k1 * dz * ir;
+      lp += 2.0 * k1 * ir - 2.0 * w * k1 * iu;
+    }
+  }
+  if (d.use_jastrow_en) {
+    const double wn = __ldg(d.jastrow_en_w);
+    for (int A = 0; A < t.natom; ++A) {
+      const double dx = x - t.en_p[3 * A].h, dy = y - t.en_p[3 * A + 1].h,
+                   dz = z - t.en_p[3 * A + 2].h;
+      const double r = sqrt_nr(dx * dx + dy * dy + dz * dz);
+      const double iu = rcp_nr(1.0 + wn * r);
+      kn += r * iu;
+      const double ir = rcp_nr(r);
+      const double k1 = iu * iu;
+      gx += k1 * dx * ir;
+      gy += k1 * dy * ir;
+      gz += k1 * dz * ir;
+      lp += 2.0 * k1 * ir - 2.0 * wn * k1 * iu;
+    }
+  }
+  const double jl = lp + gx * gx + gy * gy + gz * gz;
+  *jrow = 0.5 * ks + kn;
+  double ven = 0.0;
+  for (int A = 0; A < t.natom; ++A) {
+    const double dx = x - t.atom_p[3 * A].h, dy = y - t.atom_p[3 * A + 1].h,
+                 dz = z - t.atom_p[3 * A + 2].h;
+    ven -= t.atom_z[A] * rcp_nr(sqrt_nr(dx * dx + dy * dy + dz * dz));
+  }
+  *vrow = 0.5 * vs + ven;
+  const int64_t cs = nwb;
+  for (int j0 = 0; j0 < nmu; j0 += 8) {
+    double a0[8], ad[8], al[8];
+#pragma unroll
+    for (int jj = 0; jj < 8; ++jj) a0[jj] = ad[jj] = al[jj] = 0.0;
+    auto acc = [&](int a, const AOVal<double>& o) {
+      const double gdot = 2.0 * (gx * o.gx + gy * o.gy + gz * o.gz);
+      double wv[8];
+      load_w<8>(t.W + (int64_t)a * t.ncol + j0, wv);
+#pragma unroll
+      for (int jj = 0; jj < 8; ++jj) {
+        a0[jj] = fma(o.v, wv[jj], a0[jj]);
+        ad[jj] = fma(gdot, wv[jj], ad[jj]);
+        al[jj] = fma(o.lap, wv[jj], al[jj]);
+      }
+    };
+    plain_aos(t, x, y, z, acc);
+#pragma unroll
+    for (int jj = 0; jj < 8; ++jj)
+      if (j0 + jj < nmu) {
+        mo[((int64_t)e * nmu + j0 + jj) * cs] = a0[jj];
+        bk[((int64_t)e * nmu + j0 + jj) * cs] = -0.5 * (al[jj] + ad[jj] + jl * a0[jj]);
+      }
+  }
+}
+
+// After ep_eval<double, JC, true>: re-evaluates the block's walkers with a large
+// excitation ratio. Every thread of the block calls it.
+__device__ __noinline__ inline void ep_plain_walkers(const qmc_wf_desc& d, const EPPtrs& p,
+                                                     unsigned char* scr, int64_t ss, int64_t w0,
+                                                     int64_t nw) {
+  const EPShape& S = p.S;
+  const int nwb = S.nwb, tid = threadIdx.x, ns = S.nslot;
+  const EPLayout L = ep_layout(d, 1);
+  const bool dsm = S.o_det >= 0;
+  unsigned char* const dbase = dsm ? p.smem + S.o_det : scr;
+  const int64_t dss = dsm ? nwb : ss;
+  int* const flag = reinterpret_cast<int*>(p.smem + S.o_iel);
+  const int slot = tid / nwb, wl = tid - slot * nwb;
+  bool any = false;
+  if (tid < nwb) {
+    if (w0 + wl < nw) {
+      const double* dv = rptr<double>(dbase, L.dv, dss, dsm ? wl : w0 + wl);
+      for (int u = 0; u < d.ndet[0] + d.ndet[1]; ++u)
+        any |= __double2hiint(fabs(dv[u * dss])) > __double2hiint(kPlainRatio);
+    }
+    flag[wl] = any;
+  }
+  if (!__syncthreads_or(any)) return;
+  // W itself again (ep_tables keeps it as limbs)
+  const Tables<double> t = load_tables<double>(d, d.nmo_used, S.ncol, p.smem + S.o_tab);
+  const XP<double>* P = reinterpret_cast<const XP<double>*>(p.smem + S.o_pos);
+  double* MO = reinterpret_cast<double*>(p.smem + S.o_mo);
+  double* BK = reinterpret_cast<double*>(p.smem + S.o_bk);
+  double* JR = reinterpret_cast<double*>(p.smem + S.o_jrow);
+  double* VR = reinterpret_cast<double*>(p.smem + S.o_vrow);
+  const bool mine = slot < ns && flag[wl];
+  for (int e = slot; e < d.nelec && mine; e += ns)
+    plain_electron(d, t, P + wl * S.pstride, e, MO + wl, BK + wl, nwb, &JR[e * nwb + wl],
+                   &VR[e * nwb + wl]);
+  __syncthreads();
+  if (tid < 2 * nwb && flag[wl])
+    ep_det<double, true, true>(d, L, dbase, dss, dsm ? wl : w0 + wl, slot, MO, BK, wl, nwb,
+                               reinterpret_cast<double*>(p.smem + S.o_dref), d.det_table[slot]);
+  __syncthreads();
+  if (tid < nwb && flag[wl]) ep_combine<double, true>(d, t, p, dbase, dss, dsm, w0, wl);
 }
 
 // Stage the positions of walkers [w0, w0 + nwb) into shared memory as split
