@@ -236,11 +236,106 @@ __device__ __noinline__ void adj_sum_adjoints(const qmc_wf_desc& d, const AdjSha
   }
 }
 
+// The two above by a warp, a lane per determinant, for a spin of n <= kSumN electrons.
+__device__ __noinline__ void adj_sum_values_warp(const qmc_wf_desc& d, const AdjShape& A,
+                                                 const GradWork& k, int s, int n_) {
+  const GradShape& S = A.g;
+  const int r0 = s ? d.nup : 0, nmu = d.nmo_used, o = s ? d.ndet[0] : 0;
+  const MView<double> M = grad_view(k, S.mo, r0, nmu), B = grad_view(k, A.bk, r0, nmu);
+  sum_dispatch(n_, [&](auto Nc) {
+    constexpr int N = decltype(Nc)::value;
+    for (int u = threadIdx.x & 31; u < d.ndet[s]; u += 32) {
+      DetRegs<N> D;
+      D.factor(d, s, u, [&](int i, int c) { return M(i, c); });
+      double tr = 0.0;
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+        double y[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) y[i] = B(D.perm[i], D.cols[j]);
+        D.solve(y);
+        tr += y[j];
+      }
+      k.at(S.dv + o + u) = D.det;
+      k.at(A.ov + o + u) = D.det * tr;
+    }
+  });
+}
+
+__device__ __noinline__ void adj_sum_adjoints_warp(const qmc_wf_desc& d, const AdjShape& A,
+                                                   const GradWork& k, const AdjCold& cold, int s,
+                                                   int n_) {
+  const GradShape& S = A.g;
+  const int lane = threadIdx.x & 31, r0 = s ? d.nup : 0, nmu = d.nmo_used, nd = d.ndet[s];
+  const int nmax = d.nup > d.ndown ? d.nup : d.ndown;
+  const int so = s ? d.ndet[0] : 0, oo = s ? 0 : d.ndet[0];
+  const double is = k.at(S.val + GV_INV), R = k.at(A.r);
+  const MView<double> M = grad_view(k, S.mo, r0, nmu), L = grad_view(k, S.lu, r0, nmu),
+                      B = grad_view(k, A.bk, r0, nmu);
+  const MView<double> GB = adj_cold(cold, 4 * (int64_t)nmax * nmax + (int64_t)r0 * nmu, nmu);
+  for (int i = lane; i < n_ * nmu; i += 32) L(i / nmu, i % nmu) = GB(i / nmu, i % nmu) = 0.0;
+  __syncwarp();
+  sum_dispatch(n_, [&](auto Nc) {
+    constexpr int N = decltype(Nc)::value;
+    for (int u0 = 0; u0 < nd; u0 += 32) {
+      const int u = u0 + lane, m = nd - u0 < 32 ? nd - u0 : 32;
+      // d KE = dT D_u dT_u + (dD D_u + dT T_u D_u) d log D_u
+      double dT = 0.0, dD = 0.0, t = 0.0, sd = 0.0;
+      if (u < nd)
+        for (int c = 0; c < d.ncfg; ++c) {
+          if (__ldg(d.cfg_det[s] + c) != u) continue;
+          const int v = oo + __ldg(d.cfg_det[1 - s] + c);
+          const double w = __ldg(d.ci_weight + c) * is;
+          dT = fma(w, k.at(S.dv + v), dT);
+          dD = fma(w, k.at(A.ov + v) - R * k.at(S.dv + v), dD);
+        }
+      const bool on = u < nd && !(dT == 0.0 && dD == 0.0);
+      DetRegs<N> D;
+      double X[N][N];  // [column][row] of A_u^-1
+      if (on) {
+        D.factor(d, s, u, [&](int i, int c) { return M(i, c); });
+#pragma unroll
+        for (int i = 0; i < N; ++i) D.unit(i, X[i]);
+        t = dT * D.det;
+        sd = fma(dT, k.at(A.ov + so + u), dD * D.det);
+      }
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        double y[N];  // column i of X B_u X
+        if (on) {
+          double z[N];
+#pragma unroll
+          for (int r = 0; r < N; ++r) {
+            z[r] = 0.0;
+#pragma unroll
+            for (int c = 0; c < N; ++c) z[r] = fma(B(r, D.cols[c]), X[i][c], z[r]);
+          }
+#pragma unroll
+          for (int j = 0; j < N; ++j) {
+            y[j] = 0.0;
+#pragma unroll
+            for (int c = 0; c < N; ++c) y[j] = fma(X[c][j], z[c], y[j]);
+          }
+        }
+        for (int q = 0; q < m; ++q) {
+          if (lane == q && on)
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+              L(i, D.cols[j]) += sd * X[i][j] - t * y[j];
+              GB(i, D.cols[j]) += t * X[i][j];
+            }
+          __syncwarp();
+        }
+      }
+    }
+  });
+}
+
 // E_L determinant phase, one thread per (walker, spin): the factors and X
 // (`lu`), Y_occ | M over the kinetic rows, x and n of every unique determinant and
-// the base trace; the determinants D_u and n_u = D_u T_u of the explicit sums.
-__device__ inline void adj_el_determinants(const qmc_wf_desc& d, const AdjShape& A,
-                                           const GradWork& k, const AdjCold& cold, int s) {
+// the base trace. Returns whether the spin sums over explicit determinants instead.
+__device__ inline bool adj_el_determinants(const qmc_wf_desc& d, const AdjShape& A,
+                                           const GradWork& k, int s) {
   const GradShape& S = A.g;
   const int n = s ? d.ndown : d.nup, r0 = s ? d.nup : 0, nmu = d.nmo_used;
   const int nd = d.ndet[s], o = s ? d.ndet[0] : 0;
@@ -291,15 +386,15 @@ __device__ inline void adj_el_determinants(const qmc_wf_desc& d, const AdjShape&
       }
     }
   }
-  if (n > 0 && sum) adj_sum_values(d, A, k, cold, s);
   k.at(A.r + 1 + s) = base;
   k.at(S.val + GV_G + s) = sum ? 1.0 : 0.0;
+  return sum;
 }
 
-// E_L adjoint phase, one thread per (walker, spin): F_M and F_X - Y_occ^T F_M, or the
-// sums of G_A (`lu`) and G_B (scratch) over the explicit determinants.
+// E_L adjoint phase, one thread per (walker, spin): the CI sums, F_M and F_X - Y_occ^T
+// F_M, unless the spin sums over explicit determinants.
 __device__ inline void adj_el_adjoints(const qmc_wf_desc& d, const AdjShape& A, const GradWork& k,
-                                       const AdjCold& cold, int s) {
+                                       int s) {
   const GradShape& S = A.g;
   const int n = s ? d.ndown : d.nup, r0 = s ? d.nup : 0, nmu = d.nmo_used;
   const int so = s ? d.ndet[0] : 0, oo = s ? 0 : d.ndet[0];
@@ -317,12 +412,8 @@ __device__ inline void adj_el_adjoints(const qmc_wf_desc& d, const AdjShape& A, 
     k.at(S.val + GV_INV) = is;
     k.at(A.r) = R;
   }
-  if (n == 0) return;
+  if (n == 0 || k.at(S.val + GV_G + s) != 0.0) return;
   const MView<double> L = grad_view(k, S.lu, r0, nmu), B = grad_view(k, A.bk, r0, nmu);
-  if (k.at(S.val + GV_G + s) != 0.0) {
-    adj_sum_adjoints(d, A, k, cold, s, is, R);
-    return;
-  }
   const int nv = d.max_orb[s] - n, fm = A.fm + s * S.fs, fk = A.fk + s * S.fs;
   if (nv <= 0) return;
   for (int i = 0; i < n * nv; ++i) k.at(fm + i) = k.at(fk + i) = 0.0;
@@ -743,9 +834,24 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
                                     &k.at(A.bk + e * nmu), k.ws, 0, t.ngroup);
         }
       __syncthreads();
-      if (tid < 2 * nwb) adj_el_determinants(d, A, k, cold, slot);
-      __syncthreads();
-      if (tid < 2 * nwb) adj_el_adjoints(d, A, k, cold, slot);
+      bool sum = false;
+      if (tid < 2 * nwb) sum = adj_el_determinants(d, A, k, slot);
+      sum = __syncthreads_or(sum);
+      auto at = [&](int q) { return AdjCold{cold.p + (q - wl), ss}; };
+      if (sum) {
+        sum_channels(d, S, k, wl, slot, [&](int s) { adj_sum_values(d, A, k, cold, s); },
+                     [&](const GradWork& kq, int, int s, int n) { adj_sum_values_warp(d, A, kq, s, n); });
+        __syncthreads();
+      }
+      if (tid < 2 * nwb) adj_el_adjoints(d, A, k, slot);
+      if (sum) {
+        __syncthreads();
+        sum_channels(d, S, k, wl, slot,
+                     [&](int s) { adj_sum_adjoints(d, A, k, cold, s, k.at(S.val + GV_INV), k.at(A.r)); },
+                     [&](const GradWork& kq, int q, int s, int n) {
+                       adj_sum_adjoints_warp(d, A, kq, at(q), s, n);
+                     });
+      }
       if (tid < nwb) k.at(A.r + 3) = w < nw ? gout[w] : 0.0;
       __syncthreads();
     } else {
@@ -758,9 +864,8 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
                                      &k.at(S.mo + e * nmu), nullptr, k.ws, 0, t.ngroup);
         }
       __syncthreads();
-      if (tid < 2 * nwb) grad_determinants(d, S, k, slot);
+      grad_determinant_phases(d, S, k, wl, slot);
       __syncthreads();
-      if (tid < 2 * nwb) grad_adjoints(d, S, k, slot);
       if (tid < nwb) {
         double logj = 0.0, dw = 0.0, dn = 0.0;
         for (int e = 0; e < ne; ++e) {

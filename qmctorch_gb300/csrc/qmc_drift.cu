@@ -181,6 +181,23 @@ __device__ __noinline__ void drift_explicit(const qmc_wf_desc& d, const DriftSha
   }
 }
 
+// The same by a warp for a proposal with a large ratio (n <= kSumN): the determinants
+// to `dvf`, G to gx.
+__device__ __noinline__ void drift_sum_warp(const qmc_wf_desc& d, const DriftShape& S,
+                                            const DriftWork& k, int s, int n, int er) {
+  const int r0 = s ? d.nup : 0, nmu = d.nmo_used;
+  const double* const oth = k.cp + (int64_t)(S.dv0 + (s ? 0 : d.ndet[0])) * k.cs;
+  sum_dispatch(n, [&](auto N) {
+    sum_warp<decltype(N)::value, true>(
+        d, s,
+        [&](int i, int c) {
+          return r0 + i == er ? k.H(S.phi + c) : k.C(S.ma + (r0 + i) * nmu + c);
+        },
+        [&](int u, double det) { k.H(S.dvf + u) = det; }, [&](int u) { return oth[u * k.cs]; },
+        [&](int i, int c) -> double& { return k.C(S.gx + (r0 + i) * nmu + c); });
+  });
+}
+
 // Excitation mode: F(i, v) = d Sigma / d X of spin s at H(S.f + s nmax nv + i nv + v)
 // from X and the other spin's relative determinants.
 __device__ inline void drift_adjoint(const qmc_wf_desc& d, const DriftShape& S,
@@ -523,6 +540,7 @@ __global__ void __launch_bounds__(kGradThreads)
       }
     __syncthreads();
     // ---- determinants at the proposal ----
+    bool warp_sum = false;
     if (!ex) {
       if (on)
         for (int i = slot; i < n + nv; i += ns) {
@@ -552,14 +570,24 @@ __global__ void __launch_bounds__(kGradThreads)
         bool sum = false;
         for (int u = 0; u < d.ndet[sm]; ++u)
           sum |= __double2hiint(fabs(k.H(S.dvf + u))) > __double2hiint(kGradRatio);
-        k.H(S.val + DV_FLAG) = sum ? 1.0 : 0.0;
-        if (sum)
+        k.H(S.val + DV_FLAG) = sum ? e + 1.0 : 0.0;
+        warp_sum = sum && n <= kSumN;
+        if (sum && !warp_sum)
           drift_explicit(d, S, k, sm, e, k.hp + (int64_t)S.dvf * k.hs, k.hs, dv0(1 - sm), k.cs);
       }
     } else if (slot == 0) {
       drift_explicit(d, S, k, sm, e, k.hp + (int64_t)S.dvf * k.hs, k.hs, dv0(1 - sm), k.cs);
     }
-    __syncthreads();
+    if (__syncthreads_or(warp_sum)) {
+      for (int q = tid >> 5; q < S.nwb; q += blockDim.x >> 5) {
+        DriftWork kq = k;
+        kq.hp += q - wl;
+        kq.cp += q - wl;
+        const int eq = (int)kq.H(S.val + DV_FLAG) - 1, s = eq < d.nup ? 0 : 1;
+        if (eq >= 0 && nof(s) <= kSumN) drift_sum_warp(d, S, kq, s, nof(s), eq);
+      }
+      __syncthreads();
+    }
     const double* const dvf = k.hp + (int64_t)S.dvf * k.hs;
     if (slot < 2) {
       const CView<double> X{k.hp + (int64_t)S.xp * k.hs, (int64_t)nv * k.hs, k.hs};

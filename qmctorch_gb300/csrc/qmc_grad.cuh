@@ -23,6 +23,7 @@
 // ([item][walker]), or in the caller's scratch when they do not fit.
 #pragma once
 
+#include <type_traits>
 #include <math.h>
 
 #include "qmc_host.cuh"
@@ -47,8 +48,8 @@ enum { GV_SIGMA = 0, GV_INV = 1, GV_DD = 2, GV_DET = 3, GV_ACC = 5, GV_G = 6, GV
 // An excitation ratio above this takes the walker's spin to the sum over explicit
 // determinants: where the ground determinant is that much smaller than an excited
 // one, the double excitations' 2 x 2 minors of X cancel by about as much. H2O: one
-// spin in 5,000; the sums take about 0.1 ms in one thread of a block, so the line
-// lies where they are rare and the relative error is still below 1e-11.
+// spin in 5,000. The line lies where the sums are rare and the relative error is still
+// below 1e-11.
 constexpr double kGradRatio = 4096.0;
 
 inline GradShape grad_shape(const qmc_wf_desc& d, int nwb, int nslot, int jc, bool in_smem) {
@@ -288,10 +289,160 @@ __device__ __forceinline__ MView<double> grad_view(const GradWork& k, int off, i
   return MView<double>{k.p + ((int64_t)off + (int64_t)row0 * nmu) * k.ws, (int64_t)nmu * k.ws, k.ws};
 }
 
+// The sums over explicit determinants (explicit mode, large ratios). A spin of up to
+// kSumN electrons has a warp: a lane factors a determinant in registers (the steps of
+// lu_factor and lu_solve in their order) and the lanes add their terms one after the
+// other, in the determinants' order. As one thread's chain over the determinants,
+// with its matrices in memory, the block waited some 190 us for one such walker (H2O:
+// HMC 4.19 -> 3.42 ms, E_L adjoint step 2.56 -> 1.89 ms). Larger spins do not fit the
+// registers and keep the chain: in explicit mode every thread has one.
+constexpr int kSumN = 5;
+
+template <int N>
+struct DetRegs {
+  double a[N][N], det;     // factors, 1 / U_kk on the diagonal
+  int perm[N], cols[N];    // the row of A that row k of the factors came from
+
+  // Factors the columns of unique determinant u; row(i, c): MO c of the spin's electron i.
+  template <typename Row>
+  __device__ __forceinline__ void factor(const qmc_wf_desc& d, int s, int u, const Row& row) {
+    int c[QMC_MAX_NSPIN];
+    det_columns(d, s, u, c);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      cols[j] = c[j];
+      perm[j] = j;
+#pragma unroll
+      for (int i = 0; i < N; ++i) a[i][j] = row(i, c[j]);
+    }
+    det = 1.0;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      int p = k;
+      double amax = fabs(a[k][k]);
+#pragma unroll
+      for (int i = k + 1; i < N; ++i) {
+        const double v = fabs(a[i][k]);
+        if (v > amax) {
+          amax = v;
+          p = i;
+        }
+      }
+#pragma unroll
+      for (int i = k + 1; i < N; ++i) {
+        const bool sw = i == p;
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+          const double x = a[k][j], y = a[i][j];
+          a[k][j] = sw ? y : x;
+          a[i][j] = sw ? x : y;
+        }
+        const int x = perm[k], y = perm[i];
+        perm[k] = sw ? y : x;
+        perm[i] = sw ? x : y;
+      }
+      if (p != k) det = -det;
+      const double akk = a[k][k];
+      det *= akk;
+      const double inv = akk != 0.0 ? prcp(akk) : 0.0;
+      a[k][k] = inv;
+#pragma unroll
+      for (int i = k + 1; i < N; ++i) {
+        const double l = a[i][k] * inv;
+        a[i][k] = l;
+#pragma unroll
+        for (int j = k + 1; j < N; ++j) a[i][j] = fma(-l, a[k][j], a[i][j]);
+      }
+    }
+  }
+  // A x = b for b in the factors' row order
+  __device__ __forceinline__ void solve(double (&x)[N]) const {
+#pragma unroll
+    for (int i = 1; i < N; ++i)
+#pragma unroll
+      for (int k = 0; k < i; ++k) x[i] = fma(-a[i][k], x[k], x[i]);
+#pragma unroll
+    for (int i = N - 1; i >= 0; --i) {
+#pragma unroll
+      for (int k = i + 1; k < N; ++k) x[i] = fma(-a[i][k], x[k], x[i]);
+      x[i] *= a[i][i];
+    }
+  }
+  __device__ __forceinline__ void unit(int col, double (&x)[N]) const {  // column of A^-1
+#pragma unroll
+    for (int i = 0; i < N; ++i) x[i] = perm[i] == col ? 1.0 : 0.0;
+    solve(x);
+  }
+};
+
+// Calls f with the spin's electron count as a constant; n is 1 .. kSumN.
+template <typename F>
+__device__ __forceinline__ void sum_dispatch(int n, const F& f) {
+  static_assert(kSumN == 5, "the cases below");
+  switch (n) {
+    case 1: f(std::integral_constant<int, 1>{}); break;
+    case 2: f(std::integral_constant<int, 2>{}); break;
+    case 3: f(std::integral_constant<int, 3>{}); break;
+    case 4: f(std::integral_constant<int, 4>{}); break;
+    case 5: f(std::integral_constant<int, 5>{}); break;
+  }
+}
+
+// The coefficient of determinant u of spin s: sum_c c_c D(other spin's).
+template <typename D>
+__device__ __forceinline__ double sum_coef(const qmc_wf_desc& d, int s, int u, const D& other) {
+  double coef = 0.0;
+  for (int c = 0; c < d.ncfg; ++c)
+    if (__ldg(d.cfg_det[s] + c) == u)
+      coef = fma(__ldg(d.ci_weight + c), other(__ldg(d.cfg_det[1 - s] + c)), coef);
+  return coef;
+}
+
+// A warp: the determinants of spin s to dst(u), and with ADJ g(i, c) += coef_u det_u
+// A_u^-T over them (g zeroed here).
+template <int N, bool ADJ, typename Row, typename Dst, typename Other, typename G>
+__device__ __forceinline__ void sum_warp(const qmc_wf_desc& d, int s, const Row& row,
+                                         const Dst& dst, const Other& other, const G& g) {
+  const int lane = threadIdx.x & 31, nd = d.ndet[s];
+  if (ADJ) {
+    for (int i = lane; i < N * d.nmo_used; i += 32) g(i / d.nmo_used, i % d.nmo_used) = 0.0;
+    __syncwarp();
+  }
+  for (int u0 = 0; u0 < nd; u0 += 32) {
+    const int u = u0 + lane;
+    DetRegs<N> D;
+    double scale = 0.0;
+    bool on = false;
+    if (u < nd) {
+      D.factor(d, s, u, row);
+      dst(u, D.det);
+      if (ADJ) {
+        const double coef = sum_coef(d, s, u, other);
+        on = coef != 0.0;
+        scale = coef * D.det;
+      }
+    }
+    if (!ADJ) continue;
+    const int m = nd - u0 < 32 ? nd - u0 : 32;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {  // row i of A_u^-T: column i of A_u^-1
+      double y[N];
+      if (on) D.unit(i, y);
+      for (int q = 0; q < m; ++q) {
+        if (lane == q && on)
+#pragma unroll
+          for (int j = 0; j < N; ++j) {
+            double& v = g(i, D.cols[j]);
+            v = fma(scale, y[j], v);
+          }
+        __syncwarp();
+      }
+    }
+  }
+}
+
 // The matrix of unique determinant u of spin s from the MO rows, factored in the
-// spin's part of `y`; returns the determinant. The explicit sums are one thread's
-// serial chain: a block that holds such a walker waits some 190 us for it (H2O, 1000
-// gradients: 101 us without one, 289 us with).
+// spin's part of `y`; returns the determinant.
 __device__ __noinline__ inline double grad_factor(const qmc_wf_desc& d, const GradShape& S, const GradWork& k,
                                      int s, int u, int* cols, int* piv) {
   const int n = s ? d.ndown : d.nup, r0 = s ? d.nup : 0, nmu = d.nmo_used;
@@ -338,11 +489,45 @@ __device__ __noinline__ inline void grad_sum_adjoints(const qmc_wf_desc& d, cons
   }
 }
 
+// A warp's version of the two above, for a spin of n <= kSumN.
+template <bool ADJ>
+__device__ __noinline__ inline void grad_sum_warp(const qmc_wf_desc& d, const GradShape& S,
+                                                  const GradWork& k, int s, int n) {
+  const int r0 = s ? d.nup : 0, dv = S.dv + (s ? d.ndet[0] : 0), oth = S.dv + (s ? 0 : d.ndet[0]);
+  const MView<double> M = grad_view(k, S.mo, r0, d.nmo_used), L = grad_view(k, S.lu, r0, d.nmo_used);
+  sum_dispatch(n, [&](auto N) {
+    sum_warp<decltype(N)::value, ADJ>(
+        d, s, [&](int i, int c) { return M(i, c); },
+        [&](int u, double det) { if (!ADJ) k.at(dv + u) = det; },
+        [&](int u) { return k.at(oth + u); }, [&](int i, int c) -> double& { return L(i, c); });
+  });
+}
+
+// The block's (walker, spin) channels that sum over explicit determinants: chain(s) for
+// this thread's own of more than kSumN electrons, warp(k, wl, s, n) for the others, one
+// after the other. The flags are behind a barrier. k, wl, slot: this thread's.
+template <typename Chain, typename Warp>
+__device__ __forceinline__ void sum_channels(const qmc_wf_desc& d, const GradShape& S,
+                                             const GradWork& k, int wl, int slot,
+                                             const Chain& chain, const Warp& warp) {
+  const int tid = threadIdx.x, nwb = S.nwb;
+  if (tid < 2 * nwb && (slot ? d.ndown : d.nup) > kSumN && k.at(S.val + GV_G + slot) != 0.0)
+    chain(slot);
+  for (int ch = tid >> 5; ch < 2 * nwb; ch += blockDim.x >> 5) {
+    const int s = ch / nwb, q = ch - s * nwb, n = s ? d.ndown : d.nup;
+    if (n == 0 || n > kSumN) continue;
+    GradWork kq = k;
+    kq.wl += q - wl;
+    kq.p = kq.p0 + kq.wl;
+    if (kq.at(S.val + GV_G + s) != 0.0) warp(kq, q, s, n);
+  }
+}
+
 // Determinant phase, one thread per (walker, spin): excitation mode factors a
 // copy of the MO rows (occupied columns: the LU, virtual columns: X) and writes
 // the determinants relative to det A; explicit mode (and a walker with a large
-// ratio) the determinants themselves.
-__device__ inline void grad_determinants(const qmc_wf_desc& d, const GradShape& S,
+// ratio) leaves the determinants themselves to the sums and returns true.
+__device__ inline bool grad_determinants(const qmc_wf_desc& d, const GradShape& S,
                                          const GradWork& k, int s) {
   const int n = s ? d.ndown : d.nup, r0 = s ? d.nup : 0, nmu = d.nmo_used;
   const int nd = d.ndet[s], dv = S.dv + (s ? d.ndet[0] : 0);
@@ -366,17 +551,15 @@ __device__ inline void grad_determinants(const qmc_wf_desc& d, const GradShape& 
     for (int u = 0; u < nd; ++u)
       sum |= __double2hiint(fabs(k.at(dv + u))) > __double2hiint(kGradRatio);
   }
-  if (n > 0 && sum) {
-    grad_sum_values(d, S, k, s);
-    det = 1.0;
-  }
+  if (sum) det = 1.0;
   k.at(S.val + GV_DET + s) = det;
   k.at(S.val + GV_G + s) = sum ? 1.0 : 0.0;
+  return sum;
 }
 
 // Adjoint phase, one thread per (walker, spin), after both spins'
-// determinants: the CI sum, and F or, where the spin sums over explicit
-// determinants, G.
+// determinants: the CI sum, and F unless the spin sums over explicit determinants
+// (their G: grad_sums).
 __device__ inline void grad_adjoints(const qmc_wf_desc& d, const GradShape& S, const GradWork& k,
                                      int s) {
   const int n = s ? d.ndown : d.nup, r0 = s ? d.nup : 0, nmu = d.nmo_used;
@@ -394,11 +577,7 @@ __device__ inline void grad_adjoints(const qmc_wf_desc& d, const GradShape& S, c
     k.at(S.val + GV_DD) = dd;
     k.at(S.val + GV_INV) = dd * sigma == 0.0 ? nan("") : 1.0 / sigma;
   }
-  if (n == 0) return;
-  if (k.at(S.val + GV_G + s) != 0.0) {
-    grad_sum_adjoints(d, S, k, s);
-    return;
-  }
+  if (n == 0 || k.at(S.val + GV_G + s) != 0.0) return;
   const int nv = d.max_orb[s] - n;
   const MView<double> X{L.p + n * L.cs, L.rs, L.cs};
   const int f0 = S.f + s * S.fs;
@@ -422,6 +601,24 @@ __device__ inline void grad_adjoints(const qmc_wf_desc& d, const GradShape& S, c
       k.at(f0 + i2) = fma(-cd, x1, k.at(f0 + i2));
     }
   }
+}
+
+// Both determinant phases and the sums. Every thread of the block calls it; what it
+// writes is behind the caller's next barrier.
+__device__ inline void grad_determinant_phases(const qmc_wf_desc& d, const GradShape& S,
+                                               const GradWork& k, int wl, int slot) {
+  bool sum = false;
+  if (threadIdx.x < 2 * S.nwb) sum = grad_determinants(d, S, k, slot);
+  sum = __syncthreads_or(sum);
+  if (sum) {
+    sum_channels(d, S, k, wl, slot, [&](int s) { grad_sum_values(d, S, k, s); },
+                 [&](const GradWork& kq, int, int s, int n) { grad_sum_warp<false>(d, S, kq, s, n); });
+    __syncthreads();
+  }
+  if (threadIdx.x < 2 * S.nwb) grad_adjoints(d, S, k, slot);
+  if (sum)  // own arrays: nothing of grad_adjoints is read or written
+    sum_channels(d, S, k, wl, slot, [&](int s) { grad_sum_adjoints(d, S, k, s); },
+                 [&](const GradWork& kq, int, int s, int n) { grad_sum_warp<true>(d, S, kq, s, n); });
 }
 
 // Column i of A^-1 of spin s (A y = e_i with the factors in `lu`):
@@ -539,9 +736,7 @@ __device__ inline void grad_evaluate(const qmc_wf_desc& d, const GradTables& t,
                                   nullptr, b.k.ws, 0, t.t.ngroup);
     }
   __syncthreads();
-  if (threadIdx.x < 2 * S.nwb) grad_determinants(d, S, b.k, b.slot);
-  __syncthreads();
-  if (threadIdx.x < 2 * S.nwb) grad_adjoints(d, S, b.k, b.slot);
+  grad_determinant_phases(d, S, b.k, b.wl, b.slot);
   __syncthreads();
 }
 
