@@ -102,6 +102,11 @@ __host__ __device__ inline EPLayout ep_layout(const qmc_wf_desc& d, int kind) {
 // shared-memory and scratch layouts
 // ---------------------------------------------------------------------------
 constexpr int64_t kDetSmemBytes = 16384;
+// least room of ep_plain_walkers (in the threads' AO slots): Jastrow terms of the
+// electrons, AO values and derivatives of one
+__host__ __device__ inline int64_t plain_bytes(const qmc_wf_desc& d) {
+  return 8 * (4 * (int64_t)d.nelec + 5 * (int64_t)d.nao);
+}
 // AOs per chunk of the FP64 local energy's contraction (two values per AO)
 constexpr int kFixElAOs = 8;
 static_assert(kFixElAOs >= QMC_MAX_COMP && kFixElAOs <= kFixAOs, "a chunk holds an AO group");
@@ -180,6 +185,7 @@ __host__ __device__ inline EPShape ep_shape(const qmc_wf_desc& d, int kind, int 
   if (kind == 1 || !kMixed<R>)
     o += align8((int64_t)s.nthreads * (kind == 1 ? (kMixed<R> ? 3 : 2) * kFixElAOs : kFixAOs) *
                 (int64_t)sizeof(R));
+  if (kind == 1 && !kMixed<R> && o < s.o_fix + plain_bytes(d)) o = s.o_fix + plain_bytes(d);
   s.o_ecol = o;
   if (!kMixed<R>) o += align8((int64_t)s.ncol * 4);
   // the determinant phase works in shared memory when the block's arrays are
@@ -1514,21 +1520,30 @@ __device__ inline void ep_eval(const qmc_wf_desc& d, const Tables<R>& t, const E
 // H2O: about one block of 16 walkers in 100 does the second evaluation.
 constexpr double kPlainRatio = 4096.0;
 
-// All AOs of one electron with derivatives.
+// AOs of group g of the electron at (x, y, z), with derivatives.
 template <typename F>
-__device__ inline void plain_aos(const Tables<double>& t, double x, double y, double z, F& f) {
-  for (int g = 0; g < t.ngroup; ++g) {
-    const int A = t.group_atom[g];
-    const double dx = x - t.atom_p[3 * A].h, dy = y - t.atom_p[3 * A + 1].h,
-                 dz = z - t.atom_p[3 * A + 2].h;
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    if (t.radial != QMC_RADIAL_GTO) {
-      group_sto<double, true>(t, g, dx, dy, dz, r2, f);
-      continue;
-    }
-    const int np = t.group_prim[g + 1] - t.group_prim[g];
-    for (int a = t.group_ao[g]; a < t.group_ao[g + 1]; ++a) {
-      double G0 = 0.0, G1 = 0.0, G2 = 0.0;
+__device__ inline void plain_group(const Tables<double>& t, int g, double x, double y, double z,
+                                   const F& f) {
+  const int A = t.group_atom[g];
+  const double dx = x - t.atom_p[3 * A].h, dy = y - t.atom_p[3 * A + 1].h,
+               dz = z - t.atom_p[3 * A + 2].h;
+  const double r2 = dx * dx + dy * dy + dz * dz;
+  if (t.radial != QMC_RADIAL_GTO) {
+    group_sto<double, true>(t, g, dx, dy, dz, r2, f);
+    return;
+  }
+  const int np = t.group_prim[g + 1] - t.group_prim[g], ga = t.group_ao[g];
+  const int kind = t.group_kind[g];
+  double sh[2][3];  // radial sums that components share
+  for (int a = ga; a < t.group_ao[g + 1]; ++a) {
+    const int c = a - ga;
+    const int share = kind == GK_P ? 0 : (kind == GK_D ? (c == 0 || c == 3 || c == 5 ? 0 : 1) : -1);
+    double G0 = 0.0, G1 = 0.0, G2 = 0.0;
+    if (share >= 0 && c > share) {
+      G0 = sh[share][0];
+      G1 = sh[share][1];
+      G2 = sh[share][2];
+    } else {
       for (int p = 0; p < np; ++p) {
         const int wi = t.ao_wofs[a] + p;
         const double al = t.walpha[wi];
@@ -1538,22 +1553,27 @@ __device__ inline void plain_aos(const Tables<double>& t, double x, double y, do
         G1 = fma(w, e1, G1);
         G2 = fma(w, e2, G2);
       }
-      const int kx = t.ao_k[3 * a], ky = t.ao_k[3 * a + 1], kz = t.ao_k[3 * a + 2];
-      const double px = pk0(dx, kx), py = pk0(dy, ky), pz = pk0(dz, kz);
-      const double qx = pk1(dx, kx) * py * pz, qy = px * pk1(dy, ky) * pz,
-                   qz = px * py * pk1(dz, kz);
-      const double lapP = pk2(dx, kx) * py * pz + px * pk2(dy, ky) * pz + px * py * pk2(dz, kz);
-      f(a, ao_from<double, true>(px * py * pz, qx, qy, qz, lapP, kx + ky + kz, dx, dy, dz, r2, G0,
-                                 G1, G2, t.vscale ? t.vscale[a] : 1.0));
+      if (share >= 0) {
+        sh[share][0] = G0;
+        sh[share][1] = G1;
+        sh[share][2] = G2;
+      }
     }
+    const int kx = t.ao_k[3 * a], ky = t.ao_k[3 * a + 1], kz = t.ao_k[3 * a + 2];
+    const double px = pk0(dx, kx), py = pk0(dy, ky), pz = pk0(dz, kz);
+    const double qx = pk1(dx, kx) * py * pz, qy = px * pk1(dy, ky) * pz,
+                 qz = px * py * pk1(dz, kz);
+    const double lapP = pk2(dx, kx) * py * pz + px * pk2(dy, ky) * pz + px * py * pk2(dz, kz);
+    f(a, ao_from<double, true>(px * py * pz, qx, qy, qz, lapP, kx + ky + kz, dx, dy, dz, r2, G0,
+                               G1, G2, t.vscale ? t.vscale[a] : 1.0));
   }
 }
 
-// The electron phase of one electron.
-__device__ inline void plain_electron(const qmc_wf_desc& d, const Tables<double>& t,
-                                      const XP<double>* pw, int e, double* mo, double* bk, int nwb,
-                                      double* jrow, double* vrow) {
-  const int ne = d.nelec, nmu = d.nmo_used;
+// Jastrow and Coulomb rows of electron e; jt: grad U and lap U + |grad U|^2.
+__device__ inline void plain_jastrow(const qmc_wf_desc& d, const Tables<double>& t,
+                                     const XP<double>* pw, int e, double* jrow, double* vrow,
+                                     double* jt) {
+  const int ne = d.nelec;
   const double x = pw[3 * e].h, y = pw[3 * e + 1].h, z = pw[3 * e + 2].h;
   double gx = 0.0, gy = 0.0, gz = 0.0, ks = 0.0, vs = 0.0, lp = 0.0, kn = 0.0;
   const double w = d.use_jastrow ? __ldg(d.jastrow_w) : 0.0;
@@ -1599,29 +1619,65 @@ __device__ inline void plain_electron(const qmc_wf_desc& d, const Tables<double>
     ven -= t.atom_z[A] * rcp_nr(sqrt_nr(dx * dx + dy * dy + dz * dz));
   }
   *vrow = 0.5 * vs + ven;
-  const int64_t cs = nwb;
-  for (int j0 = 0; j0 < nmu; j0 += 8) {
-    double a0[8], ad[8], al[8];
-#pragma unroll
-    for (int jj = 0; jj < 8; ++jj) a0[jj] = ad[jj] = al[jj] = 0.0;
-    auto acc = [&](int a, const AOVal<double>& o) {
-      const double gdot = 2.0 * (gx * o.gx + gy * o.gy + gz * o.gz);
-      double wv[8];
-      load_w<8>(t.W + (int64_t)a * t.ncol + j0, wv);
-#pragma unroll
-      for (int jj = 0; jj < 8; ++jj) {
-        a0[jj] = fma(o.v, wv[jj], a0[jj]);
-        ad[jj] = fma(gdot, wv[jj], ad[jj]);
-        al[jj] = fma(o.lap, wv[jj], al[jj]);
+  jt[0] = gx;
+  jt[1] = gy;
+  jt[2] = gz;
+  jt[3] = jl;
+}
+
+// MO and kinetic rows of one walker by the whole block. An FP64 warp instruction costs
+// its 64 cycles with one active lane as with 32, so the work is dealt out: a thread
+// per (electron, AO group) puts values and derivatives into `buf`, one per (electron,
+// column) sums them in AO order (H2O: a block with such a walker took 172 us more with a
+// thread per electron, 104 us now).
+__device__ inline void plain_rows(const qmc_wf_desc& d, const Tables<double>& t,
+                                  const XP<double>* pw, double* mo, double* bk, double* jrow,
+                                  double* vrow, int nwb, double* buf, int64_t nbuf) {
+  const int tid = threadIdx.x, nt = blockDim.x, ne = d.nelec, nao = d.nao, nmu = d.nmo_used;
+  const int64_t room = (nbuf - 4 * ne) / (5 * nao);
+  const int ec = room < ne ? (int)room : ne;
+  double* const ao = buf + 4 * ne;
+  const int skip = nt >= 64 ? 32 : 0;  // the first warp has the Jastrow rows
+  if (tid < 32)
+    for (int e = tid; e < ne; e += nt < 32 ? nt : 32)
+      plain_jastrow(d, t, pw, e, jrow + e * nwb, vrow + e * nwb, buf + 4 * e);
+  for (int e0 = 0; e0 < ne; e0 += ec) {
+    const int ne1 = ne - e0 < ec ? ne - e0 : ec;
+    for (int i = tid - skip; i >= 0 && i < ne1 * t.ngroup; i += nt - skip) {
+      const int el = i / t.ngroup, e = e0 + el;
+      double* const row = ao + (int64_t)el * nao * 5;
+      plain_group(t, i - el * t.ngroup, pw[3 * e].h, pw[3 * e + 1].h, pw[3 * e + 2].h,
+                  [&](int a, const AOVal<double>& o) {
+                    double* const q = row + a * 5;
+                    q[0] = o.v;
+                    q[1] = o.gx;
+                    q[2] = o.gy;
+                    q[3] = o.gz;
+                    q[4] = o.lap;
+                  });
+    }
+    __syncthreads();
+    for (int i = tid; i < ne1 * nao; i += nt) {
+      const double* const g = buf + 4 * (e0 + i / nao);
+      double* const q = ao + (int64_t)i * 5;
+      q[1] = 2.0 * (g[0] * q[1] + g[1] * q[2] + g[2] * q[3]);
+    }
+    __syncthreads();
+    for (int i = tid; i < ne1 * nmu; i += nt) {
+      const int el = i / nmu, j = i - el * nmu;
+      const double* q = ao + (int64_t)el * nao * 5;
+      double a0 = 0.0, ad = 0.0, al = 0.0;
+      for (int a = 0; a < nao; ++a, q += 5) {
+        const double w = t.W[(int64_t)a * t.ncol + j];
+        a0 = fma(q[0], w, a0);
+        ad = fma(q[1], w, ad);
+        al = fma(q[4], w, al);
       }
-    };
-    plain_aos(t, x, y, z, acc);
-#pragma unroll
-    for (int jj = 0; jj < 8; ++jj)
-      if (j0 + jj < nmu) {
-        mo[((int64_t)e * nmu + j0 + jj) * cs] = a0[jj];
-        bk[((int64_t)e * nmu + j0 + jj) * cs] = -0.5 * (al[jj] + ad[jj] + jl * a0[jj]);
-      }
+      const int64_t at = (int64_t)((e0 + el) * nmu + j) * nwb;
+      mo[at] = a0;
+      bk[at] = -0.5 * (al + ad + buf[4 * (e0 + el) + 3] * a0);
+    }
+    __syncthreads();
   }
 }
 
@@ -1631,7 +1687,7 @@ __device__ __noinline__ inline void ep_plain_walkers(const qmc_wf_desc& d, const
                                                      unsigned char* scr, int64_t ss, int64_t w0,
                                                      int64_t nw) {
   const EPShape& S = p.S;
-  const int nwb = S.nwb, tid = threadIdx.x, ns = S.nslot;
+  const int nwb = S.nwb, tid = threadIdx.x;
   const EPLayout L = ep_layout(d, 1);
   const bool dsm = S.o_det >= 0;
   unsigned char* const dbase = dsm ? p.smem + S.o_det : scr;
@@ -1655,16 +1711,24 @@ __device__ __noinline__ inline void ep_plain_walkers(const qmc_wf_desc& d, const
   double* BK = reinterpret_cast<double*>(p.smem + S.o_bk);
   double* JR = reinterpret_cast<double*>(p.smem + S.o_jrow);
   double* VR = reinterpret_cast<double*>(p.smem + S.o_vrow);
-  const bool mine = slot < ns && flag[wl];
-  for (int e = slot; e < d.nelec && mine; e += ns)
-    plain_electron(d, t, P + wl * S.pstride, e, MO + wl, BK + wl, nwb, &JR[e * nwb + wl],
-                   &VR[e * nwb + wl]);
-  __syncthreads();
+  // the first of these walkers work in the AO slots, which are free now, the others where
+  // the block's determinants are
+  const int64_t fit = (S.o_ecol - S.o_fix) / L.bytes_per_slot;
+  int rank = 0;
+  for (int q = 0; q < wl; ++q) rank += flag[q] != 0;
+  const bool in = rank < fit;
+  unsigned char* const wbase = in ? p.smem + S.o_fix + (rank - wl) * (int)sizeof(double) : dbase;
+  const int64_t wss = in ? fit : dss;
+  const bool wsm = in || dsm;
+  for (int q = 0; q < nwb; ++q)
+    if (flag[q])
+      plain_rows(d, t, P + q * S.pstride, MO + q, BK + q, JR + q, VR + q, nwb,
+                 reinterpret_cast<double*>(p.smem + S.o_fix), (S.o_ecol - S.o_fix) / 8);
   if (tid < 2 * nwb && flag[wl])
-    ep_det<double, true, true>(d, L, dbase, dss, dsm ? wl : w0 + wl, slot, MO, BK, wl, nwb,
+    ep_det<double, true, true>(d, L, wbase, wss, wsm ? wl : w0 + wl, slot, MO, BK, wl, nwb,
                                reinterpret_cast<double*>(p.smem + S.o_dref), d.det_table[slot]);
   __syncthreads();
-  if (tid < nwb && flag[wl]) ep_combine<double, true>(d, t, p, dbase, dss, dsm, w0, wl);
+  if (tid < nwb && flag[wl]) ep_combine<double, true>(d, t, p, wbase, wss, wsm, w0, wl);
 }
 
 // Stage the positions of walkers [w0, w0 + nwb) into shared memory as split
