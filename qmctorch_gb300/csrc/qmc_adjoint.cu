@@ -1018,6 +1018,13 @@ static AdjShape adj_plan(const qmc_wf_desc& d, bool el, int jc, K kernel, int64_
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   AdjShape best = adj_shape(d, el, 1, 2, jc, true);
+  const PlanKey key = plan_key((const void*)kernel, dev, nw, d, best.smem);
+  PlanChoice got;
+  if (plan_find(key, &got)) {
+    best = adj_shape(d, el, got.nwb, got.nslot, jc, got.in_smem);
+    best.grid = got.grid;
+    return best;
+  }
   best.smem = -1;
   double best_cost = 0.0;
   for (int in_smem = 1; in_smem >= 0 && best.smem < 0; --in_smem)
@@ -1049,6 +1056,7 @@ static AdjShape adj_plan(const qmc_wf_desc& d, bool el, int jc, K kernel, int64_
           best_cost = cost;
         }
       }
+  if (best.smem >= 0) plan_keep(key, {best.g.nwb, best.g.nslot, best.o_work >= 0, best.grid});
   return best;
 }
 

@@ -776,6 +776,9 @@ static DriftShape drift_plan(const qmc_wf_desc& d, int64_t nw) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   DriftShape best = drift_shape(d, 1, 2, true);
+  const PlanKey key = plan_key((const void*)drift_kernel, dev, nw, d, best.smem);
+  PlanChoice got;
+  if (plan_find(key, &got)) return drift_shape(d, got.nwb, got.nslot, got.in_smem);
   best.smem = -1;
   double best_cost = 0.0;
   const int most = d.nelec > 16 ? 16 : (d.nelec < 2 ? 2 : d.nelec);
@@ -805,6 +808,7 @@ static DriftShape drift_plan(const qmc_wf_desc& d, int64_t nw) {
           best_cost = cost;
         }
       }
+  if (best.smem >= 0) plan_keep(key, {best.nwb, best.nslot, best.o_hot >= 0, 0});
   return best;
 }
 

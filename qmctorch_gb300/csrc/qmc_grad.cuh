@@ -23,6 +23,7 @@
 // ([item][walker]), or in the caller's scratch when they do not fit.
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 #include <math.h>
 
@@ -740,6 +741,43 @@ __device__ inline void grad_evaluate(const qmc_wf_desc& d, const GradTables& t,
   __syncthreads();
 }
 
+// The launch plans' choices, kept per kernel, device, walker count and the sizes that the
+// shapes depend on (a search asks the occupancy calculator some 40 times, 0.1 ms).
+struct PlanKey {
+  const void* kernel;
+  int64_t v[16];
+  bool operator==(const PlanKey& o) const {
+    return kernel == o.kernel && std::equal(v, v + 16, o.v);
+  }
+};
+struct PlanChoice {
+  int nwb, nslot;
+  bool in_smem;
+  int grid;
+};
+inline PlanKey plan_key(const void* kernel, int dev, int64_t nw, const qmc_wf_desc& d,
+                        int64_t smem) {
+  return PlanKey{kernel, {dev, nw, smem, d.nelec, d.nup, d.ndown, d.nao, d.nmo_used, d.nweight,
+                          d.det_mode, d.ncfg, d.max_orb[0], d.max_orb[1], d.ndet[0], d.ndet[1],
+                          d.ngroup}};
+}
+inline std::mutex plan_mutex;
+inline std::vector<std::pair<PlanKey, PlanChoice>> plan_choices;  // at most 256
+inline bool plan_find(const PlanKey& key, PlanChoice* c) {
+  std::lock_guard<std::mutex> g(plan_mutex);
+  for (const auto& kv : plan_choices)
+    if (kv.first == key) {
+      *c = kv.second;
+      return true;
+    }
+  return false;
+}
+inline void plan_keep(const PlanKey& key, const PlanChoice& c) {
+  std::lock_guard<std::mutex> g(plan_mutex);
+  if (plan_choices.size() >= 256) plan_choices.clear();
+  plan_choices.emplace_back(key, c);
+}
+
 // Launch plan. The kernels are FP64 bound (the pipe was 100 % busy on an SM with
 // 15 warps), and a warp instruction costs the same with idle lanes, so of the
 // block sizes that fit the one with the least warp work on the busiest SM is
@@ -750,28 +788,13 @@ __device__ inline void grad_evaluate(const qmc_wf_desc& d, const GradTables& t,
 // SM, one round) against 8 x 10 in two rounds, 4.75 -> 3.5 ms for the HMC kernel.
 template <typename K>
 inline GradShape grad_plan(const qmc_wf_desc& d, int jc, K kernel, int64_t nw) {
-  struct Key {
-    const void* k;
-    int dev, jc;
-    int64_t nw, smem, total, ne;
-    bool operator==(const Key& o) const {
-      return k == o.k && dev == o.dev && jc == o.jc && nw == o.nw && smem == o.smem &&
-             total == o.total && ne == o.ne;
-    }
-  };
   int dev = 0, nsm = 1;
   cudaGetDevice(&dev);
-  const GradShape one = grad_shape(d, 1, 2, jc, true);
-  const Key key{(const void*)kernel, dev, jc, nw, one.smem, one.total, d.nelec};
-  static std::mutex mu;
-  static std::vector<std::pair<Key, GradShape>> cache;
-  {
-    std::lock_guard<std::mutex> g(mu);
-    for (const auto& kv : cache)
-      if (kv.first == key) return kv.second;
-  }
+  GradShape best = grad_shape(d, 1, 2, jc, true);
+  const PlanKey key = plan_key((const void*)kernel, dev, nw, d, best.smem);
+  PlanChoice got;
+  if (plan_find(key, &got)) return grad_shape(d, got.nwb, got.nslot, jc, got.in_smem);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  GradShape best = one;
   best.smem = -1;
   double best_cost = 0.0;
   for (int in_smem = 1; in_smem >= 0 && best.smem < 0; --in_smem)
@@ -803,11 +826,7 @@ inline GradShape grad_plan(const qmc_wf_desc& d, int jc, K kernel, int64_t nw) {
           best_cost = cost;
         }
       }
-  if (best.smem >= 0) {
-    std::lock_guard<std::mutex> g(mu);
-    if (cache.size() > 256) cache.clear();
-    cache.emplace_back(key, best);
-  }
+  if (best.smem >= 0) plan_keep(key, {best.nwb, best.nslot, best.o_work >= 0, 0});
   return best;
 }
 
