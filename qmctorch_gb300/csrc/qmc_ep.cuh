@@ -109,6 +109,12 @@ __host__ __device__ inline int64_t plain_bytes(const qmc_wf_desc& d) {
 }
 // AOs per chunk of the FP64 local energy's contraction (two values per AO)
 constexpr int kFixElAOs = 8;
+// FP32 local energy: up to this many columns are summed in registers, in one pass over
+// the AOs; more go through the threads' slots in shared memory (ep_float_rows), where
+// the registers would take a pass per eight. H2O (7 columns) through the slots: 1.09e8
+// E_L/s, in registers 1.55e8; C6H6 (21 columns) in registers 4.57 ms, through the
+// slots 2.83.
+constexpr int kFloatRegCols = 8;
 static_assert(kFixElAOs >= QMC_MAX_COMP && kFixElAOs <= kFixAOs, "a chunk holds an AO group");
 
 struct EPShape {
@@ -156,7 +162,8 @@ __host__ __device__ inline EPShape ep_shape(const qmc_wf_desc& d, int kind, int 
   s.o_bk = o;
   if (kind == 1) o += align8(d.nelec * nmu * nwb * (int64_t)sizeof(R));
   s.o_bd = o;
-  if (kind == 1 && kMixed<R>) o += align8(d.nelec * nmu * nwb * (int64_t)sizeof(R));
+  if (kind == 1 && kMixed<R> && nmu > kFloatRegCols)
+    o += align8(d.nelec * nmu * nwb * (int64_t)sizeof(R));
   s.o_jrow = o;
   o += align8((int64_t)d.nelec * nwb * 8);
   s.o_vrow = o;
@@ -182,7 +189,7 @@ __host__ __device__ inline EPShape ep_shape(const qmc_wf_desc& d, int kind, int 
     o += align8(2 * nmax * nmax * nwb * (int64_t)sizeof(R));
   }
   s.o_fix = o;
-  if (kind == 1 || !kMixed<R>)
+  if (!kMixed<R> || (kind == 1 && d.nmo_used > kFloatRegCols))
     o += align8((int64_t)s.nthreads * (kind == 1 ? (kMixed<R> ? 3 : 2) * kFixElAOs : kFixAOs) *
                 (int64_t)sizeof(R));
   if (kind == 1 && !kMixed<R> && o < s.o_fix + plain_bytes(d)) o = s.o_fix + plain_bytes(d);
@@ -721,8 +728,34 @@ __device__ inline void ep_electron(const qmc_wf_desc& d, const Tables<R>& t, con
                              reinterpret_cast<int2*>(fix), fix_stride, mrow,
                              brow, cs, 0, t.ngroup);
   } else if constexpr (KIN) {
-    ep_float_rows(t, nmu, ex, ey, ez, gx, gy, gz, jl, fix, fix_stride, mrow, brow,
-                  bd + (int64_t)e * nmu * cs, cs);
+    if (nmu > kFloatRegCols) {
+      ep_float_rows(t, nmu, ex, ey, ez, gx, gy, gz, jl, fix, fix_stride, mrow, brow,
+                    bd + (int64_t)e * nmu * cs, cs);
+      return;
+    }
+    uint64_t m[4], b[4], l[4];  // value, gradient and Laplacian sums
+#pragma unroll
+    for (int q = 0; q < 4; ++q) m[q] = b[q] = l[q] = 0;
+    auto acc = [&](int a, const AOVal<R>& o) {
+      const ulonglong2* w = reinterpret_cast<const ulonglong2*>(t.W + (int64_t)a * t.ncol);
+      const float g = 2.0f * (gx * o.gx + gy * o.gy + gz * o.gz);
+      const uint64_t xx = pack2(o.v, o.v), yy = pack2(g, g), zz = pack2(o.lap, o.lap);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint64_t c = q % 2 ? w[q / 2].y : w[q / 2].x;
+        m[q] = fma2(xx, c, m[q]);
+        b[q] = fma2(yy, c, b[q]);
+        l[q] = fma2(zz, c, l[q]);
+      }
+    };
+    for_each_ao_ep<R, KIN>(t, ex, ey, ez, acc);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (j < nmu) {
+        const float x = unpack2(m[j / 2], j % 2);
+        mrow[j * cs] = x;
+        brow[j * cs] = -0.5f * (unpack2(l[j / 2], j % 2) + unpack2(b[j / 2], j % 2) + jl * x);
+      }
   } else {
     for (int j0 = 0; j0 < nmu; j0 += JC) {
       uint64_t m[JC / 2];
