@@ -28,7 +28,7 @@ SOURCES = ["qmc_wf_kernels.cu", "qmc_staged.cu", "qmc_metropolis.cu", "qmc_capi_
 # translation units compiled more than once, with defines: (source, object, flags)
 INSTANCES = [("qmc_metropolis_inst.cu", "qmc_metropolis_%s_%d" % (r, jc),
               ["-DQMC_INST_R=%s" % r, "-DQMC_INST_JC=%d" % jc])
-             for r in ("float", "double") for jc in (8, 16, 24)]
+             for r, jc in (("float", 8), ("float", 16), ("float", 24), ("double", 8))]
 INSTANCES += [("qmc_hmc_inst.cu", "qmc_hmc_%d" % jc, ["-DQMC_INST_JC=%d" % jc])
               for jc in (8, 16, 24)]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

@@ -129,16 +129,25 @@ struct EPShape {
   int64_t smem;  // dynamic shared memory bytes
   int64_t o_tab, o_pos, o_pnew, o_mo, o_bk, o_jrow, o_vrow, o_dref, o_psi, o_f, o_kin, o_v,
       o_iel, o_acc;
-  int64_t o_bd;         // FP32 local energy: gradient part of the kinetic rows
+  int level;     // what the shape does without to fit (ep_shape)
+  int64_t o_bd;         // FP32 local energy: gradient part of the kinetic rows, or -1: registers
   int64_t o_lu;         // the factors of el_diagonal's cooperative phase, or -1: work arrays
-  int64_t o_fix, o_ecol;  // the threads' AO values (FP64: as limbs); FP64: W's column exponents
+  int64_t o_fix, fix_bytes;  // the threads' AO values (FP64: as limbs)
+  int64_t o_ecol;            // FP64: W's column exponents, or -1: W is not in limbs (ep_plain_rows)
   int64_t o_det;  // determinant-phase work arrays of the block's walkers, or -1: HBM scratch
 };
 
+// level 0: everything that helps; 1: el_diagonal's factors in the work arrays; 2: the least
+// shared memory, without the threads' AO slots and what only they are for (FP64: sums of
+// FP64 multiply-adds, no second evaluation of walkers near a node; FP32 local energy: columns
+// in registers, a pass over the AOs per eight). The plan search takes the first level at
+// which a block of one walker fits.
+constexpr int kEPLevels = 3;
 template <typename R>
 __host__ __device__ inline EPShape ep_shape(const qmc_wf_desc& d, int kind, int nwb, int jc,
-                                           int nslot, bool pos_global = false) {
+                                           int nslot, bool pos_global = false, int level = 0) {
   EPShape s;
+  s.level = level;
   s.nwb = nwb;
   s.nslot = nslot;
   s.pos_global = (kind == 2 && pos_global) ? 1 : 0;
@@ -161,9 +170,11 @@ __host__ __device__ inline EPShape ep_shape(const qmc_wf_desc& d, int kind, int 
   o += align8(d.nelec * nmu * nwb * (int64_t)sizeof(R));
   s.o_bk = o;
   if (kind == 1) o += align8(d.nelec * nmu * nwb * (int64_t)sizeof(R));
-  s.o_bd = o;
-  if (kind == 1 && kMixed<R> && nmu > kFloatRegCols)
+  s.o_bd = -1;
+  if (kind == 1 && kMixed<R> && nmu > kFloatRegCols && level < 2) {
+    s.o_bd = o;
     o += align8(d.nelec * nmu * nwb * (int64_t)sizeof(R));
+  }
   s.o_jrow = o;
   o += align8((int64_t)d.nelec * nwb * 8);
   s.o_vrow = o;
@@ -183,18 +194,24 @@ __host__ __device__ inline EPShape ep_shape(const qmc_wf_desc& d, int kind, int 
   s.o_acc = o;
   o += align8(nwb * 4);
   s.o_lu = -1;
-  if (kind == 1 && el_diagonal(d) && nslot >= 4) {
+  if (kind == 1 && el_diagonal(d) && nslot >= 4 && level < 1) {
     const int64_t nmax = d.nup > d.ndown ? d.nup : d.ndown;
     s.o_lu = o;
     o += align8(2 * nmax * nmax * nwb * (int64_t)sizeof(R));
   }
+  const bool fixed = !kMixed<R> && level < 2;
   s.o_fix = o;
-  if (!kMixed<R> || (kind == 1 && d.nmo_used > kFloatRegCols))
+  if (fixed || s.o_bd >= 0)
     o += align8((int64_t)s.nthreads * (kind == 1 ? (kMixed<R> ? 3 : 2) * kFixElAOs : kFixAOs) *
                 (int64_t)sizeof(R));
-  if (kind == 1 && !kMixed<R> && o < s.o_fix + plain_bytes(d)) o = s.o_fix + plain_bytes(d);
-  s.o_ecol = o;
-  if (!kMixed<R>) o += align8((int64_t)s.ncol * 4);
+  if (kind == 1 && !kMixed<R> && level < 2 && o < s.o_fix + plain_bytes(d))
+    o = s.o_fix + plain_bytes(d);
+  s.fix_bytes = o - s.o_fix;
+  s.o_ecol = -1;
+  if (fixed) {
+    s.o_ecol = o;
+    o += align8((int64_t)s.ncol * 4);
+  }
   // the determinant phase works in shared memory when the block's arrays are
   // small (the psi / Metropolis kernels of small molecules), else in HBM scratch
   const int64_t det_bytes = (int64_t)nwb * ep_layout(d, kind == 1 ? 1 : 0).bytes_per_slot;
@@ -541,6 +558,37 @@ __device__ inline void ep_fixed_rows(const Tables<double>& t, const int* ecol, i
     for (int j = 0; j < nmu; ++j) bk[j * rs] = -0.5 * fma(jl, mo[j * rs], bk[j * rs]);
 }
 
+// The same rows by FP64 multiply-adds with W itself, a pass over the AOs per eight columns.
+template <bool KIN, bool CUT>
+__device__ __noinline__ inline void ep_plain_rows(const Tables<double>& t, int nmu, double x,
+                                                  double y, double z, double gx, double gy,
+                                                  double gz, double jl, double* mo, double* bk,
+                                                  int64_t rs, int gb, int ge) {
+  for (int j0 = 0; j0 < nmu; j0 += 8) {
+    double m[8], b[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m[j] = b[j] = 0.0;
+    auto acc = [&](int a, const AOVal<double>& o) {
+      const double k = KIN ? o.lap + 2.0 * (gx * o.gx + gy * o.gy + gz * o.gz) : 0.0;
+      if (is_zero(o.v) && (!KIN || is_zero(k))) return;  // cut primitives
+      const double* const w = t.W + (int64_t)a * t.ncol + j0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        m[j] = fma(o.v, w[j], m[j]);
+        if (KIN) b[j] = fma(k, w[j], b[j]);
+      }
+    };
+    for_each_ao_ep<double, KIN, decltype(acc), CUT>(t, XP<double>{x, 0.0}, XP<double>{y, 0.0},
+                                                    XP<double>{z, 0.0}, acc, gb, ge);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (j0 + j < nmu) {
+        mo[(j0 + j) * rs] = m[j];
+        if (KIN) bk[(j0 + j) * rs] = -0.5 * fma(jl, m[j], b[j]);
+      }
+  }
+}
+
 // Two FP32 multiply-adds in one instruction, each rounded as fmaf.
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t d;
@@ -723,38 +771,45 @@ __device__ inline void ep_electron(const qmc_wf_desc& d, const Tables<R>& t, con
   R* mrow = mo + (int64_t)e * nmu * cs;
   R* brow = KIN ? bk + (int64_t)e * nmu * cs : nullptr;
   if constexpr (!kMixed<R>) {
-    ep_fixed_rows<KIN, true>(t, ecol, nmu, ex.h, ey.h, ez.h, gx, gy, gz, jl,
-                             reinterpret_cast<int2*>(fix), fix_stride, mrow,
-                             brow, cs, 0, t.ngroup);
+    if (ecol)
+      ep_fixed_rows<KIN, true>(t, ecol, nmu, ex.h, ey.h, ez.h, gx, gy, gz, jl,
+                               reinterpret_cast<int2*>(fix), fix_stride, mrow,
+                               brow, cs, 0, t.ngroup);
+    else
+      ep_plain_rows<KIN, true>(t, nmu, ex.h, ey.h, ez.h, gx, gy, gz, jl, mrow, brow, cs, 0,
+                               t.ngroup);
   } else if constexpr (KIN) {
-    if (nmu > kFloatRegCols) {
+    if (bd) {
       ep_float_rows(t, nmu, ex, ey, ez, gx, gy, gz, jl, fix, fix_stride, mrow, brow,
                     bd + (int64_t)e * nmu * cs, cs);
       return;
     }
-    uint64_t m[4], b[4], l[4];  // value, gradient and Laplacian sums
+    for (int j0 = 0; j0 < nmu; j0 += 8) {
+      uint64_t m[4], b[4], l[4];  // value, gradient and Laplacian sums
 #pragma unroll
-    for (int q = 0; q < 4; ++q) m[q] = b[q] = l[q] = 0;
-    auto acc = [&](int a, const AOVal<R>& o) {
-      const ulonglong2* w = reinterpret_cast<const ulonglong2*>(t.W + (int64_t)a * t.ncol);
-      const float g = 2.0f * (gx * o.gx + gy * o.gy + gz * o.gz);
-      const uint64_t xx = pack2(o.v, o.v), yy = pack2(g, g), zz = pack2(o.lap, o.lap);
+      for (int q = 0; q < 4; ++q) m[q] = b[q] = l[q] = 0;
+      auto acc = [&](int a, const AOVal<R>& o) {
+        const ulonglong2* w = reinterpret_cast<const ulonglong2*>(t.W + (int64_t)a * t.ncol + j0);
+        const float g = 2.0f * (gx * o.gx + gy * o.gy + gz * o.gz);
+        const uint64_t xx = pack2(o.v, o.v), yy = pack2(g, g), zz = pack2(o.lap, o.lap);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint64_t c = q % 2 ? w[q / 2].y : w[q / 2].x;
-        m[q] = fma2(xx, c, m[q]);
-        b[q] = fma2(yy, c, b[q]);
-        l[q] = fma2(zz, c, l[q]);
-      }
-    };
-    for_each_ao_ep<R, KIN>(t, ex, ey, ez, acc);
+        for (int q = 0; q < 4; ++q) {
+          const uint64_t c = q % 2 ? w[q / 2].y : w[q / 2].x;
+          m[q] = fma2(xx, c, m[q]);
+          b[q] = fma2(yy, c, b[q]);
+          l[q] = fma2(zz, c, l[q]);
+        }
+      };
+      for_each_ao_ep<R, KIN>(t, ex, ey, ez, acc);
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (j < nmu) {
-        const float x = unpack2(m[j / 2], j % 2);
-        mrow[j * cs] = x;
-        brow[j * cs] = -0.5f * (unpack2(l[j / 2], j % 2) + unpack2(b[j / 2], j % 2) + jl * x);
-      }
+      for (int j = 0; j < 8; ++j)
+        if (j0 + j < nmu) {
+          const float x = unpack2(m[j / 2], j % 2);
+          mrow[(j0 + j) * cs] = x;
+          brow[(j0 + j) * cs] =
+              -0.5f * (unpack2(l[j / 2], j % 2) + unpack2(b[j / 2], j % 2) + jl * x);
+        }
+    }
   } else {
     for (int j0 = 0; j0 < nmu; j0 += JC) {
       uint64_t m[JC / 2];
@@ -1434,12 +1489,15 @@ struct EPPtrs {
   EPShape S;
 };
 
-// The block's tables for the electron-parallel kernels (FP64: W as limbs).
+// The block's tables for the electron-parallel kernels (FP64: W as limbs, unless the
+// shape goes without).
 template <typename R>
 __device__ inline Tables<R> ep_tables(const qmc_wf_desc& d, const EPShape& S, unsigned char* smem) {
   const Tables<R> t = load_tables<R>(d, d.nmo_used, S.ncol, smem + S.o_tab);
-  if constexpr (!kMixed<R>)
-    fix_table(const_cast<R*>(t.W), t.nao, t.ncol, reinterpret_cast<int*>(smem + S.o_ecol));
+  if constexpr (!kMixed<R>) {
+    if (S.o_ecol >= 0)
+      fix_table(const_cast<R*>(t.W), t.nao, t.ncol, reinterpret_cast<int*>(smem + S.o_ecol));
+  }
   return t;
 }
 
@@ -1516,8 +1574,8 @@ __device__ inline void ep_eval(const qmc_wf_desc& d, const Tables<R>& t, const E
         ep_electron<R, JC, KIN>(d, t, pbuf + wl * S.pstride, e, MO + wl, BK + wl, nwb,
                                 &JR[e * nwb + wl], &VR[e * nwb + wl],
                                 reinterpret_cast<R*>(p.smem + S.o_fix) + tid, S.nthreads,
-                                reinterpret_cast<const int*>(p.smem + S.o_ecol),
-                                reinterpret_cast<R*>(p.smem + S.o_bd) + wl);
+                                S.o_ecol >= 0 ? reinterpret_cast<const int*>(p.smem + S.o_ecol) : nullptr,
+                                S.o_bd >= 0 ? reinterpret_cast<R*>(p.smem + S.o_bd) + wl : nullptr);
     }
   }
   __syncthreads();
@@ -1745,7 +1803,7 @@ __device__ __noinline__ inline void ep_plain_walkers(const qmc_wf_desc& d, const
   double* VR = reinterpret_cast<double*>(p.smem + S.o_vrow);
   // the first of these walkers work in the AO slots, which are free now, the others where
   // the block's determinants are
-  const int64_t fit = (S.o_ecol - S.o_fix) / L.bytes_per_slot;
+  const int64_t fit = S.fix_bytes / L.bytes_per_slot;
   int rank = 0;
   for (int q = 0; q < wl; ++q) rank += flag[q] != 0;
   const bool in = rank < fit;
@@ -1755,7 +1813,7 @@ __device__ __noinline__ inline void ep_plain_walkers(const qmc_wf_desc& d, const
   for (int q = 0; q < nwb; ++q)
     if (flag[q])
       plain_rows(d, t, P + q * S.pstride, MO + q, BK + q, JR + q, VR + q, nwb,
-                 reinterpret_cast<double*>(p.smem + S.o_fix), (S.o_ecol - S.o_fix) / 8);
+                 reinterpret_cast<double*>(p.smem + S.o_fix), S.fix_bytes / 8);
   if (tid < 2 * nwb && flag[wl])
     ep_det<double, true, true>(d, L, wbase, wss, wsm ? wl : w0 + wl, slot, MO, BK, wl, nwb,
                                reinterpret_cast<double*>(p.smem + S.o_dref), d.det_table[slot]);

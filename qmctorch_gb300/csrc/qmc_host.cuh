@@ -89,7 +89,10 @@ static inline int64_t scratch_slot_bytes(const qmc_wf_desc* d, int kind) {
 //   wave, the k with the best last-wave fill is taken.
 // * The FP64 local-energy kernel (heaviest electron phase: AO Hessian
 //   diagonals in FP64) keeps one thread per electron (k = 1).
-// Plans are cached per (kernel, device, walker count, shape inputs).
+// * Where no block fits, not even of one walker, the search goes on with the shapes that
+//   need less shared memory (ep_shape's levels).
+// The choices (not the shapes, which depend on more) are cached per (kernel, device,
+// walker count, shape inputs).
 template <typename R, typename K>
 static inline EPShape ep_plan(const qmc_wf_desc& d, int kind, int jc, K kernel, int64_t nw,
                               int bound = 0, bool* single_wave = nullptr) {
@@ -102,26 +105,29 @@ static inline EPShape ep_plan(const qmc_wf_desc& d, int kind, int jc, K kernel, 
   const EPShape s1 = ep_shape<R>(d, kind, 1, jc, ne), s2 = ep_shape<R>(d, kind, 2, jc, ne);
   struct Key {
     const void* kernel;
-    int dev, kind, jc, ne, bound;
-    int64_t nw, smem1, smem2;
+    int dev, kind, jc, ne, bound, nup, nmo, nao;
+    int64_t nw, smem1, smem2, det;
     bool operator==(const Key& o) const {
       return kernel == o.kernel && dev == o.dev && kind == o.kind && jc == o.jc && ne == o.ne &&
-             bound == o.bound && nw == o.nw && smem1 == o.smem1 && smem2 == o.smem2;
+             bound == o.bound && nup == o.nup && nmo == o.nmo && nao == o.nao && nw == o.nw &&
+             smem1 == o.smem1 && smem2 == o.smem2 && det == o.det;
     }
   };
   struct Plan {
-    EPShape s;
-    bool one_wave;
+    int nwb, nslot, level;
+    bool pos_global, one_wave;
   };
-  const Key key{(const void*)kernel, dev, kind, jc, ne, bound, nw, s1.smem, s2.smem};
+  const Key key{(const void*)kernel, dev, kind, jc, ne, bound, d.nup, d.nmo_used, d.nao, nw,
+                s1.smem, s2.smem, ep_layout(d, kind == 1 ? 1 : 0).bytes_per_slot};
   static std::mutex mu;
   static std::vector<std::pair<Key, Plan>> cache;
   {
     std::lock_guard<std::mutex> g(mu);
     for (const auto& kv : cache)
       if (kv.first == key) {
-        if (single_wave) *single_wave = kv.second.one_wave;
-        return kv.second.s;
+        const Plan& c = kv.second;
+        if (single_wave) *single_wave = c.one_wave;
+        return ep_shape<R>(d, kind, c.nwb, jc, c.nslot, c.pos_global, c.level);
       }
   }
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -136,6 +142,7 @@ static inline EPShape ep_plan(const qmc_wf_desc& d, int kind, int jc, K kernel, 
   // no plan gives one wave that way, a second pass moves them to the
   // (L2-resident) scratch, read once per step by the proposal and written on
   // acceptance, which frees a position row per walker of shared memory.
+  for (int level = 0; level < kEPLevels && best.smem < 0; ++level)
   for (int pg = 0; pg < (kind == 2 ? 2 : 1) && !one_wave; ++pg)
   for (int nwb = nwb0; nwb >= 1 && !one_wave; nwb /= 2) {
     // the first block size that fits is kept, except by the persistent
@@ -146,7 +153,7 @@ static inline EPShape ep_plan(const qmc_wf_desc& d, int kind, int jc, K kernel, 
     for (int k = 1; k <= kmax; ++k) {
       const int nslot = (ne + k - 1) / k;
       if (k > 1 && nslot == (ne + k - 2) / (k - 1)) continue;  // same slot count as k - 1
-      const EPShape s = ep_shape<R>(d, kind, nwb, jc, nslot, pg == 1);
+      const EPShape s = ep_shape<R>(d, kind, nwb, jc, nslot, pg == 1, level);
       if (s.nthreads > bound || s.smem > (kMixed<R> ? 200 : 227) * 1024) continue;
       if (prepare_smem(kernel, s.smem) != QMC_OK) continue;
       int occ = 0;
@@ -172,7 +179,7 @@ static inline EPShape ep_plan(const qmc_wf_desc& d, int kind, int jc, K kernel, 
   if (best.smem >= 0) {
     std::lock_guard<std::mutex> g(mu);
     if (cache.size() > 256) cache.clear();
-    cache.emplace_back(key, Plan{best, one_wave});
+    cache.emplace_back(key, Plan{best.nwb, best.nslot, best.level, best.pos_global != 0, one_wave});
   }
   if (single_wave) *single_wave = one_wave;
   return best;

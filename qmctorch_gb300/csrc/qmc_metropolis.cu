@@ -17,8 +17,6 @@ QMC_MET_EXTERN(float, 8)
 QMC_MET_EXTERN(float, 16)
 QMC_MET_EXTERN(float, 24)
 QMC_MET_EXTERN(double, 8)
-QMC_MET_EXTERN(double, 16)
-QMC_MET_EXTERN(double, 24)
 #undef QMC_MET_EXTERN
 }  // namespace qmc
 
@@ -29,7 +27,8 @@ using namespace qmc;
 int qmc_sweep_run(const qmc_wf_desc* d, const qmc_metropolis_args* a, void* stream);
 bool qmc_sweep_eligible(const qmc_wf_desc* d, const qmc_metropolis_args* a);
 
-// column-chunk class of the electron-parallel kernels (JC = 8, 16, 24)
+// column-chunk class of the electron-parallel kernels (FP32: JC = 8, 16, 24; FP64 has one
+// instance, whose batches keep to the classes)
 static inline int mo_chunk_class(int nmo_used) { return nmo_used <= 8 ? 0 : (nmo_used <= 16 ? 1 : 2); }
 
 extern "C" {
@@ -54,9 +53,7 @@ int qmc_metropolis_run(const qmc_wf_desc* d, const qmc_metropolis_args* a, void*
     if (d->nmo_used <= 16) return launch_metropolis<float, 16>(d, a, scr, s);
     return launch_metropolis<float, 24>(d, a, scr, s);
   }
-  if (d->nmo_used <= 8) return launch_metropolis<double, 8>(d, a, scr, s);
-  if (d->nmo_used <= 16) return launch_metropolis<double, 16>(d, a, scr, s);
-  return launch_metropolis<double, 24>(d, a, scr, s);
+  return launch_metropolis<double, 8>(d, a, scr, s);
 }
 
 int qmc_metropolis_plan(const qmc_wf_desc* d, int64_t nwalkers, int32_t* plan) {
@@ -68,9 +65,7 @@ int qmc_metropolis_plan(const qmc_wf_desc* d, int64_t nwalkers, int32_t* plan) {
     if (d->nmo_used <= 16) return plan_metropolis<float, 16>(d, nwalkers, plan);
     return plan_metropolis<float, 24>(d, nwalkers, plan);
   }
-  if (d->nmo_used <= 8) return plan_metropolis<double, 8>(d, nwalkers, plan);
-  if (d->nmo_used <= 16) return plan_metropolis<double, 16>(d, nwalkers, plan);
-  return plan_metropolis<double, 24>(d, nwalkers, plan);
+  return plan_metropolis<double, 8>(d, nwalkers, plan);
 }
 
 int qmc_metropolis_run_batch(const qmc_wf_desc* descs, const qmc_metropolis_args* args,
@@ -102,9 +97,7 @@ int qmc_metropolis_run_batch(const qmc_wf_desc* descs, const qmc_metropolis_args
     if (d->nmo_used <= 16) return launch_metropolis_batch<float, 16>(descs, args, scratch, njobs, s);
     return launch_metropolis_batch<float, 24>(descs, args, scratch, njobs, s);
   }
-  if (d->nmo_used <= 8) return launch_metropolis_batch<double, 8>(descs, args, scratch, njobs, s);
-  if (d->nmo_used <= 16) return launch_metropolis_batch<double, 16>(descs, args, scratch, njobs, s);
-  return launch_metropolis_batch<double, 24>(descs, args, scratch, njobs, s);
+  return launch_metropolis_batch<double, 8>(descs, args, scratch, njobs, s);
 }
 
 }  // extern "C"

@@ -1,5 +1,5 @@
 // One (R, JC) instantiation of the Metropolis kernels; the build compiles this
-// file once per pair with -DQMC_INST_R=<float|double> -DQMC_INST_JC=<8|16|24>.
+// file once per pair with -DQMC_INST_R=<float|double> -DQMC_INST_JC=<8|16|24> (double: 8).
 #include "qmc_metropolis.cuh"
 
 #if !defined(QMC_INST_R) || !defined(QMC_INST_JC)

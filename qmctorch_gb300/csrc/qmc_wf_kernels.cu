@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(EPElBound<R>::kThreads) ep_eloc_kernel(const q
   ep_stage_positions<R>(pos, w0, nw, S.nwb, 3 * d.nelec, S.pstride, P);
   ep_eval<R, JC, true, ELCOOP>(d, t, EPPtrs{smem, S}, P, scr, ss, w0, nw);
   if constexpr (!kMixed<R>) {
-    if (d.det_mode == QMC_DET_EXCITATION && d.ndet[0] + d.ndet[1] > 2)
+    if (S.level < 2 && d.det_mode == QMC_DET_EXCITATION && d.ndet[0] + d.ndet[1] > 2)
       ep_plain_walkers(d, EPPtrs{smem, S}, scr, ss, w0, nw);
   }
   const int tid = threadIdx.x;
@@ -76,9 +76,12 @@ static int launch_psi(const qmc_wf_desc* d, const double* pos, int64_t nw, doubl
 template <typename R>
 static int dispatch_psi(const qmc_wf_desc* d, const double* pos, int64_t nw, double* psi,
                         unsigned char* scr, cudaStream_t s) {
-  if (d->nmo_used <= 8) return launch_psi<R, 8>(d, pos, nw, psi, scr, s);
-  if (d->nmo_used <= 16) return launch_psi<R, 16>(d, pos, nw, psi, scr, s);
-  return launch_psi<R, 24>(d, pos, nw, psi, scr, s);
+  // the columns per pass over the AOs; FP64 sums all of them in one (ep_fixed_rows)
+  if constexpr (kMixed<R>) {
+    if (d->nmo_used > 16) return launch_psi<R, 24>(d, pos, nw, psi, scr, s);
+    if (d->nmo_used > 8) return launch_psi<R, 16>(d, pos, nw, psi, scr, s);
+  }
+  return launch_psi<R, 8>(d, pos, nw, psi, scr, s);
 }
 
 template <typename R, int JC, bool ELCOOP>
