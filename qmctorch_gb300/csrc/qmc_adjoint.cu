@@ -242,24 +242,11 @@ __device__ __noinline__ void adj_sum_values_warp(const qmc_wf_desc& d, const Adj
   const GradShape& S = A.g;
   const int r0 = s ? d.nup : 0, nmu = d.nmo_used, o = s ? d.ndet[0] : 0;
   const MView<double> M = grad_view(k, S.mo, r0, nmu), B = grad_view(k, A.bk, r0, nmu);
-  sum_dispatch(n_, [&](auto Nc) {
-    constexpr int N = decltype(Nc)::value;
-    for (int u = threadIdx.x & 31; u < d.ndet[s]; u += 32) {
-      DetRegs<N> D;
-      D.factor(d, s, u, [&](int i, int c) { return M(i, c); });
-      double tr = 0.0;
-#pragma unroll
-      for (int j = 0; j < N; ++j) {
-        double y[N];
-#pragma unroll
-        for (int i = 0; i < N; ++i) y[i] = B(D.perm[i], D.cols[j]);
-        D.solve(y);
-        tr += y[j];
-      }
-      k.at(S.dv + o + u) = D.det;
-      k.at(A.ov + o + u) = D.det * tr;
-    }
-  });
+  sum_traces(d, s, n_, [&](int i, int c) { return M(i, c); }, [&](int i, int c) { return B(i, c); },
+             [&](int u, double det, double tr) {
+               k.at(S.dv + o + u) = det;
+               k.at(A.ov + o + u) = det * tr;
+             });
 }
 
 __device__ __noinline__ void adj_sum_adjoints_warp(const qmc_wf_desc& d, const AdjShape& A,

@@ -19,6 +19,7 @@
 // mixed method, so that every difference in the inner loops is FP32 work.
 #pragma once
 
+#include "qmc_detsum.cuh"
 #include "qmc_device.cuh"
 #include "qmc_fixdot.cuh"
 
@@ -102,11 +103,6 @@ __host__ __device__ inline EPLayout ep_layout(const qmc_wf_desc& d, int kind) {
 // shared-memory and scratch layouts
 // ---------------------------------------------------------------------------
 constexpr int64_t kDetSmemBytes = 16384;
-// least room of ep_plain_walkers (in the threads' AO slots): Jastrow terms of the
-// electrons, AO values and derivatives of one
-__host__ __device__ inline int64_t plain_bytes(const qmc_wf_desc& d) {
-  return 8 * (4 * (int64_t)d.nelec + 5 * (int64_t)d.nao);
-}
 // AOs per chunk of the FP64 local energy's contraction (two values per AO)
 constexpr int kFixElAOs = 8;
 // FP32 local energy: up to this many columns are summed in registers, in one pass over
@@ -132,15 +128,14 @@ struct EPShape {
   int level;     // what the shape does without to fit (ep_shape)
   int64_t o_bd;         // FP32 local energy: gradient part of the kinetic rows, or -1: registers
   int64_t o_lu;         // the factors of el_diagonal's cooperative phase, or -1: work arrays
-  int64_t o_fix, fix_bytes;  // the threads' AO values (FP64: as limbs)
-  int64_t o_ecol;            // FP64: W's column exponents, or -1: W is not in limbs (ep_plain_rows)
+  int64_t o_fix;   // the threads' AO values (FP64: as limbs)
+  int64_t o_ecol;  // FP64: W's column exponents, or -1: W is not in limbs (ep_plain_rows)
   int64_t o_det;  // determinant-phase work arrays of the block's walkers, or -1: HBM scratch
 };
 
 // level 0: everything that helps; 1: el_diagonal's factors in the work arrays; 2: the least
-// shared memory, without the threads' AO slots and what only they are for (FP64: sums of
-// FP64 multiply-adds, no second evaluation of walkers near a node; FP32 local energy: columns
-// in registers, a pass over the AOs per eight). The plan search takes the first level at
+// shared memory, without the threads' AO slots (FP64: sums of FP64 multiply-adds; FP32 local
+// energy: columns in registers, a pass over the AOs per eight). The plan search takes the first level at
 // which a block of one walker fits.
 constexpr int kEPLevels = 3;
 template <typename R>
@@ -204,9 +199,6 @@ __host__ __device__ inline EPShape ep_shape(const qmc_wf_desc& d, int kind, int 
   if (fixed || s.o_bd >= 0)
     o += align8((int64_t)s.nthreads * (kind == 1 ? (kMixed<R> ? 3 : 2) * kFixElAOs : kFixAOs) *
                 (int64_t)sizeof(R));
-  if (kind == 1 && !kMixed<R> && level < 2 && o < s.o_fix + plain_bytes(d))
-    o = s.o_fix + plain_bytes(d);
-  s.fix_bytes = o - s.o_fix;
   s.o_ecol = -1;
   if (fixed) {
     s.o_ecol = o;
@@ -1168,7 +1160,7 @@ __device__ inline bool el_channel_regs_n(const qmc_wf_desc& d, int spin, CView<R
   }
 }
 
-template <typename R, bool OP, bool PLAIN = false>
+template <typename R, bool OP>
 __device__ inline void ep_det(const qmc_wf_desc& d, const EPLayout& L, unsigned char* scr,
                               int64_t ss, int64_t w, int spin, R* mo_s, const R* bk_s, int wl,
                               int nwb, double* dref, const int* dtab) {
@@ -1214,7 +1206,7 @@ __device__ inline void ep_det(const qmc_wf_desc& d, const EPLayout& L, unsigned 
     wk.X = MView<R>{rows + n * cs, rs, cs};
   }
   double* ov = OP ? rptr<double>(scr, L.ov, ss, w) + (spin ? d.ndet[0] * ss : 0) : nullptr;
-  spin_channel<R, OP, T, PLAIN>(d, spin, mo, bk, wk, SpinOut<T>{dv, ov, ss, &dref[spin * nwb + wl]});
+  spin_channel<R, OP, T>(d, spin, mo, bk, wk, SpinOut<T>{dv, ov, ss, &dref[spin * nwb + wl]});
 }
 
 // Block-cooperative LU of the psi / Metropolis determinant phase for spin
@@ -1535,6 +1527,71 @@ __device__ inline void ep_combine(const qmc_wf_desc& d, const Tables<R>& t, cons
   }
 }
 
+// FP64 local energy, walkers next to a node of the ground determinant: an excitation ratio
+// (a determinant relative to the ground one) of K amplifies the rounding of A^-1 A_virt and
+// A^-1 B by about K^2 in the double excitations' 2 x 2 minors. Above kElRatio (and where the
+// ground determinant is zero) a spin's determinants and traces are formed one by one,
+// from the same MO rows, whatever the block's other walkers do. The instance with small
+// channels (ELCOOP false) only: larger ones do not fit the registers.
+constexpr double kElRatio = 256.0;
+__device__ __forceinline__ bool ep_sum_applies(const qmc_wf_desc& d) {
+  return d.det_mode == QMC_DET_EXCITATION && d.ndet[0] + d.ndet[1] > 2;
+}
+
+__device__ __noinline__ inline void ep_sum_warp(const qmc_wf_desc& d, int s, int n, const double* mo,
+                                                const double* bk, int64_t rs, int64_t cs,
+                                                double* dv, double* ov, int64_t ss) {
+  sum_traces(d, s, n, [&](int i, int c) { return mo[i * rs + c * cs]; },
+             [&](int i, int c) { return bk[i * rs + c * cs]; },
+             [&](int u, double det, double tr) {
+               dv[u * ss] = det;
+               ov[u * ss] = tr;
+             });
+}
+
+// Behind the determinant phase (its values need no barrier between): every thread of the
+// block calls it; the caller's barrier follows.
+__device__ inline void ep_sum_channels(const qmc_wf_desc& d, const EPPtrs& p, const EPLayout& L,
+                                       unsigned char* dbase, int64_t dss, bool dsm, int64_t w0,
+                                       int64_t nw) {
+  const EPShape& S = p.S;
+  const int nwb = S.nwb, tid = threadIdx.x;
+  int* const flag = reinterpret_cast<int*>(p.smem + S.o_iel);  // [walker], 2 bits
+  double* const dref = reinterpret_cast<double*>(p.smem + S.o_dref);
+  auto values = [&](const Region& r, int s, int wl) {
+    return rptr<double>(dbase, r, dss, dsm ? wl : w0 + wl) + (s ? d.ndet[0] * dss : 0);
+  };
+  bool any = false;
+  if (tid < 2 * nwb) {
+    const int s = tid / nwb, wl = tid - s * nwb, n = s ? d.ndown : d.nup;
+    if (w0 + wl < nw && n > 0 && n <= kSumN) {
+      const double* const dv = values(L.dv, s, wl);
+      any = dref[tid] == 0.0;
+      for (int u = 0; u < d.ndet[s]; ++u)
+        any |= __double2hiint(fabs(dv[u * dss])) > __double2hiint(kElRatio);
+    }
+  }
+  if (!__syncthreads_or(any)) return;
+  if (tid < nwb) flag[tid] = 0;
+  __syncthreads();
+  if (any) {
+    const int s = tid / nwb;
+    atomicOr(flag + tid - s * nwb, 1 << s);
+    dref[tid] = 1.0;
+  }
+  __syncthreads();
+  const int64_t cs = nwb, rs = (int64_t)d.nmo_used * nwb;
+  const double* const MO = reinterpret_cast<const double*>(p.smem + S.o_mo);
+  const double* const BK = reinterpret_cast<const double*>(p.smem + S.o_bk);
+  for (int ch = tid >> 5; ch < 2 * nwb; ch += blockDim.x >> 5) {
+    const int s = ch / nwb, wl = ch - s * nwb;
+    if (!((flag[wl] >> s) & 1)) continue;
+    const int64_t at = (s ? d.nup : 0) * rs + wl;
+    ep_sum_warp(d, s, s ? d.ndown : d.nup, MO + at, BK + at, rs, cs, values(L.dv, s, wl),
+                values(L.ov, s, wl), dss);
+  }
+}
+
 // Evaluate psi (and, with KIN, the kinetic energy and potentials) for the
 // block's walkers at split positions `pbuf` (shared memory, [nwb][3 nelec]).
 // Results in shared memory: psi[wl], and with KIN kin[wl], v[wl] (V_en + V_ee),
@@ -1593,232 +1650,11 @@ __device__ inline void ep_eval(const qmc_wf_desc& d, const Tables<R>& t, const E
       ep_det<R, KIN>(d, L, dbase, dss, dsm ? wl : w0 + wl, spin, MO, BK, wl, nwb, DREF,
                      d.det_table[spin]);
   }
+  if constexpr (KIN && !kMixed<R> && !ELCOOP) {
+    if (ep_sum_applies(d)) ep_sum_channels(d, p, L, dbase, dss, dsm, w0, nw);
+  }
   __syncthreads();
   if (tid < nwb && w0 + tid < nw) ep_combine<R, KIN>(d, t, p, dbase, dss, dsm, w0, tid);
-}
-
-// ---------------------------------------------------------------------------
-// FP64 local energy: walkers next to a node of the ground determinant
-// ---------------------------------------------------------------------------
-// Where an excitation ratio (a determinant relative to the ground one) exceeds
-// kPlainRatio, the 2 x 2 minors of the double excitations cancel, and the local
-// energy amplifies the last bits of everything before it by about the ratio's
-// square (H2O: up to 1e-4 Ha, one walker in some 1e5). Such a walker is evaluated
-// again with the plain sequence of FP64 instructions (FP64-pipe exp, square root,
-// reciprocal, multiply-adds in AO order, IEEE pivots), whatever the other walkers of
-// its block do: its energy does not depend on the fixed-point functions' last bits.
-// H2O: about one block of 16 walkers in 100 does the second evaluation.
-constexpr double kPlainRatio = 4096.0;
-
-// AOs of group g of the electron at (x, y, z), with derivatives.
-template <typename F>
-__device__ inline void plain_group(const Tables<double>& t, int g, double x, double y, double z,
-                                   const F& f) {
-  const int A = t.group_atom[g];
-  const double dx = x - t.atom_p[3 * A].h, dy = y - t.atom_p[3 * A + 1].h,
-               dz = z - t.atom_p[3 * A + 2].h;
-  const double r2 = dx * dx + dy * dy + dz * dz;
-  if (t.radial != QMC_RADIAL_GTO) {
-    group_sto<double, true>(t, g, dx, dy, dz, r2, f);
-    return;
-  }
-  const int np = t.group_prim[g + 1] - t.group_prim[g], ga = t.group_ao[g];
-  const int kind = t.group_kind[g];
-  double sh[2][3];  // radial sums that components share
-  for (int a = ga; a < t.group_ao[g + 1]; ++a) {
-    const int c = a - ga;
-    const int share = kind == GK_P ? 0 : (kind == GK_D ? (c == 0 || c == 3 || c == 5 ? 0 : 1) : -1);
-    double G0 = 0.0, G1 = 0.0, G2 = 0.0;
-    if (share >= 0 && c > share) {
-      G0 = sh[share][0];
-      G1 = sh[share][1];
-      G2 = sh[share][2];
-    } else {
-      for (int p = 0; p < np; ++p) {
-        const int wi = t.ao_wofs[a] + p;
-        const double al = t.walpha[wi];
-        if (al * r2 > (double)kRadialCut) continue;
-        const double e0 = exp_tang(-al * r2), e1 = al * e0, e2 = al * e1, w = t.wd[wi];
-        G0 = fma(w, e0, G0);
-        G1 = fma(w, e1, G1);
-        G2 = fma(w, e2, G2);
-      }
-      if (share >= 0) {
-        sh[share][0] = G0;
-        sh[share][1] = G1;
-        sh[share][2] = G2;
-      }
-    }
-    const int kx = t.ao_k[3 * a], ky = t.ao_k[3 * a + 1], kz = t.ao_k[3 * a + 2];
-    const double px = pk0(dx, kx), py = pk0(dy, ky), pz = pk0(dz, kz);
-    const double qx = pk1(dx, kx) * py * pz, qy = px * pk1(dy, ky) * pz,
-                 qz = px * py * pk1(dz, kz);
-    const double lapP = pk2(dx, kx) * py * pz + px * pk2(dy, ky) * pz + px * py * pk2(dz, kz);
-    f(a, ao_from<double, true>(px * py * pz, qx, qy, qz, lapP, kx + ky + kz, dx, dy, dz, r2, G0,
-                               G1, G2, t.vscale ? t.vscale[a] : 1.0));
-  }
-}
-
-// Jastrow and Coulomb rows of electron e; jt: grad U and lap U + |grad U|^2.
-__device__ inline void plain_jastrow(const qmc_wf_desc& d, const Tables<double>& t,
-                                     const XP<double>* pw, int e, double* jrow, double* vrow,
-                                     double* jt) {
-  const int ne = d.nelec;
-  const double x = pw[3 * e].h, y = pw[3 * e + 1].h, z = pw[3 * e + 2].h;
-  double gx = 0.0, gy = 0.0, gz = 0.0, ks = 0.0, vs = 0.0, lp = 0.0, kn = 0.0;
-  const double w = d.use_jastrow ? __ldg(d.jastrow_w) : 0.0;
-  for (int j = 0; j < ne; ++j) {
-    if (j == e) continue;
-    const double dx = x - pw[3 * j].h, dy = y - pw[3 * j + 1].h, dz = z - pw[3 * j + 2].h;
-    const double r = sqrt_nr(dx * dx + dy * dy + dz * dz);
-    vs += rcp_nr(r);
-    if (d.use_jastrow) {
-      const double w0 = same_spin(d, e, j) ? 0.25 : 0.5;
-      const double iu = rcp_nr(1.0 + w * r);
-      ks += w0 * r * iu;
-      const double ir = rcp_nr(r);
-      const double k1 = w0 * iu * iu;
-      gx += k1 * dx * ir;
-      gy += k1 * dy * ir;
-      gz += k1 * dz * ir;
-      lp += 2.0 * k1 * ir - 2.0 * w * k1 * iu;
-    }
-  }
-  if (d.use_jastrow_en) {
-    const double wn = __ldg(d.jastrow_en_w);
-    for (int A = 0; A < t.natom; ++A) {
-      const double dx = x - t.en_p[3 * A].h, dy = y - t.en_p[3 * A + 1].h,
-                   dz = z - t.en_p[3 * A + 2].h;
-      const double r = sqrt_nr(dx * dx + dy * dy + dz * dz);
-      const double iu = rcp_nr(1.0 + wn * r);
-      kn += r * iu;
-      const double ir = rcp_nr(r);
-      const double k1 = iu * iu;
-      gx += k1 * dx * ir;
-      gy += k1 * dy * ir;
-      gz += k1 * dz * ir;
-      lp += 2.0 * k1 * ir - 2.0 * wn * k1 * iu;
-    }
-  }
-  const double jl = lp + gx * gx + gy * gy + gz * gz;
-  *jrow = 0.5 * ks + kn;
-  double ven = 0.0;
-  for (int A = 0; A < t.natom; ++A) {
-    const double dx = x - t.atom_p[3 * A].h, dy = y - t.atom_p[3 * A + 1].h,
-                 dz = z - t.atom_p[3 * A + 2].h;
-    ven -= t.atom_z[A] * rcp_nr(sqrt_nr(dx * dx + dy * dy + dz * dz));
-  }
-  *vrow = 0.5 * vs + ven;
-  jt[0] = gx;
-  jt[1] = gy;
-  jt[2] = gz;
-  jt[3] = jl;
-}
-
-// MO and kinetic rows of one walker by the whole block. An FP64 warp instruction costs
-// its 64 cycles with one active lane as with 32, so the work is dealt out: a thread
-// per (electron, AO group) puts values and derivatives into `buf`, one per (electron,
-// column) sums them in AO order (H2O: a block with such a walker took 172 us more with a
-// thread per electron, 104 us now).
-__device__ inline void plain_rows(const qmc_wf_desc& d, const Tables<double>& t,
-                                  const XP<double>* pw, double* mo, double* bk, double* jrow,
-                                  double* vrow, int nwb, double* buf, int64_t nbuf) {
-  const int tid = threadIdx.x, nt = blockDim.x, ne = d.nelec, nao = d.nao, nmu = d.nmo_used;
-  const int64_t room = (nbuf - 4 * ne) / (5 * nao);
-  const int ec = room < ne ? (int)room : ne;
-  double* const ao = buf + 4 * ne;
-  const int skip = nt >= 64 ? 32 : 0;  // the first warp has the Jastrow rows
-  if (tid < 32)
-    for (int e = tid; e < ne; e += nt < 32 ? nt : 32)
-      plain_jastrow(d, t, pw, e, jrow + e * nwb, vrow + e * nwb, buf + 4 * e);
-  for (int e0 = 0; e0 < ne; e0 += ec) {
-    const int ne1 = ne - e0 < ec ? ne - e0 : ec;
-    for (int i = tid - skip; i >= 0 && i < ne1 * t.ngroup; i += nt - skip) {
-      const int el = i / t.ngroup, e = e0 + el;
-      double* const row = ao + (int64_t)el * nao * 5;
-      plain_group(t, i - el * t.ngroup, pw[3 * e].h, pw[3 * e + 1].h, pw[3 * e + 2].h,
-                  [&](int a, const AOVal<double>& o) {
-                    double* const q = row + a * 5;
-                    q[0] = o.v;
-                    q[1] = o.gx;
-                    q[2] = o.gy;
-                    q[3] = o.gz;
-                    q[4] = o.lap;
-                  });
-    }
-    __syncthreads();
-    for (int i = tid; i < ne1 * nao; i += nt) {
-      const double* const g = buf + 4 * (e0 + i / nao);
-      double* const q = ao + (int64_t)i * 5;
-      q[1] = 2.0 * (g[0] * q[1] + g[1] * q[2] + g[2] * q[3]);
-    }
-    __syncthreads();
-    for (int i = tid; i < ne1 * nmu; i += nt) {
-      const int el = i / nmu, j = i - el * nmu;
-      const double* q = ao + (int64_t)el * nao * 5;
-      double a0 = 0.0, ad = 0.0, al = 0.0;
-      for (int a = 0; a < nao; ++a, q += 5) {
-        const double w = t.W[(int64_t)a * t.ncol + j];
-        a0 = fma(q[0], w, a0);
-        ad = fma(q[1], w, ad);
-        al = fma(q[4], w, al);
-      }
-      const int64_t at = (int64_t)((e0 + el) * nmu + j) * nwb;
-      mo[at] = a0;
-      bk[at] = -0.5 * (al + ad + buf[4 * (e0 + el) + 3] * a0);
-    }
-    __syncthreads();
-  }
-}
-
-// After ep_eval<double, JC, true>: re-evaluates the block's walkers with a large
-// excitation ratio. Every thread of the block calls it.
-__device__ __noinline__ inline void ep_plain_walkers(const qmc_wf_desc& d, const EPPtrs& p,
-                                                     unsigned char* scr, int64_t ss, int64_t w0,
-                                                     int64_t nw) {
-  const EPShape& S = p.S;
-  const int nwb = S.nwb, tid = threadIdx.x;
-  const EPLayout L = ep_layout(d, 1);
-  const bool dsm = S.o_det >= 0;
-  unsigned char* const dbase = dsm ? p.smem + S.o_det : scr;
-  const int64_t dss = dsm ? nwb : ss;
-  int* const flag = reinterpret_cast<int*>(p.smem + S.o_iel);
-  const int slot = tid / nwb, wl = tid - slot * nwb;
-  bool any = false;
-  if (tid < nwb) {
-    if (w0 + wl < nw) {
-      const double* dv = rptr<double>(dbase, L.dv, dss, dsm ? wl : w0 + wl);
-      for (int u = 0; u < d.ndet[0] + d.ndet[1]; ++u)
-        any |= __double2hiint(fabs(dv[u * dss])) > __double2hiint(kPlainRatio);
-    }
-    flag[wl] = any;
-  }
-  if (!__syncthreads_or(any)) return;
-  // W itself again (ep_tables keeps it as limbs)
-  const Tables<double> t = load_tables<double>(d, d.nmo_used, S.ncol, p.smem + S.o_tab);
-  const XP<double>* P = reinterpret_cast<const XP<double>*>(p.smem + S.o_pos);
-  double* MO = reinterpret_cast<double*>(p.smem + S.o_mo);
-  double* BK = reinterpret_cast<double*>(p.smem + S.o_bk);
-  double* JR = reinterpret_cast<double*>(p.smem + S.o_jrow);
-  double* VR = reinterpret_cast<double*>(p.smem + S.o_vrow);
-  // the first of these walkers work in the AO slots, which are free now, the others where
-  // the block's determinants are
-  const int64_t fit = S.fix_bytes / L.bytes_per_slot;
-  int rank = 0;
-  for (int q = 0; q < wl; ++q) rank += flag[q] != 0;
-  const bool in = rank < fit;
-  unsigned char* const wbase = in ? p.smem + S.o_fix + (rank - wl) * (int)sizeof(double) : dbase;
-  const int64_t wss = in ? fit : dss;
-  const bool wsm = in || dsm;
-  for (int q = 0; q < nwb; ++q)
-    if (flag[q])
-      plain_rows(d, t, P + q * S.pstride, MO + q, BK + q, JR + q, VR + q, nwb,
-                 reinterpret_cast<double*>(p.smem + S.o_fix), S.fix_bytes / 8);
-  if (tid < 2 * nwb && flag[wl])
-    ep_det<double, true, true>(d, L, wbase, wss, wsm ? wl : w0 + wl, slot, MO, BK, wl, nwb,
-                               reinterpret_cast<double*>(p.smem + S.o_dref), d.det_table[slot]);
-  __syncthreads();
-  if (tid < nwb && flag[wl]) ep_combine<double, true>(d, t, p, wbase, wss, wsm, w0, wl);
 }
 
 // Stage the positions of walkers [w0, w0 + nwb) into shared memory as split

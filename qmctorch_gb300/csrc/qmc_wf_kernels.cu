@@ -41,10 +41,6 @@ __global__ void __launch_bounds__(EPElBound<R>::kThreads) ep_eloc_kernel(const q
   XP<R>* P = reinterpret_cast<XP<R>*>(smem + S.o_pos);
   ep_stage_positions<R>(pos, w0, nw, S.nwb, 3 * d.nelec, S.pstride, P);
   ep_eval<R, JC, true, ELCOOP>(d, t, EPPtrs{smem, S}, P, scr, ss, w0, nw);
-  if constexpr (!kMixed<R>) {
-    if (S.level < 2 && d.det_mode == QMC_DET_EXCITATION && d.ndet[0] + d.ndet[1] > 2)
-      ep_plain_walkers(d, EPPtrs{smem, S}, scr, ss, w0, nw);
-  }
   const int tid = threadIdx.x;
   if (tid < S.nwb && w0 + tid < nw) {
     const double k = reinterpret_cast<const double*>(smem + S.o_kin)[tid];
