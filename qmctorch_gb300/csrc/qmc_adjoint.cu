@@ -253,66 +253,70 @@ __device__ __noinline__ void adj_sum_adjoints_warp(const qmc_wf_desc& d, const A
                                                    const GradWork& k, const AdjCold& cold, int s,
                                                    int n_) {
   const GradShape& S = A.g;
-  const int lane = threadIdx.x & 31, r0 = s ? d.nup : 0, nmu = d.nmo_used, nd = d.ndet[s];
+  const int r0 = s ? d.nup : 0, nmu = d.nmo_used, nd = d.ndet[s];
   const int nmax = d.nup > d.ndown ? d.nup : d.ndown;
   const int so = s ? d.ndet[0] : 0, oo = s ? 0 : d.ndet[0];
   const double is = k.at(S.val + GV_INV), R = k.at(A.r);
   const MView<double> M = grad_view(k, S.mo, r0, nmu), L = grad_view(k, S.lu, r0, nmu),
                       B = grad_view(k, A.bk, r0, nmu);
   const MView<double> GB = adj_cold(cold, 4 * (int64_t)nmax * nmax + (int64_t)r0 * nmu, nmu);
-  for (int i = lane; i < n_ * nmu; i += 32) L(i / nmu, i % nmu) = GB(i / nmu, i % nmu) = 0.0;
-  __syncwarp();
   sum_dispatch(n_, [&](auto Nc) {
     constexpr int N = decltype(Nc)::value;
     for (int u0 = 0; u0 < nd; u0 += 32) {
-      const int u = u0 + lane, m = nd - u0 < 32 ? nd - u0 : 32;
+      const SumLanes l = sum_lanes(nd, N, u0);
       // d KE = dT D_u dT_u + (dD D_u + dT T_u D_u) d log D_u
       double dT = 0.0, dD = 0.0, t = 0.0, sd = 0.0;
-      if (u < nd)
-        for (int c = 0; c < d.ncfg; ++c) {
-          if (__ldg(d.cfg_det[s] + c) != u) continue;
-          const int v = oo + __ldg(d.cfg_det[1 - s] + c);
-          const double w = __ldg(d.ci_weight + c) * is;
-          dT = fma(w, k.at(S.dv + v), dT);
-          dD = fma(w, k.at(A.ov + v) - R * k.at(S.dv + v), dD);
-        }
-      const bool on = u < nd && !(dT == 0.0 && dD == 0.0);
+      sum_configs(
+          d, s, l.u,
+          [&](int v, double& a, double& b) {
+            a = k.at(S.dv + oo + v);
+            b = k.at(A.ov + oo + v) - R * a;
+          },
+          [&](double w, double a, double b) {
+            dT = fma(w * is, a, dT);
+            dD = fma(w * is, b, dD);
+          });
+      const bool on = l.u < nd && !(dT == 0.0 && dD == 0.0);
       DetRegs<N> D;
       double X[N][N];  // [column][row] of A_u^-1
       if (on) {
-        D.factor(d, s, u, [&](int i, int c) { return M(i, c); });
+        D.factor(d, s, l.u, [&](int i, int c) { return M(i, c); });
 #pragma unroll
         for (int i = 0; i < N; ++i) D.unit(i, X[i]);
         t = dT * D.det;
-        sd = fma(dT, k.at(A.ov + so + u), dD * D.det);
+        sd = fma(dT, k.at(A.ov + so + l.u), dD * D.det);
       }
+#pragma unroll 1
+      for (int i0 = 0; i0 < N; i0 += l.groups) {
+        const int i = i0 + l.g;
+        double y[N], z1[N];  // rows of G_A and G_B, with column i of X B_u X
 #pragma unroll
-      for (int i = 0; i < N; ++i) {
-        double y[N];  // column i of X B_u X
+        for (int j = 0; j < N; ++j) y[j] = z1[j] = 0.0;
         if (on) {
-          double z[N];
+          double xi[N], z[N];
+#pragma unroll
+          for (int c = 0; c < N; ++c) {
+            xi[c] = X[0][c];
+#pragma unroll
+            for (int q = 1; q < N; ++q) xi[c] = q == i ? X[q][c] : xi[c];
+          }
 #pragma unroll
           for (int r = 0; r < N; ++r) {
             z[r] = 0.0;
 #pragma unroll
-            for (int c = 0; c < N; ++c) z[r] = fma(B(r, D.cols[c]), X[i][c], z[r]);
+            for (int c = 0; c < N; ++c) z[r] = fma(B(r, D.cols[c]), xi[c], z[r]);
           }
 #pragma unroll
           for (int j = 0; j < N; ++j) {
             y[j] = 0.0;
 #pragma unroll
             for (int c = 0; c < N; ++c) y[j] = fma(X[c][j], z[c], y[j]);
+            y[j] = sd * xi[j] - t * y[j];
+            z1[j] = t * xi[j];
           }
         }
-        for (int q = 0; q < m; ++q) {
-          if (lane == q && on)
-#pragma unroll
-            for (int j = 0; j < N; ++j) {
-              L(i, D.cols[j]) += sd * X[i][j] - t * y[j];
-              GB(i, D.cols[j]) += t * X[i][j];
-            }
-          __syncwarp();
-        }
+        sum_columns<N>(l, D.cols, y, N, on, nd, i0, nmu, u0 == 0, L);
+        sum_columns<N>(l, D.cols, z1, N, on, nd, i0, nmu, u0 == 0, GB);
       }
     }
   });

@@ -41,7 +41,10 @@ namespace qmc {
 // (without the l terms for the other spin), f_v(i) = sum_k A'^-1(k, i) F(k, v),
 // F = d Sigma / d X (qmc_grad.cuh); the moved electron's comes from one pass over
 // its AOs. Explicit mode (CAS), and a proposal with a large excitation ratio
-// (kGradRatio), refactor the moved spin's determinants.
+// (kGradRatio), refactor the moved spin's determinants. A spin that has such a ratio at the
+// start, or a ground determinant of zero, has no use of A^-1 and X there: its
+// determinants are summed one by one at the start and at every proposal, whichever
+// electron moves.
 struct DriftShape {
   int nwb, nslot, nthreads, ncol;
   int64_t o_wl, o_ecol, o_fix;  // W as limbs, its column exponents, the threads' AO limbs
@@ -50,14 +53,25 @@ struct DriftShape {
   // (accepted and proposed), Jastrow gradient, the moved electron's MO row, its
   // partial rows, r, t, X', F of both spins, the proposal's determinants, G of
   // the moved electron, partial sums, scalars
-  int xs, dr, gj, phi, part, r, t, xp, f, dvf, g, red, val, hot;
+  int xs, dr, gj, phi, part, r, t, xp, f, fs, dvf, g, red, val, hot;  // fs: a spin's F
   // cold (scratch): MO values and gradients, LU | X, Z | m, A^-1 by columns,
-  // determinants, Jastrow of the start, pivots, work of the explicit sums
-  int ma, mg, lx, zm, inv, dv0, jg0, ju, jen, piv, lu, ginv, gx, cold;
+  // determinants, Jastrow of the start, pivots, work of the explicit sums, cofactors of the
+  // start's determinants (of a spin that sums them, [determinant][row][column])
+  int ma, mg, lx, zm, inv, dv0, jg0, ju, jen, piv, lu, ginv, gx, cof, cofs, cold;  // cofs: a spin's
 };
+// scalars: Sigma, q, det A of the start's spins (1 where the spin sums its determinants),
+// whether the moved spin sums them, the accepted drift's half, the accepted electron and its
+// position, the start's spins that sum their determinants, the moved electron
 enum { DV_SIGMA = 0, DV_Q = 1, DV_DET = 2, DV_FLAG = 4, DV_CUR = 5, DV_EACC = 6, DV_XACC = 7,
-       DV_N = 10 };
+       DV_START = 10, DV_MOVED = 12, DV_N = 13 };
 constexpr int kDriftRed = 6;  // partial sums per slot: du, a1, a2, the moved electron's grad U
+
+// Whether a spin's sums at a proposal that leaves its rows alone take the start's cofactors
+// from the scratch (excitation mode, few enough for a warp's lanes).
+__host__ __device__ inline bool drift_cofactors(const qmc_wf_desc& d, int s) {
+  const int n = s ? d.ndown : d.nup;
+  return d.det_mode == QMC_DET_EXCITATION && n <= kSumN && d.ndet[s] <= 32;
+}
 
 static DriftShape drift_shape(const qmc_wf_desc& d, int nwb, int nslot, bool in_smem) {
   DriftShape s;
@@ -83,7 +97,8 @@ static DriftShape drift_shape(const qmc_wf_desc& d, int nwb, int nslot, bool in_
   s.r = take(nmax);
   s.t = take(nv);
   s.xp = take(nmax * nv);
-  s.f = take(2 * nmax * nv);
+  s.fs = nmax * nv;
+  s.f = take(2 * s.fs);
   s.dvf = take(d.ndet[0] > d.ndet[1] ? d.ndet[0] : d.ndet[1]);
   s.g = take(nmu);
   s.red = take(nslot * kDriftRed);
@@ -103,6 +118,12 @@ static DriftShape drift_shape(const qmc_wf_desc& d, int nwb, int nslot, bool in_
   s.lu = take(2 * nmax * nmax);
   s.ginv = take(2 * nmax * nmax);
   s.gx = take(ne * nmu);
+  s.cofs = 0;
+  for (int q = 0; q < 2; ++q) {
+    const int n = q ? d.ndown : d.nup, m = drift_cofactors(d, q) ? d.ndet[q] * n * n : 0;
+    s.cofs = m > s.cofs ? m : s.cofs;
+  }
+  s.cof = take(2 * s.cofs);
   s.cold = o;
   s.o_wl = (tables_smem_bytes<double>(d, s.ncol) + 15) & ~int64_t(15);
   s.o_ecol = s.o_wl + (int64_t)d.nao * s.ncol * 8;
@@ -181,21 +202,155 @@ __device__ __noinline__ void drift_explicit(const qmc_wf_desc& d, const DriftSha
   }
 }
 
-// The same by a warp for a proposal with a large ratio (n <= kSumN): the determinants
-// to `dvf`, G to gx.
+// A lane's determinant for the sums of a few walkers' spins (start_sums and below). Rolled,
+// in local memory, where sum_warp's is unrolled in registers: a walker in some hundred
+// sums, so what counts here is what the code costs the others (registers around the call,
+// instruction cache: H2O without any sum 5.05 -> 4.71 ms for 50 steps), and the time of one sum is the
+// same (it waits for the FP64 pipe, which the block's other warps and the SM's other block hold).
+struct DetSum {
+  double a[kSumN * kSumN], det;    // factors, 1 / U_kk on the diagonal
+  int perm[kSumN], cols[kSumN];    // the row of A that row k of the factors came from
+
+  // Factors the columns of unique determinant u of n electrons; row(i, c): MO c of the
+  // spin's electron i.
+  template <typename Row>
+  __device__ __forceinline__ void factor(const qmc_wf_desc& d, int s, int n, int u, const Row& row) {
+    det_columns(d, s, u, cols);
+    double v[kSumN * kSumN];  // all loads in flight together
+#pragma unroll
+    for (int i = 0; i < kSumN; ++i)
+#pragma unroll
+      for (int j = 0; j < kSumN; ++j) v[i * kSumN + j] = i < n && j < n ? row(i, cols[j]) : 0.0;
+#pragma unroll
+    for (int i = 0; i < kSumN * kSumN; ++i) a[i] = v[i];
+    det = 1.0;
+#pragma unroll 1
+    for (int k = 0; k < n; ++k) perm[k] = k;
+#pragma unroll 1
+    for (int k = 0; k < n; ++k) {
+      int p = k;
+      double amax = fabs(a[k * kSumN + k]);
+#pragma unroll 1
+      for (int i = k + 1; i < n; ++i) {
+        const double x = fabs(a[i * kSumN + k]);
+        if (x > amax) {
+          amax = x;
+          p = i;
+        }
+      }
+      if (p != k) {
+        det = -det;
+        const int q = perm[k];
+        perm[k] = perm[p];
+        perm[p] = q;
+#pragma unroll 1
+        for (int j = 0; j < n; ++j) {
+          const double x = a[k * kSumN + j];
+          a[k * kSumN + j] = a[p * kSumN + j];
+          a[p * kSumN + j] = x;
+        }
+      }
+      const double akk = a[k * kSumN + k];
+      det *= akk;
+      const double inv = akk != 0.0 ? prcp(akk) : 0.0;
+      a[k * kSumN + k] = inv;
+#pragma unroll 1
+      for (int i = k + 1; i < n; ++i) {
+        const double l = a[i * kSumN + k] * inv;
+        a[i * kSumN + k] = l;
+#pragma unroll 1
+        for (int j = k + 1; j < n; ++j)
+          a[i * kSumN + j] = fma(-l, a[k * kSumN + j], a[i * kSumN + j]);
+      }
+    }
+  }
+  // A x = b for b in the factors' row order
+  __device__ __forceinline__ void solve(double* x, int n) const {
+#pragma unroll 1
+    for (int i = 1; i < n; ++i) {
+      double v = x[i];
+#pragma unroll 1
+      for (int k = 0; k < i; ++k) v = fma(-a[i * kSumN + k], x[k], v);
+      x[i] = v;
+    }
+#pragma unroll 1
+    for (int i = n - 1; i >= 0; --i) {
+      double v = x[i];
+#pragma unroll 1
+      for (int k = i + 1; k < n; ++k) v = fma(-a[i * kSumN + k], x[k], v);
+      x[i] = v * a[i * kSumN + i];
+    }
+  }
+  __device__ __forceinline__ void unit(int col, double* x, int n) const {  // column of A^-1
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) x[i] = perm[i] == col ? 1.0 : 0.0;
+    solve(x, n);
+  }
+};
+
+// The same by a warp for a spin of n <= kSumN electrons (dst: null where the
+// determinants are there already; ADJ: with G; cof: keeps det_u A_u^-T where the shape has
+// room for it).
+template <bool ADJ>
 __device__ __noinline__ void drift_sum_warp(const qmc_wf_desc& d, const DriftShape& S,
-                                            const DriftWork& k, int s, int n, int er) {
-  const int r0 = s ? d.nup : 0, nmu = d.nmo_used;
-  const double* const oth = k.cp + (int64_t)(S.dv0 + (s ? 0 : d.ndet[0])) * k.cs;
-  sum_dispatch(n, [&](auto N) {
-    sum_warp<decltype(N)::value, true>(
-        d, s,
-        [&](int i, int c) {
-          return r0 + i == er ? k.H(S.phi + c) : k.C(S.ma + (r0 + i) * nmu + c);
-        },
-        [&](int u, double det) { k.H(S.dvf + u) = det; }, [&](int u) { return oth[u * k.cs]; },
-        [&](int i, int c) -> double& { return k.C(S.gx + (r0 + i) * nmu + c); });
-  });
+                                            const DriftWork& k, int s, int n, int er, double* dst,
+                                            int64_t ds, const double* oth, int64_t os, bool cof) {
+  const int r0 = s ? d.nup : 0, nmu = d.nmo_used, nd = d.ndet[s];
+  for (int u0 = 0; u0 < nd; u0 += 32) {
+    const SumLanes l = sum_lanes(nd, n, u0);
+    DetSum D;
+    if (l.u < nd) {
+      D.factor(d, s, n, l.u, [&](int i, int c) {
+        return r0 + i == er ? k.H(S.phi + c) : k.C(S.ma + (r0 + i) * nmu + c);
+      });
+      if (dst && l.g == 0) dst[l.u * ds] = D.det;
+    }
+    if (!ADJ) continue;
+    double coef = 0.0;
+    sum_configs(d, s, l.u, [&](int v, double& a, double&) { a = oth[v * os]; },
+                [&](double w, double a, double) { coef = fma(w, a, coef); });
+    const bool on = l.u < nd && (cof || coef != 0.0);  // of weight zero: adds nothing
+#pragma unroll 1
+    for (int i0 = 0; i0 < n; i0 += l.groups) {  // row i of A_u^-T: column i of A_u^-1
+      const int i = i0 + l.g;
+      double y[kSumN];
+      if (on && i < n) {
+        D.unit(i, y, n);
+#pragma unroll 1
+        for (int j = 0; j < n; ++j) {
+          const double c = y[j] * D.det;
+          if (cof) k.C(S.cof + s * S.cofs + (l.u * n + i) * n + j) = c;
+          y[j] = coef * c;
+        }
+      }
+      sum_columns<0>(l, D.cols, y, n, on && coef != 0.0, nd, i0, nmu, u0 == 0,
+                     [&](int i, int c) -> double& { return k.C(S.gx + (r0 + i) * nmu + c); });
+    }
+  }
+}
+
+// G of a spin whose rows are the start's, from its cofactors there.
+__device__ __noinline__ void drift_cof_warp(const qmc_wf_desc& d, const DriftShape& S,
+                                            const DriftWork& k, int s, int n, const double* oth,
+                                            int64_t os) {
+  const int r0 = s ? d.nup : 0, nmu = d.nmo_used, nd = d.ndet[s];
+  const SumLanes l = sum_lanes(nd, n, 0);
+  int cols[kSumN];
+  if (l.u < nd) det_columns(d, s, l.u, cols);
+  double coef = 0.0;
+  sum_configs(d, s, l.u, [&](int v, double& a, double&) { a = oth[v * os]; },
+              [&](double w, double a, double) { coef = fma(w, a, coef); });
+  const bool on = l.u < nd && coef != 0.0;
+#pragma unroll 1
+  for (int i0 = 0; i0 < n; i0 += l.groups) {
+    const int i = i0 + l.g;
+    double y[kSumN];
+#pragma unroll
+    for (int j = 0; j < kSumN; ++j)
+      y[j] = on && i < n && j < n ? coef * k.C(S.cof + s * S.cofs + (l.u * n + i) * n + j) : 0.0;
+    sum_columns<0>(l, cols, y, n, on, nd, i0, nmu, true,
+                   [&](int i, int c) -> double& { return k.C(S.gx + (r0 + i) * nmu + c); });
+  }
 }
 
 // Excitation mode: F(i, v) = d Sigma / d X of spin s at H(S.f + s nmax nv + i nv + v)
@@ -205,9 +360,7 @@ __device__ inline void drift_adjoint(const qmc_wf_desc& d, const DriftShape& S,
                                      int64_t os) {
   const int n = s ? d.ndown : d.nup, nv = d.max_orb[s] - n;
   if (nv <= 0) return;
-  const int nmax = d.nup > d.ndown ? d.nup : d.ndown;
-  const int f0 = S.f + s * (S.dvf - S.f) / 2;
-  (void)nmax;
+  const int f0 = S.f + s * S.fs;
   for (int i = 0; i < n * nv; ++i) k.H(f0 + i) = 0.0;
   for (int c = 0; c < d.ncfg; ++c) {
     const int* e = d.det_table[s] + 5 * __ldg(d.cfg_det[s] + c);
@@ -324,12 +477,35 @@ __global__ void __launch_bounds__(kGradThreads)
   auto nof = [&](int s) { return s ? d.ndown : d.nup; };
   auto r0of = [&](int s) { return s ? d.nup : 0; };
   auto nvof = [&](int s) { return ex ? 0 : d.max_orb[s] - nof(s); };
-  auto f0of = [&](int s) { return S.f + s * (S.dvf - S.f) / 2; };
+  auto f0of = [&](int s) { return S.f + s * S.fs; };
   auto dv0 = [&](int s) { return k.cp + (int64_t)(S.dv0 + (s ? d.ndet[0] : 0)) * k.cs; };
   // X of the start: the virtual columns beside the LU
   auto x0 = [&](int s) {
     return CView<double>{k.cp + ((int64_t)S.lx + r0of(s) * nmu + nof(s)) * k.cs,
                          (int64_t)nmu * k.cs, k.cs};
+  };
+  auto view = [&](int q) {  // of the block's walker q
+    DriftWork kq = k;
+    kq.hp += q - wl;
+    kq.cp += q - wl;
+    return kq;
+  };
+  // the start's spins that sum their determinants: f(view, spin)
+  auto start_sums = [&](const auto& f) {
+    sum_tasks(
+        2 * S.nwb,
+        [&](int ch) {
+          const int s = ch / S.nwb;
+          return nof(s) <= kSumN && view(ch - s * S.nwb).H(S.val + DV_START + s) != 0.0;
+        },
+        [&](int ch) {
+          const int s = ch / S.nwb;
+          f(view(ch - s * S.nwb), s);
+        });
+  };
+  auto electron = [&](const DriftWork& kq) { return (int)kq.H(S.val + DV_MOVED); };  // moved
+  auto dets = [&](const DriftWork& kq, int s) {  // the start's determinants of spin s
+    return kq.cp + (int64_t)(S.dv0 + (s ? d.ndet[0] : 0)) * kq.cs;
   };
   double* const pos = a.pos + ws * nc;
   // this thread's AO groups of the moved electron: an even share of the AOs
@@ -346,6 +522,7 @@ __global__ void __launch_bounds__(kGradThreads)
   if (on)
     for (int e = slot; e < ne; e += ns) drift_start_rows(d, t, S, k, e);
   __syncthreads();
+  bool start_sum = false;  // of this thread's walker and spin; then of any in the block
   if (slot < 2) {
     const int s = spin, n = nof(s);
     double det = 1.0;
@@ -364,10 +541,28 @@ __global__ void __launch_bounds__(kGradThreads)
       const MView<double> X{M.p + n * M.cs, M.rs, M.cs};
       if (nv > 0) lu_solve<double>(M, n, piv, X.c(), X, nv);
       excitation_values<double, double>(d, d.det_table[s], s, X.c(), nv > 0 ? nv : 1, dv0(s), k.cs);
+      start_sum = det == 0.0;
+      for (int u = 0; u < d.ndet[s]; ++u)
+        start_sum |= __double2hiint(fabs(dv0(s)[u * k.cs])) > __double2hiint(kGradRatio);
+      if (start_sum) {
+        det = 1.0;
+        if (n > kSumN) drift_explicit(d, S, k, s, -1, dv0(s), k.cs, nullptr, 0);
+      }
     }
     k.H(S.val + DV_DET + s) = det;
+    k.H(S.val + DV_START + s) = start_sum ? 1.0 : 0.0;
   }
-  __syncthreads();
+  start_sum = __syncthreads_or(start_sum);
+  if (start_sum) {
+    start_sums([&](const DriftWork& kq, int s) {
+      drift_sum_warp<false>(d, S, kq, s, nof(s), -1, dets(kq, s), kq.cs, nullptr, 0, false);
+    });
+    __syncthreads();
+    start_sums([&](const DriftWork& kq, int s) {
+      drift_sum_warp<true>(d, S, kq, s, nof(s), -1, nullptr, 0, dets(kq, 1 - s), kq.cs,
+                           drift_cofactors(d, s));
+    });
+  }
   // A^-1 by columns; F, or G in explicit mode
   if (!ex && on)
     for (int e = slot; e < ne; e += ns) {
@@ -391,9 +586,10 @@ __global__ void __launch_bounds__(kGradThreads)
       }
     }
   if (slot < 2) {
-    if (ex)
+    const bool sum = k.H(S.val + DV_START + spin) != 0.0;
+    if (ex || (sum && nof(spin) > kSumN))
       drift_explicit(d, S, k, spin, -1, dv0(spin), k.cs, dv0(1 - spin), k.cs);
-    else
+    else if (!sum)
       drift_adjoint(d, S, k, spin, x0(spin), dv0(1 - spin), k.cs);
     if (slot == 0) {
       double sigma = 0.0;
@@ -425,7 +621,7 @@ __global__ void __launch_bounds__(kGradThreads)
       const int s = e < d.nup ? 0 : 1, n = nof(s), nv = nvof(s), i = e - r0of(s);
       double g[3] = {0.0, 0.0, 0.0};
       const int mg = S.mg + 3 * e * nmu;
-      if (ex) {
+      if (ex || k.H(S.val + DV_START + s) != 0.0) {
         for (int j = 0; j < nmu; ++j)
           for (int q = 0; q < 3; ++q)
             g[q] = fma(k.C(S.gx + e * nmu + j), k.C(mg + q * nmu + j), g[q]);
@@ -556,21 +752,24 @@ __global__ void __launch_bounds__(kGradThreads)
         }
       __syncthreads();
       if (slot == 0) {
-        const double q = 1.0 / k.H(S.r + l);
-        for (int v = 0; v < nv; ++v) {
-          const double tq = k.H(S.t + v) * q;
-          k.H(S.t + v) = tq;
-          for (int j = 0; j < n; ++j)
-            k.H(S.xp + j * nv + v) = fma(k.C(S.inv + e * nmax + j), tq, x0(sm)(j, v));
+        bool sum = k.H(S.val + DV_START + sm) != 0.0;
+        if (!sum) {
+          const double q = 1.0 / k.H(S.r + l);
+          for (int v = 0; v < nv; ++v) {
+            const double tq = k.H(S.t + v) * q;
+            k.H(S.t + v) = tq;
+            for (int j = 0; j < n; ++j)
+              k.H(S.xp + j * nv + v) = fma(k.C(S.inv + e * nmax + j), tq, x0(sm)(j, v));
+          }
+          k.H(S.val + DV_Q) = q;
+          const CView<double> X{k.hp + (int64_t)S.xp * k.hs, (int64_t)nv * k.hs, k.hs};
+          excitation_values<double, double>(d, d.det_table[sm], sm, X, nv > 0 ? nv : 1,
+                                            k.hp + (int64_t)S.dvf * k.hs, k.hs);
+          for (int u = 0; u < d.ndet[sm]; ++u)
+            sum |= __double2hiint(fabs(k.H(S.dvf + u))) > __double2hiint(kGradRatio);
         }
-        k.H(S.val + DV_Q) = q;
-        const CView<double> X{k.hp + (int64_t)S.xp * k.hs, (int64_t)nv * k.hs, k.hs};
-        excitation_values<double, double>(d, d.det_table[sm], sm, X, nv > 0 ? nv : 1,
-                                          k.hp + (int64_t)S.dvf * k.hs, k.hs);
-        bool sum = false;
-        for (int u = 0; u < d.ndet[sm]; ++u)
-          sum |= __double2hiint(fabs(k.H(S.dvf + u))) > __double2hiint(kGradRatio);
-        k.H(S.val + DV_FLAG) = sum ? e + 1.0 : 0.0;
+        k.H(S.val + DV_FLAG) = sum ? 1.0 : 0.0;
+        k.H(S.val + DV_MOVED) = (double)e;
         warp_sum = sum && n <= kSumN;
         if (sum && !warp_sum)
           drift_explicit(d, S, k, sm, e, k.hp + (int64_t)S.dvf * k.hs, k.hs, dv0(1 - sm), k.cs);
@@ -579,15 +778,37 @@ __global__ void __launch_bounds__(kGradThreads)
       drift_explicit(d, S, k, sm, e, k.hp + (int64_t)S.dvf * k.hs, k.hs, dv0(1 - sm), k.cs);
     }
     if (__syncthreads_or(warp_sum)) {
-      for (int q = tid >> 5; q < S.nwb; q += blockDim.x >> 5) {
-        DriftWork kq = k;
-        kq.hp += q - wl;
-        kq.cp += q - wl;
-        const int eq = (int)kq.H(S.val + DV_FLAG) - 1, s = eq < d.nup ? 0 : 1;
-        if (eq >= 0 && nof(s) <= kSumN) drift_sum_warp(d, S, kq, s, nof(s), eq);
-      }
+      sum_tasks(
+          S.nwb,
+          [&](int q) {
+            const DriftWork kq = view(q);
+            return kq.H(S.val + DV_FLAG) != 0.0 && nof(electron(kq) < d.nup ? 0 : 1) <= kSumN;
+          },
+          [&](int q) {
+            const DriftWork kq = view(q);
+            const int eq = electron(kq), s = eq < d.nup ? 0 : 1;
+            drift_sum_warp<true>(d, S, kq, s, nof(s), eq, kq.hp + (int64_t)S.dvf * kq.hs, kq.hs,
+                                 dets(kq, 1 - s), kq.cs, false);
+          });
       __syncthreads();
     }
+    if (start_sum)  // the other spin's G, with the moved spin's determinants
+      sum_tasks(
+          S.nwb,
+          [&](int q) {
+            const DriftWork kq = view(q);
+            const int s = electron(kq) < d.nup ? 1 : 0;
+            return nof(s) <= kSumN && kq.H(S.val + DV_START + s) != 0.0;
+          },
+          [&](int q) {
+            const DriftWork kq = view(q);
+            const int s = electron(kq) < d.nup ? 1 : 0;
+            const double* const dvf = kq.hp + (int64_t)S.dvf * kq.hs;
+            if (drift_cofactors(d, s))
+              drift_cof_warp(d, S, kq, s, nof(s), dvf, kq.hs);
+            else
+              drift_sum_warp<true>(d, S, kq, s, nof(s), -1, nullptr, 0, dvf, kq.hs, false);
+          });
     const double* const dvf = k.hp + (int64_t)S.dvf * k.hs;
     if (slot < 2) {
       const CView<double> X{k.hp + (int64_t)S.xp * k.hs, (int64_t)nv * k.hs, k.hs};
@@ -596,8 +817,11 @@ __global__ void __launch_bounds__(kGradThreads)
         const int s = slot == 0 ? sm : 1 - sm;
         if (s == sm) {
           if (k.H(S.val + DV_FLAG) == 0.0) drift_adjoint(d, S, k, s, X, dv0(1 - s), k.cs);
-        } else
+        } else if (k.H(S.val + DV_START + s) == 0.0) {
           drift_adjoint(d, S, k, s, x0(s), dvf, k.hs);
+        } else if (nof(s) > kSumN) {
+          drift_explicit(d, S, k, s, -1, k.hp + (int64_t)S.part * k.hs, 0, dvf, k.hs);
+        }
       } else if (slot == 1) {
         // the moved spin's G from the determinants phase; the other's now
         drift_explicit(d, S, k, 1 - sm, -1, k.hp + (int64_t)S.part * k.hs, 0, dvf, k.hs);
@@ -616,7 +840,9 @@ __global__ void __launch_bounds__(kGradThreads)
     // thread's AO groups of the moved electron ----
     const double sigma = k.H(S.val + DV_SIGMA), is = 1.0 / sigma;
     if (on) {
-      const bool sum = ex || k.H(S.val + DV_FLAG) != 0.0;  // the moved spin's G is in gx
+      // whether the moved spin's G, and the other's, is in gx
+      const bool sum = ex || k.H(S.val + DV_FLAG) != 0.0;
+      const bool osum = ex || k.H(S.val + DV_START + 1 - sm) != 0.0;
       const double q0 = ex ? 0.0 : k.H(S.val + DV_Q);
       double a1 = 0.0, a2 = 0.0;
       const int eacc = (int)k.H(S.val + DV_EACC);
@@ -625,7 +851,7 @@ __global__ void __launch_bounds__(kGradThreads)
           const int s = i < d.nup ? 0 : 1, mg = S.mg + 3 * i * nmu, ns_ = nof(s), nvs = nvof(s);
           double g[3] = {0.0, 0.0, 0.0};
           const bool moved = s == sm;
-          if (ex || (sum && moved)) {
+          if (moved ? sum : osum) {
             for (int j = 0; j < nmu; ++j)
               for (int q = 0; q < 3; ++q)
                 g[q] = fma(k.C(S.gx + i * nmu + j), k.C(mg + q * nmu + j), g[q]);

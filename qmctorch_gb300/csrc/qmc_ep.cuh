@@ -1583,13 +1583,13 @@ __device__ inline void ep_sum_channels(const qmc_wf_desc& d, const EPPtrs& p, co
   const int64_t cs = nwb, rs = (int64_t)d.nmo_used * nwb;
   const double* const MO = reinterpret_cast<const double*>(p.smem + S.o_mo);
   const double* const BK = reinterpret_cast<const double*>(p.smem + S.o_bk);
-  for (int ch = tid >> 5; ch < 2 * nwb; ch += blockDim.x >> 5) {
-    const int s = ch / nwb, wl = ch - s * nwb;
-    if (!((flag[wl] >> s) & 1)) continue;
-    const int64_t at = (s ? d.nup : 0) * rs + wl;
-    ep_sum_warp(d, s, s ? d.ndown : d.nup, MO + at, BK + at, rs, cs, values(L.dv, s, wl),
-                values(L.ov, s, wl), dss);
-  }
+  sum_tasks(2 * nwb, [&](int ch) { return ((flag[ch % nwb] >> (ch / nwb)) & 1) != 0; },
+            [&](int ch) {
+              const int s = ch / nwb, wl = ch - s * nwb;
+              const int64_t at = (s ? d.nup : 0) * rs + wl;
+              ep_sum_warp(d, s, s ? d.ndown : d.nup, MO + at, BK + at, rs, cs,
+                          values(L.dv, s, wl), values(L.ov, s, wl), dss);
+            });
 }
 
 // Evaluate psi (and, with KIN, the kinetic energy and potentials) for the

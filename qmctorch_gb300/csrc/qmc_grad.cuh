@@ -290,55 +290,36 @@ __device__ __forceinline__ MView<double> grad_view(const GradWork& k, int off, i
   return MView<double>{k.p + ((int64_t)off + (int64_t)row0 * nmu) * k.ws, (int64_t)nmu * k.ws, k.ws};
 }
 
-// The coefficient of determinant u of spin s: sum_c c_c D(other spin's).
-template <typename D>
-__device__ __forceinline__ double sum_coef(const qmc_wf_desc& d, int s, int u, const D& other) {
-  double coef = 0.0;
-  for (int c = 0; c < d.ncfg; ++c)
-    if (__ldg(d.cfg_det[s] + c) == u)
-      coef = fma(__ldg(d.ci_weight + c), other(__ldg(d.cfg_det[1 - s] + c)), coef);
-  return coef;
-}
-
-// A warp: the determinants of spin s to dst(u), and with ADJ g(i, c) += coef_u det_u
-// A_u^-T over them (g zeroed here).
+// A warp: the determinants of spin s to dst(u), and with ADJ g(i, c) = the sum of coef_u
+// det_u A_u^-T over them, coef_u = sum_c c_c D(other spin's).
 template <int N, bool ADJ, typename Row, typename Dst, typename Other, typename G>
 __device__ __forceinline__ void sum_warp(const qmc_wf_desc& d, int s, const Row& row,
                                          const Dst& dst, const Other& other, const G& g) {
-  const int lane = threadIdx.x & 31, nd = d.ndet[s];
-  if (ADJ) {
-    for (int i = lane; i < N * d.nmo_used; i += 32) g(i / d.nmo_used, i % d.nmo_used) = 0.0;
-    __syncwarp();
-  }
+  const int nd = d.ndet[s];
   for (int u0 = 0; u0 < nd; u0 += 32) {
-    const int u = u0 + lane;
+    const SumLanes l = sum_lanes(nd, N, u0);
     DetRegs<N> D;
-    double scale = 0.0;
-    bool on = false;
-    if (u < nd) {
-      D.factor(d, s, u, row);
-      dst(u, D.det);
-      if (ADJ) {
-        const double coef = sum_coef(d, s, u, other);
-        on = coef != 0.0;
-        scale = coef * D.det;
-      }
+    if (l.u < nd) {
+      D.factor(d, s, l.u, row);
+      if (l.g == 0) dst(l.u, D.det);
     }
     if (!ADJ) continue;
-    const int m = nd - u0 < 32 ? nd - u0 : 32;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {  // row i of A_u^-T: column i of A_u^-1
+    double coef = 0.0;
+    sum_configs(d, s, l.u, [&](int v, double& a, double&) { a = other(v); },
+                [&](double w, double a, double) { coef = fma(w, a, coef); });
+    const bool on = l.u < nd && coef != 0.0;  // a determinant of weight zero adds nothing
+    const double scale = on ? coef * D.det : 0.0;
+#pragma unroll 1
+    for (int i0 = 0; i0 < N; i0 += l.groups) {  // row i of A_u^-T: column i of A_u^-1
       double y[N];
-      if (on) D.unit(i, y);
-      for (int q = 0; q < m; ++q) {
-        if (lane == q && on)
 #pragma unroll
-          for (int j = 0; j < N; ++j) {
-            double& v = g(i, D.cols[j]);
-            v = fma(scale, y[j], v);
-          }
-        __syncwarp();
+      for (int j = 0; j < N; ++j) y[j] = 0.0;
+      if (on) {
+        D.unit(i0 + l.g, y);
+#pragma unroll
+        for (int j = 0; j < N; ++j) y[j] *= scale;
       }
+      sum_columns<N>(l, D.cols, y, N, on, nd, i0, d.nmo_used, u0 == 0, g);
     }
   }
 }
@@ -406,8 +387,8 @@ __device__ __noinline__ inline void grad_sum_warp(const qmc_wf_desc& d, const Gr
 }
 
 // The block's (walker, spin) channels that sum over explicit determinants: chain(s) for
-// this thread's own of more than kSumN electrons, warp(k, wl, s, n) for the others, one
-// after the other. The flags are behind a barrier. k, wl, slot: this thread's.
+// this thread's own of more than kSumN electrons, warp(k, wl, s, n) for the others. The flags
+// are behind a barrier. k, wl, slot: this thread's.
 template <typename Chain, typename Warp>
 __device__ __forceinline__ void sum_channels(const qmc_wf_desc& d, const GradShape& S,
                                              const GradWork& k, int wl, int slot,
@@ -415,14 +396,22 @@ __device__ __forceinline__ void sum_channels(const qmc_wf_desc& d, const GradSha
   const int tid = threadIdx.x, nwb = S.nwb;
   if (tid < 2 * nwb && (slot ? d.ndown : d.nup) > kSumN && k.at(S.val + GV_G + slot) != 0.0)
     chain(slot);
-  for (int ch = tid >> 5; ch < 2 * nwb; ch += blockDim.x >> 5) {
-    const int s = ch / nwb, q = ch - s * nwb, n = s ? d.ndown : d.nup;
-    if (n == 0 || n > kSumN) continue;
+  auto view = [&](int q) {
     GradWork kq = k;
     kq.wl += q - wl;
     kq.p = kq.p0 + kq.wl;
-    if (kq.at(S.val + GV_G + s) != 0.0) warp(kq, q, s, n);
-  }
+    return kq;
+  };
+  sum_tasks(
+      2 * nwb,
+      [&](int ch) {
+        const int s = ch / nwb, n = s ? d.ndown : d.nup;
+        return n > 0 && n <= kSumN && view(ch - s * nwb).at(S.val + GV_G + s) != 0.0;
+      },
+      [&](int ch) {
+        const int s = ch / nwb, q = ch - s * nwb;
+        warp(view(q), q, s, s ? d.ndown : d.nup);
+      });
 }
 
 // Determinant phase, one thread per (walker, spin): excitation mode factors a
