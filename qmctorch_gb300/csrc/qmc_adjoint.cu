@@ -32,8 +32,14 @@
 //
 // FP64 pipe bound (2 lanes per clock and SM), so counted in FP64 instructions:
 // H2O cc-pVDZ single_double(4,4), about 29,000 per walker for E_L; 4000 walkers 4.3 -> 1.5 ms.
+// Compiled twice: with limbs and the C entry points, and with -DQMC_INST_FIXED=0 for the
+// instances without limbs.
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#ifndef QMC_INST_FIXED
+#define QMC_INST_FIXED 1
+#endif
 
 #include "qmc_grad.cuh"
 #include "qmc_host.cuh"
@@ -46,6 +52,9 @@ constexpr int kAdjBlocks = 608;  // most blocks (rows of partial sums): 4 per SM
 // QMC_MAX_COMP components, five rows each for E_L, two for psi) and at least some
 // of its exponentials.
 __host__ __device__ constexpr int adj_tile_rows(bool el) { return el ? 40 : 24; }
+__host__ __device__ constexpr int64_t adj_tile_doubles(bool el, int jc, int ts) {
+  return (int64_t)(adj_tile_rows(el) + (el ? 2 : 1) * jc) * ts;
+}
 static_assert(adj_tile_rows(true) > 5 * QMC_MAX_COMP && adj_tile_rows(false) > 2 * QMC_MAX_COMP,
               "an AO group's rows fit the tile with room for its exponentials");
 
@@ -72,13 +81,14 @@ struct AdjShape {
   // Jastrow terms [8] per electron (grad U, lap U + |grad U|^2, their w derivatives)
   int bk, fm, fk, ov, jt, r, total;
   int64_t cold;  // per-walker doubles of the scratch: V, Z and G_B of the explicit sums
-  int64_t o_tile, o_work, smem;
+  int64_t o_tile, o_work, smem;  // o_tile < 0: the tile is in the scratch
   int ts, rows, parts, nparam, grid;
 };
 
-static AdjShape adj_shape(const qmc_wf_desc& d, bool el, int nwb, int nslot, int jc, bool in_smem) {
+static AdjShape adj_shape(const qmc_wf_desc& d, bool el, int nwb, int nslot, int jc, bool in_smem,
+                          bool fixed = true, bool tile_smem = true) {
   AdjShape s;
-  s.g = grad_shape(d, nwb, nslot, jc, false);
+  s.g = grad_shape(d, nwb, nslot, jc, false, fixed);
   const int ne = d.nelec, nmu = d.nmo_used, nmax = d.nup > d.ndown ? d.nup : d.ndown;
   int o = s.g.total;
   auto take = [&](int n) {
@@ -99,8 +109,12 @@ static AdjShape adj_shape(const qmc_wf_desc& d, bool el, int nwb, int nslot, int
   s.parts = adj_parts(d);
   s.nparam = adj_params(d);
   s.grid = 0;
-  s.o_tile = s.g.smem;
-  s.smem = s.o_tile + (((int64_t)(s.rows + (el ? 2 : 1) * jc) * s.ts * 8 + 15) & ~int64_t(15));
+  s.o_tile = -1;
+  s.smem = s.g.smem;
+  if (tile_smem) {
+    s.o_tile = s.smem;
+    s.smem += (adj_tile_doubles(el, jc, s.ts) * 8 + 15) & ~int64_t(15);
+  }
   s.o_work = -1;
   if (in_smem) {
     s.o_work = s.smem;
@@ -109,11 +123,16 @@ static AdjShape adj_shape(const qmc_wf_desc& d, bool el, int nwb, int nslot, int
   return s;
 }
 
-// scratch: partial sums [grid * parts][nparam], then the cold arrays and, where
-// they do not fit shared memory, the work arrays [item][walker]
+// scratch: partial sums [grid * parts][nparam], the blocks' tiles (of the plan that has them
+// there: one walker, two threads), then the cold arrays and, where they do not fit shared
+// memory, the work arrays [item][walker]
+__host__ __device__ inline int64_t adj_scratch_tiles(bool el) {
+  return kAdjBlocks * adj_tile_doubles(el, 8, 3);
+}
 static int64_t adj_scratch_bytes(const qmc_wf_desc& d, bool el, int64_t nw) {
   const AdjShape s = adj_shape(d, el, 1, 2, 8, false);
-  return 8 * ((int64_t)kAdjBlocks * s.parts * s.nparam + (s.cold + s.total) * pad_walkers(nw));
+  return 8 * ((int64_t)kAdjBlocks * s.parts * s.nparam + adj_scratch_tiles(el) +
+              (s.cold + s.total) * pad_walkers(nw));
 }
 
 // Jastrow terms of electron e for the E_L adjoint: grad U, lap U + |grad U|^2 and
@@ -164,7 +183,7 @@ __device__ __forceinline__ MView<double> adj_cold(const AdjCold& c, int64_t off,
 }
 
 // D_u and n_u = D_u T_u of spin s from the explicit determinants.
-__device__ __noinline__ void adj_sum_values(const qmc_wf_desc& d, const AdjShape& A,
+__device__ __noinline__ inline void adj_sum_values(const qmc_wf_desc& d, const AdjShape& A,
                                             const GradWork& k, const AdjCold& cold, int s) {
   const GradShape& S = A.g;
   const int n = s ? d.ndown : d.nup, r0 = s ? d.nup : 0, nmu = d.nmo_used;
@@ -187,7 +206,7 @@ __device__ __noinline__ void adj_sum_values(const qmc_wf_desc& d, const AdjShape
 }
 
 // G_A (`lu`) and G_B (scratch) of spin s summed over the explicit determinants.
-__device__ __noinline__ void adj_sum_adjoints(const qmc_wf_desc& d, const AdjShape& A,
+__device__ __noinline__ inline void adj_sum_adjoints(const qmc_wf_desc& d, const AdjShape& A,
                                               const GradWork& k, const AdjCold& cold, int s,
                                               double is, double R) {
   const GradShape& S = A.g;
@@ -237,7 +256,7 @@ __device__ __noinline__ void adj_sum_adjoints(const qmc_wf_desc& d, const AdjSha
 }
 
 // The two above by a warp, a lane per determinant, for a spin of n <= kSumN electrons.
-__device__ __noinline__ void adj_sum_values_warp(const qmc_wf_desc& d, const AdjShape& A,
+__device__ __noinline__ inline void adj_sum_values_warp(const qmc_wf_desc& d, const AdjShape& A,
                                                  const GradWork& k, int s, int n_) {
   const GradShape& S = A.g;
   const int r0 = s ? d.nup : 0, nmu = d.nmo_used, o = s ? d.ndet[0] : 0;
@@ -249,7 +268,7 @@ __device__ __noinline__ void adj_sum_values_warp(const qmc_wf_desc& d, const Adj
              });
 }
 
-__device__ __noinline__ void adj_sum_adjoints_warp(const qmc_wf_desc& d, const AdjShape& A,
+__device__ __noinline__ inline void adj_sum_adjoints_warp(const qmc_wf_desc& d, const AdjShape& A,
                                                    const GradWork& k, const AdjCold& cold, int s,
                                                    int n_) {
   const GradShape& S = A.g;
@@ -506,7 +525,7 @@ struct AdjElectron {
 // block's electrons (thread t < ncols holds one, with zero G where it has none):
 // the AO groups go through the tile a few at a time. dg[3] (E_L) gets
 // -sum_a hb_a grad AO_a, the adjoint of grad U. Every thread of the block calls it.
-template <bool EL, int JC>
+template <bool EL, int JC, bool FIXED>
 __device__ inline void adj_ao_pass(const qmc_wf_desc& d, const GradTables& tb,
                                    const AdjShape& A, double* tile, int ncols,
                                    const AdjElectron<JC>& el, int j0, int nj,
@@ -520,7 +539,7 @@ __device__ inline void adj_ao_pass(const qmc_wf_desc& d, const GradTables& tb,
   constexpr int kG = EL ? 2 * JC : JC, kT = EL ? 2 : 1, kQ = EL ? 3 : 1;
   double* const gt = tile;
   double* const rt = tile + kG * ts;
-  FixG<JC> fa, fb;
+  RowG<JC, FIXED> fa, fb;
   if (on) {
 #pragma unroll
     for (int jj = 0; jj < JC; ++jj) {
@@ -595,7 +614,7 @@ __device__ inline void adj_ao_pass(const qmc_wf_desc& d, const GradTables& tb,
           }
           const double vs = t.vscale ? t.vscale[a] : 1.0;
           // weights of the AO and of its part through B
-          const int2* const wl = reinterpret_cast<const int2*>(tb.l.W) + (int64_t)a * t.ncol + j0;
+          const int2* const wl = reinterpret_cast<const int2*>(t.W) + (int64_t)a * t.ncol + j0;
           const double ha = fa.dot(wl), hb = EL ? fb.dot(wl) : 0.0;
           AOVal<double> o{};
           if (sto) {
@@ -778,22 +797,26 @@ __device__ inline void adj_ao_pass(const qmc_wf_desc& d, const GradTables& tb,
   }
 }
 
-template <bool EL, int JC>
+template <bool EL, int JC, bool FIXED>
 __global__ void __launch_bounds__(kAdjThreads, 1)
     adjoint_kernel(const __grid_constant__ qmc_wf_desc d, const double* __restrict__ pos,
                    int64_t nw, const double* __restrict__ gout, const int* __restrict__ w_entry,
                    double* __restrict__ scr, int64_t ss, const __grid_constant__ AdjShape A) {
   extern __shared__ __align__(16) unsigned char smem[];
   const GradShape& S = A.g;
-  const GradTables tb = grad_tables(d, S, smem);
+  const GradTables tb = grad_tables<FIXED>(d, S, smem);
   const Tables<double>& t = tb.t;
   const int tid = threadIdx.x, ne = d.nelec, nmu = d.nmo_used, nwb = S.nwb;
   const int ncols = nwb * S.nslot, nmax = d.nup > d.ndown ? d.nup : d.ndown;
   const int slot = tid / nwb, wl = tid - slot * nwb;
   const bool on = slot < S.nslot;
-  double* const tile = reinterpret_cast<double*>(smem + A.o_tile);
   double* const sums = scr + (int64_t)blockIdx.x * A.parts * A.nparam;
-  double* const cold0 = scr + (int64_t)kAdjBlocks * A.parts * A.nparam;
+  double* const tiles = scr + (int64_t)kAdjBlocks * A.parts * A.nparam;
+  double* const cold0 = tiles + adj_scratch_tiles(EL);
+  double* tile = reinterpret_cast<double*>(smem + A.o_tile);
+  if constexpr (!FIXED) {
+    if (A.o_tile < 0) tile = tiles + blockIdx.x * adj_tile_doubles(EL, JC, A.ts);
+  }
   for (int i = tid; i < A.parts * A.nparam; i += blockDim.x) sums[i] = 0.0;
   const int64_t ntile = (nw + nwb - 1) / nwb;
   for (int64_t tl = blockIdx.x; tl < ntile; tl += gridDim.x) {
@@ -819,10 +842,10 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
         for (int e = slot; e < ne; e += S.nslot) {
           adj_jastrow(d, S, k, A.jt, e);
           const int j = A.jt + 8 * e;
-          ep_fixed_rows<true, true>(tb.l, tb.ecol, nmu, k.at(S.pos + 3 * e), k.at(S.pos + 3 * e + 1),
-                                    k.at(S.pos + 3 * e + 2), k.at(j), k.at(j + 1), k.at(j + 2),
-                                    k.at(j + 3), tb.fix, S.nthreads, &k.at(S.mo + e * nmu),
-                                    &k.at(A.bk + e * nmu), k.ws, 0, t.ngroup);
+          ep_rows<FIXED, true, true>(t, tb.ecol, nmu, k.at(S.pos + 3 * e), k.at(S.pos + 3 * e + 1),
+                                     k.at(S.pos + 3 * e + 2), k.at(j), k.at(j + 1), k.at(j + 2),
+                                     k.at(j + 3), tb.fix, S.nthreads, &k.at(S.mo + e * nmu),
+                                     &k.at(A.bk + e * nmu), k.ws, 0, t.ngroup);
         }
       __syncthreads();
       bool sum = false;
@@ -850,9 +873,9 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
         for (int e = slot; e < ne; e += S.nslot) {
           // log J, and its derivatives with respect to the weights (in `mom`)
           grad_jastrow<true>(d, S, k, e);
-          ep_fixed_rows<false, true>(tb.l, tb.ecol, nmu, k.at(S.pos + 3 * e), k.at(S.pos + 3 * e + 1),
-                                     k.at(S.pos + 3 * e + 2), 0.0, 0.0, 0.0, 0.0, tb.fix, S.nthreads,
-                                     &k.at(S.mo + e * nmu), nullptr, k.ws, 0, t.ngroup);
+          ep_rows<FIXED, false, true>(t, tb.ecol, nmu, k.at(S.pos + 3 * e), k.at(S.pos + 3 * e + 1),
+                                      k.at(S.pos + 3 * e + 2), 0.0, 0.0, 0.0, 0.0, tb.fix, S.nthreads,
+                                      &k.at(S.mo + e * nmu), nullptr, k.ws, 0, t.ngroup);
         }
       __syncthreads();
       grad_determinant_phases(d, S, k, wl, slot);
@@ -921,7 +944,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
           el.gb[jj] = EL && has ? scale * el.gb[jj] : 0.0;
           if (EL && has && j0 + jj < nmu) dl = fma(-0.5 * el.gb[jj], k.at(S.mo + e * nmu + j0 + jj), dl);
         }
-        adj_ao_pass<EL, JC>(d, tb, A, tile, ncols, el, j0, nmu - j0 < JC ? nmu - j0 : JC, w_entry,
+        adj_ao_pass<EL, JC, FIXED>(d, tb, A, tile, ncols, el, j0, nmu - j0 < JC ? nmu - j0 : JC, w_entry,
                             sums, dg);
       }
       if (EL && has) {
@@ -971,7 +994,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
 // partial sums, then a fixed tree), added to its output: W (row stride ldw),
 // exponents, CI weights, Pade weights. One block per parameter.
 constexpr int kRedTPB = 128;
-__global__ void __launch_bounds__(kRedTPB) adj_reduce_kernel(
+static __global__ void __launch_bounds__(kRedTPB) adj_reduce_kernel(
     const double* __restrict__ sums, int nrow, int nparam, int nao, int nmu, int nweight,
     int nent, int ncfg, double* __restrict__ g_W, int ldw, double* __restrict__ g_exp,
     double* __restrict__ g_ci, double* __restrict__ g_jw, double* __restrict__ g_jwn) {
@@ -1004,15 +1027,15 @@ __global__ void __launch_bounds__(kRedTPB) adj_reduce_kernel(
 // Launch plan, by the rule of grad_plan; the blocks take their tiles in turn, so the
 // busiest SM's work is its resident blocks times their tiles.
 template <typename K>
-static AdjShape adj_plan(const qmc_wf_desc& d, bool el, int jc, K kernel, int64_t nw) {
+static AdjShape adj_plan(const qmc_wf_desc& d, bool el, int jc, K kernel, int64_t nw, bool fixed) {
   int dev = 0, nsm = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  AdjShape best = adj_shape(d, el, 1, 2, jc, true);
+  AdjShape best = adj_shape(d, el, 1, 2, jc, true, fixed);
   const PlanKey key = plan_key((const void*)kernel, dev, nw, d, best.smem);
   PlanChoice got;
   if (plan_find(key, &got)) {
-    best = adj_shape(d, el, got.nwb, got.nslot, jc, got.in_smem);
+    best = adj_shape(d, el, got.nwb, got.nslot, jc, got.in_smem, fixed, got.tile);
     best.grid = got.grid;
     return best;
   }
@@ -1023,7 +1046,7 @@ static AdjShape adj_plan(const qmc_wf_desc& d, bool el, int jc, K kernel, int64_
       for (int per = 1; per <= 8; ++per) {
         const int nslot = (d.nelec + per - 1) / per;
         if (per > 1 && nslot == (d.nelec + per - 2) / (per - 1)) continue;
-        AdjShape s = adj_shape(d, el, nwb, nslot, jc, in_smem == 1);
+        AdjShape s = adj_shape(d, el, nwb, nslot, jc, in_smem == 1, fixed);
         if (s.g.nthreads > kAdjThreads || s.smem > 227 * 1024) continue;
         if (prepare_smem(kernel, s.smem) != QMC_OK) continue;
         int occ = 0;
@@ -1047,7 +1070,15 @@ static AdjShape adj_plan(const qmc_wf_desc& d, bool el, int jc, K kernel, int64_
           best_cost = cost;
         }
       }
-  if (best.smem >= 0) plan_keep(key, {best.g.nwb, best.g.nslot, best.o_work >= 0, best.grid});
+  if (best.smem < 0 && !fixed) {  // the tables alone
+    AdjShape s = adj_shape(d, el, 1, 2, jc, false, fixed, false);
+    if (s.smem <= 227 * 1024 && prepare_smem(kernel, s.smem) == QMC_OK) {
+      s.grid = (int)(nw < nsm ? nw : nsm);
+      best = s;
+    }
+  }
+  if (best.smem >= 0)
+    plan_keep(key, {best.g.nwb, best.g.nslot, best.o_work >= 0, best.grid, best.o_tile >= 0});
   return best;
 }
 
@@ -1059,13 +1090,13 @@ struct AdjArgs {
   double *g_exp, *g_W, *g_jw, *g_ci, *scr;
 };
 
-template <bool EL, int JC>
-static int launch_adjoint(const qmc_wf_desc& d, const AdjArgs& a, cudaStream_t s) {
-  const AdjShape A = adj_plan(d, EL, JC, adjoint_kernel<EL, JC>, a.nw);
+template <bool EL, int JC, bool FIXED>
+int launch_adjoint(const qmc_wf_desc& d, const AdjArgs& a, cudaStream_t s) {
+  const AdjShape A = adj_plan(d, EL, JC, adjoint_kernel<EL, JC, FIXED>, a.nw, FIXED);
   if (A.smem < 0) return QMC_ERR_SHAPE;
-  const int st = prepare_smem(adjoint_kernel<EL, JC>, A.smem);
+  const int st = prepare_smem(adjoint_kernel<EL, JC, FIXED>, A.smem);
   if (st) return st;
-  adjoint_kernel<EL, JC><<<(unsigned)A.grid, A.g.nthreads, A.smem, s>>>(
+  adjoint_kernel<EL, JC, FIXED><<<(unsigned)A.grid, A.g.nthreads, A.smem, s>>>(
       d, a.pos, a.nw, a.gout, a.w_entry, a.scr, pad_walkers(a.nw), A);
   adj_reduce_kernel<<<(unsigned)A.nparam, kRedTPB, 0, s>>>(
       a.scr, A.grid * A.parts, A.nparam, d.nao, d.nmo_used, d.nweight, a.nentries, d.ncfg, a.g_W,
@@ -1073,6 +1104,16 @@ static int launch_adjoint(const qmc_wf_desc& d, const AdjArgs& a, cudaStream_t s
       d.use_jastrow_en ? a.g_jw + 1 : nullptr);
   return launch_status();
 }
+
+#if !QMC_INST_FIXED
+template int launch_adjoint<false, 8, false>(const qmc_wf_desc&, const AdjArgs&, cudaStream_t);
+template int launch_adjoint<true, 8, false>(const qmc_wf_desc&, const AdjArgs&, cudaStream_t);
+}  // namespace qmc
+#else
+extern template int launch_adjoint<false, 8, false>(const qmc_wf_desc&, const AdjArgs&,
+                                                    cudaStream_t);
+extern template int launch_adjoint<true, 8, false>(const qmc_wf_desc&, const AdjArgs&,
+                                                   cudaStream_t);
 
 // The checks and the dispatch of both entry points.
 template <bool EL>
@@ -1093,7 +1134,9 @@ static int run_adjoint(const qmc_wf_desc* d0, const double* pos, int64_t nw, con
   const AdjArgs a{pos, gout, nw, weight_entry, nentries, ldw, grad_exp, grad_W, grad_jastrow_w,
                   grad_ci, (double*)scratch};
   // wider columns would not leave registers for the AO pass
-  return launch_adjoint<EL, 8>(dd, a, (cudaStream_t)stream);
+  st = launch_adjoint<EL, 8, true>(dd, a, (cudaStream_t)stream);
+  if (st == QMC_ERR_SHAPE) st = launch_adjoint<EL, 8, false>(dd, a, (cudaStream_t)stream);
+  return st;
 }
 
 }  // namespace qmc
@@ -1130,3 +1173,4 @@ int qmc_wf_local_energy_adjoint(const qmc_wf_desc* d, const double* pos, int64_t
 }
 
 }  // extern "C"
+#endif  // QMC_INST_FIXED

@@ -47,7 +47,7 @@ namespace qmc {
 // electron moves.
 struct DriftShape {
   int nwb, nslot, nthreads, ncol;
-  int64_t o_wl, o_ecol, o_fix;  // W as limbs, its column exponents, the threads' AO limbs
+  int64_t o_ecol, o_fix;  // W's column exponents (< 0: W is not in limbs), the threads' AO limbs
   int64_t smem, o_hot;  // o_hot < 0: the hot arrays too are in the scratch
   // per walker, in doubles. Hot (shared memory): start positions, the two drifts
   // (accepted and proposed), Jastrow gradient, the moved electron's MO row, its
@@ -73,7 +73,10 @@ __host__ __device__ inline bool drift_cofactors(const qmc_wf_desc& d, int s) {
   return d.det_mode == QMC_DET_EXCITATION && n <= kSumN && d.ndet[s] <= 32;
 }
 
-static DriftShape drift_shape(const qmc_wf_desc& d, int nwb, int nslot, bool in_smem) {
+// fixed: W as limbs after the start rows, and slots for the AOs'; else W itself (the least
+// shared memory)
+static DriftShape drift_shape(const qmc_wf_desc& d, int nwb, int nslot, bool in_smem,
+                              bool fixed = true) {
   DriftShape s;
   s.nwb = nwb;
   s.nslot = nslot;
@@ -125,10 +128,14 @@ static DriftShape drift_shape(const qmc_wf_desc& d, int nwb, int nslot, bool in_
   }
   s.cof = take(2 * s.cofs);
   s.cold = o;
-  s.o_wl = (tables_smem_bytes<double>(d, s.ncol) + 15) & ~int64_t(15);
-  s.o_ecol = s.o_wl + (int64_t)d.nao * s.ncol * 8;
-  s.o_fix = s.o_ecol + align8((int64_t)s.ncol * 4);
-  s.smem = (s.o_fix + (int64_t)s.nthreads * kFixAOs * 8 + 15) & ~int64_t(15);
+  s.smem = (tables_smem_bytes<double>(d, s.ncol) + 15) & ~int64_t(15);
+  s.o_ecol = -1;
+  s.o_fix = s.smem;
+  if (fixed) {
+    s.o_ecol = s.smem;
+    s.o_fix = s.o_ecol + align8((int64_t)s.ncol * 4);
+    s.smem = (s.o_fix + (int64_t)s.nthreads * kFixAOs * 8 + 15) & ~int64_t(15);
+  }
   s.o_hot = -1;
   if (in_smem) {
     s.o_hot = s.smem;
@@ -439,22 +446,15 @@ __device__ inline void drift_start_rows(const qmc_wf_desc& d, const Tables<doubl
   for (int q = 0; q < 3; ++q) k.C(S.jg0 + 3 * e + q) = g[q];
 }
 
+template <bool FIXED>
 __global__ void __launch_bounds__(kGradThreads)
     drift_kernel(const __grid_constant__ qmc_wf_desc d, const __grid_constant__ qmc_drift_args a,
                  double* __restrict__ scr, int64_t ss, double sd,
                  const __grid_constant__ DriftShape S) {
   extern __shared__ __align__(16) unsigned char smem[];
   const Tables<double> t = load_tables<double>(d, d.nmo_used, S.ncol, smem);
-  Tables<double> tl = t;  // W as limbs
-  int* const ecol = reinterpret_cast<int*>(smem + S.o_ecol);
-  {
-    double* const wl = reinterpret_cast<double*>(smem + S.o_wl);
-    for (int i = threadIdx.x; i < d.nao * S.ncol; i += blockDim.x) wl[i] = t.W[i];
-    __syncthreads();
-    fix_table(wl, d.nao, S.ncol, ecol);
-    tl.W = wl;
-  }
-  int2* const fix = reinterpret_cast<int2*>(smem + S.o_fix) + threadIdx.x;
+  int* const ecol = FIXED ? reinterpret_cast<int*>(smem + S.o_ecol) : nullptr;
+  int2* const fix = FIXED ? reinterpret_cast<int2*>(smem + S.o_fix) + threadIdx.x : nullptr;
   const int tid = threadIdx.x, slot = tid / S.nwb, wl = tid - slot * S.nwb, ns = S.nslot;
   const int64_t nw = a.nwalkers, w = (int64_t)blockIdx.x * S.nwb + wl;
   const bool on = slot < ns, live = on && w < nw;
@@ -522,6 +522,7 @@ __global__ void __launch_bounds__(kGradThreads)
   if (on)
     for (int e = slot; e < ne; e += ns) drift_start_rows(d, t, S, k, e);
   __syncthreads();
+  if constexpr (FIXED) fix_table(const_cast<double*>(t.W), d.nao, S.ncol, ecol);
   bool start_sum = false;  // of this thread's walker and spin; then of any in the block
   if (slot < 2) {
     const int s = spin, n = nof(s);
@@ -695,8 +696,8 @@ __global__ void __launch_bounds__(kGradThreads)
     // electrons' pairs with it ----
     double du = 0.0, ge[3] = {0.0, 0.0, 0.0};
     if (on) {
-      ep_fixed_rows<false, false>(tl, ecol, nmu, pe[0], pe[1], pe[2], 0.0, 0.0, 0.0, 0.0, fix,
-                                  S.nthreads, &k.H(S.part + slot * nmu), nullptr, k.hs, glo, ghi);
+      ep_rows<FIXED, false, false>(t, ecol, nmu, pe[0], pe[1], pe[2], 0.0, 0.0, 0.0, 0.0, fix,
+                                   S.nthreads, &k.H(S.part + slot * nmu), nullptr, k.hs, glo, ghi);
       if (d.use_jastrow_en && slot == e % ns) {
         const EnTerms en = en_terms(d, pe[0], pe[1], pe[2]);
         du = en.u - k.C(S.jen + e);
@@ -918,10 +919,10 @@ __global__ void __launch_bounds__(kGradThreads)
             }
           }
         }
-        FixG<8> fg;
+        RowG<8, FIXED> fg;
         fg.set(G, ecol + j0);
         auto h = [&](int ao) {
-          return fg.dot(reinterpret_cast<const int2*>(tl.W) + (int64_t)ao * t.ncol + j0);
+          return fg.dot(reinterpret_cast<const int2*>(t.W) + (int64_t)ao * t.ncol + j0);
         };
         grad_ao_backward(t, pe[0], pe[1], pe[2], h, ga, glo, ghi);
       }
@@ -997,25 +998,27 @@ __global__ void __launch_bounds__(kGradThreads)
 
 // Launch plan, by the rule of grad_plan: the least warp work on the busiest SM
 // (a walker's work is shared evenly by its threads, up to one per electron).
+template <bool FIXED>
 static DriftShape drift_plan(const qmc_wf_desc& d, int64_t nw) {
+  const auto kernel = drift_kernel<FIXED>;
   int dev = 0, nsm = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  DriftShape best = drift_shape(d, 1, 2, true);
-  const PlanKey key = plan_key((const void*)drift_kernel, dev, nw, d, best.smem);
+  DriftShape best = drift_shape(d, 1, 2, true, FIXED);
+  const PlanKey key = plan_key((const void*)kernel, dev, nw, d, best.smem);
   PlanChoice got;
-  if (plan_find(key, &got)) return drift_shape(d, got.nwb, got.nslot, got.in_smem);
+  if (plan_find(key, &got)) return drift_shape(d, got.nwb, got.nslot, got.in_smem, FIXED);
   best.smem = -1;
   double best_cost = 0.0;
   const int most = d.nelec > 16 ? 16 : (d.nelec < 2 ? 2 : d.nelec);
   for (int in_smem = 1; in_smem >= 0 && best.smem < 0; --in_smem)
     for (int nwb = 32; nwb >= 4; nwb /= 2)
       for (int nslot = 2; nslot <= most; ++nslot) {
-        const DriftShape s = drift_shape(d, nwb, nslot, in_smem == 1);
+        const DriftShape s = drift_shape(d, nwb, nslot, in_smem == 1, FIXED);
         if (s.nthreads > kGradThreads || s.smem > 227 * 1024) continue;
-        if (prepare_smem(drift_kernel, s.smem) != QMC_OK) continue;
+        if (prepare_smem(kernel, s.smem) != QMC_OK) continue;
         int occ = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, drift_kernel, s.nthreads, s.smem) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, s.nthreads, s.smem) !=
                 cudaSuccess ||
             occ < 1) {
           cudaGetLastError();
@@ -1034,8 +1037,21 @@ static DriftShape drift_plan(const qmc_wf_desc& d, int64_t nw) {
           best_cost = cost;
         }
       }
-  if (best.smem >= 0) plan_keep(key, {best.nwb, best.nslot, best.o_hot >= 0, 0});
+  if (best.smem >= 0) plan_keep(key, {best.nwb, best.nslot, best.o_hot >= 0, 0, false});
   return best;
+}
+
+template <bool FIXED>
+static int launch_drift(const qmc_wf_desc& d, const qmc_drift_args& a, double* scr,
+                        cudaStream_t s) {
+  const DriftShape S = drift_plan<FIXED>(d, a.nwalkers);
+  if (S.smem < 0) return QMC_ERR_SHAPE;
+  const int st = prepare_smem(drift_kernel<FIXED>, S.smem);
+  if (st) return st;
+  const double sd = sqrt(sqrt(a.step_size));  // covariance sqrt(step) I
+  drift_kernel<FIXED><<<(unsigned)((a.nwalkers + S.nwb - 1) / S.nwb), S.nthreads, S.smem, s>>>(
+      d, a, scr, pad_walkers(a.nwalkers), sd, S);
+  return launch_status();
 }
 
 }  // namespace qmc
@@ -1068,13 +1084,10 @@ int qmc_drift_run(const qmc_wf_desc* d0, const qmc_drift_args* a, void* scratch,
   if (!a->pos || !scratch) return QMC_ERR_ARG;
   if (a->nsnap > 0 && !a->samples) return QMC_ERR_ARG;
   if (scratch_bytes < qmc_drift_scratch_bytes(d, a->nwalkers)) return QMC_ERR_SCRATCH;
-  const DriftShape S = drift_plan(*d, a->nwalkers);
-  if (S.smem < 0) return QMC_ERR_SHAPE;
-  if ((st = prepare_smem(drift_kernel, S.smem))) return st;
-  const double sd = sqrt(sqrt(a->step_size));  // covariance sqrt(step) I
-  drift_kernel<<<(unsigned)((a->nwalkers + S.nwb - 1) / S.nwb), S.nthreads, S.smem,
-                 (cudaStream_t)stream>>>(dd, *a, (double*)scratch, pad_walkers(a->nwalkers), sd, S);
-  return launch_status();
+  st = launch_drift<true>(dd, *a, (double*)scratch, (cudaStream_t)stream);
+  // without limbs where W and the AO slots do not fit (grad_plan)
+  if (st == QMC_ERR_SHAPE) st = launch_drift<false>(dd, *a, (double*)scratch, (cudaStream_t)stream);
+  return st;
 }
 
 }  // extern "C"

@@ -581,6 +581,18 @@ __device__ __noinline__ inline void ep_plain_rows(const Tables<double>& t, int n
   }
 }
 
+// The rows by limbs (FIXED) or by FP64 multiply-adds, for the kernels with an instance of each.
+template <bool FIXED, bool KIN, bool CUT>
+__device__ __forceinline__ void ep_rows(const Tables<double>& t, const int* ecol, int nmu, double x,
+                                        double y, double z, double gx, double gy, double gz,
+                                        double jl, int2* v, int vs, double* mo, double* bk,
+                                        int64_t rs, int gb, int ge) {
+  if constexpr (FIXED)
+    ep_fixed_rows<KIN, CUT>(t, ecol, nmu, x, y, z, gx, gy, gz, jl, v, vs, mo, bk, rs, gb, ge);
+  else
+    ep_plain_rows<KIN, CUT>(t, nmu, x, y, z, gx, gy, gz, jl, mo, bk, rs, gb, ge);
+}
+
 // Two FP32 multiply-adds in one instruction, each rounded as fmaf.
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t d;

@@ -160,4 +160,26 @@ struct FixG {
   }
 };
 
+// The same weights with W itself, by FP64 multiply-adds.
+template <int N>
+struct PlainG {
+  double g[N];
+  __device__ __forceinline__ void set(const double (&G)[N], const int*) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) g[j] = G[j];
+  }
+  __device__ __forceinline__ double dot(const int2* w) const {
+    double h = 0.0;
+#pragma unroll
+    for (int j = 0; j < N; j += 2) {
+      const double2 q = reinterpret_cast<const double2*>(w)[j >> 1];
+      h = fma(g[j], q.x, h);
+      h = fma(g[j + 1], q.y, h);
+    }
+    return h;
+  }
+};
+template <int N, bool FIXED>
+using RowG = typename std::conditional<FIXED, FixG<N>, PlainG<N>>::type;
+
 }  // namespace qmc

@@ -37,7 +37,7 @@ constexpr int kGradSlots = 2 * kFixElAOs > kFixAOs ? 2 * kFixElAOs : kFixAOs;  /
 struct GradShape {
   int nwb, nslot, nthreads, ncol;
   int64_t smem, o_work;  // o_work < 0: the work arrays are in the scratch
-  int64_t o_wl, o_ecol, o_fix;  // W as limbs, its column exponents, the threads' AO limbs
+  int64_t o_ecol, o_fix;  // W's column exponents (< 0: W is not in limbs), the threads' AO limbs
   // per-walker arrays, offsets in doubles
   int fs;  // stride of the spins' F
   int pos, mom, mo, lu, f, y, dv, jg, ju, val, piv, total;
@@ -53,7 +53,10 @@ enum { GV_SIGMA = 0, GV_INV = 1, GV_DD = 2, GV_DET = 3, GV_ACC = 5, GV_G = 6, GV
 // below 1e-11.
 constexpr double kGradRatio = 4096.0;
 
-inline GradShape grad_shape(const qmc_wf_desc& d, int nwb, int nslot, int jc, bool in_smem) {
+// fixed: W as limbs (in the tables' place) and slots for the AOs'; else W itself, the least
+// shared memory.
+inline GradShape grad_shape(const qmc_wf_desc& d, int nwb, int nslot, int jc, bool in_smem,
+                            bool fixed = true) {
   GradShape s;
   s.nwb = nwb;
   s.nslot = nslot;
@@ -84,10 +87,13 @@ inline GradShape grad_shape(const qmc_wf_desc& d, int nwb, int nslot, int jc, bo
   s.piv = take((ne + 1) / 2);
   s.total = o;
   s.smem = (tables_smem_bytes<double>(d, s.ncol) + 15) & ~int64_t(15);
-  s.o_wl = s.smem;
-  s.o_ecol = s.o_wl + (int64_t)d.nao * s.ncol * 8;
-  s.o_fix = s.o_ecol + align8((int64_t)s.ncol * 4);
-  s.smem = (s.o_fix + (int64_t)s.nthreads * kGradSlots * 8 + 15) & ~int64_t(15);
+  s.o_ecol = -1;
+  s.o_fix = s.smem;
+  if (fixed) {
+    s.o_ecol = s.smem;
+    s.o_fix = s.o_ecol + align8((int64_t)s.ncol * 4);
+    s.smem = (s.o_fix + (int64_t)s.nthreads * kGradSlots * 8 + 15) & ~int64_t(15);
+  }
   s.o_work = -1;
   if (in_smem) {
     s.o_work = s.smem;
@@ -156,25 +162,25 @@ __device__ inline void grad_jastrow(const qmc_wf_desc& d, const GradShape& S, co
   k.at(S.jg + 3 * e + 2) = gz;
 }
 
-// The block's tables, with a copy of W as limbs for the contractions.
+// The block's tables (FIXED: W as limbs).
 struct GradTables {
-  Tables<double> t, l;  // l: W as limbs
+  Tables<double> t;
   const int* ecol;
   int2* fix;  // this thread's AO limb slots, stride nthreads
 };
+template <bool FIXED>
 __device__ inline GradTables grad_tables(const qmc_wf_desc& d, const GradShape& S,
                                          unsigned char* smem) {
   GradTables g;
   g.t = load_tables<double>(d, d.nmo_used, S.ncol, smem);
-  g.l = g.t;
-  double* const wl = reinterpret_cast<double*>(smem + S.o_wl);
-  for (int i = threadIdx.x; i < d.nao * S.ncol; i += blockDim.x) wl[i] = g.t.W[i];
-  g.l.W = wl;
-  int* const ecol = reinterpret_cast<int*>(smem + S.o_ecol);
-  __syncthreads();
-  fix_table(wl, d.nao, S.ncol, ecol);
-  g.ecol = ecol;
-  g.fix = reinterpret_cast<int2*>(smem + S.o_fix) + threadIdx.x;
+  g.ecol = nullptr;
+  g.fix = nullptr;
+  if constexpr (FIXED) {
+    int* const ecol = reinterpret_cast<int*>(smem + S.o_ecol);
+    fix_table(const_cast<double*>(g.t.W), d.nao, S.ncol, ecol);
+    g.ecol = ecol;
+    g.fix = reinterpret_cast<int2*>(smem + S.o_fix) + threadIdx.x;
+  }
   return g;
 }
 
@@ -565,7 +571,7 @@ __device__ __forceinline__ void grad_g_row(const qmc_wf_desc& d, const GradShape
 
 // g = sum_j G_ej grad MO_j(r_e): the determinant part of electron e's
 // gradient times Sigma (relative to dd).
-template <int JC>
+template <int JC, bool FIXED>
 __device__ inline void grad_backward(const qmc_wf_desc& d, const GradTables& t,
                                      const GradShape& S, const GradWork& k, int e, double (&g)[3]) {
   const int s = e < d.nup ? 0 : 1, nmax = d.nup > d.ndown ? d.nup : d.ndown;
@@ -575,10 +581,10 @@ __device__ inline void grad_backward(const qmc_wf_desc& d, const GradTables& t,
   for (int j0 = 0; j0 < d.nmo_used; j0 += JC) {
     double G[JC];
     grad_g_row<JC>(d, S, k, e, j0, G);
-    FixG<JC> fg;
+    RowG<JC, FIXED> fg;
     fg.set(G, t.ecol + j0);
     auto h = [&](int a) {
-      return fg.dot(reinterpret_cast<const int2*>(t.l.W) + (int64_t)a * t.t.ncol + j0);
+      return fg.dot(reinterpret_cast<const int2*>(t.t.W) + (int64_t)a * t.t.ncol + j0);
     };
     grad_ao_backward(t.t, k.at(S.pos + 3 * e), k.at(S.pos + 3 * e + 1), k.at(S.pos + 3 * e + 2), h,
                      g, 0, t.t.ngroup);
@@ -616,15 +622,16 @@ struct GradBlock {
 // Forward, determinant and adjoint phases at the positions in S.pos, which a
 // barrier has made visible: afterwards every thread of the walker may call
 // grad_backward and read val, jg and ju. Every thread of the block calls it.
+template <bool FIXED>
 __device__ inline void grad_evaluate(const qmc_wf_desc& d, const GradTables& t,
                                      const GradShape& S, const GradBlock& b) {
   if (b.on)
     for (int e = b.slot; e < d.nelec; e += S.nslot) {
       grad_jastrow(d, S, b.k, e);
-      ep_fixed_rows<false, false>(t.l, t.ecol, d.nmo_used, b.k.at(S.pos + 3 * e),
-                                  b.k.at(S.pos + 3 * e + 1), b.k.at(S.pos + 3 * e + 2), 0.0, 0.0,
-                                  0.0, 0.0, t.fix, S.nthreads, &b.k.at(S.mo + e * d.nmo_used),
-                                  nullptr, b.k.ws, 0, t.t.ngroup);
+      ep_rows<FIXED, false, false>(t.t, t.ecol, d.nmo_used, b.k.at(S.pos + 3 * e),
+                                   b.k.at(S.pos + 3 * e + 1), b.k.at(S.pos + 3 * e + 2), 0.0, 0.0,
+                                   0.0, 0.0, t.fix, S.nthreads, &b.k.at(S.mo + e * d.nmo_used),
+                                   nullptr, b.k.ws, 0, t.t.ngroup);
     }
   __syncthreads();
   grad_determinant_phases(d, S, b.k, b.wl, b.slot);
@@ -644,6 +651,7 @@ struct PlanChoice {
   int nwb, nslot;
   bool in_smem;
   int grid;
+  bool tile;
 };
 inline PlanKey plan_key(const void* kernel, int dev, int64_t nw, const qmc_wf_desc& d,
                         int64_t smem) {
@@ -676,14 +684,17 @@ inline void plan_keep(const PlanKey& key, const PlanChoice& c) {
 // keep the pipe full and by the half-empty warps of the determinant phases;
 // ties go to the larger block. 8192 H2O walkers: 32 x 5 threads (2 blocks per
 // SM, one round) against 8 x 10 in two rounds, 4.75 -> 3.5 ms for the HMC kernel.
+// fixed: of the instance with limbs. Refused (smem < 0) where no block fits; the callers then
+// take the instance with eight columns (W's rows are padded to the instance's), and after
+// that the one without limbs, which needs no more than the tables.
 template <typename K>
-inline GradShape grad_plan(const qmc_wf_desc& d, int jc, K kernel, int64_t nw) {
+inline GradShape grad_plan(const qmc_wf_desc& d, int jc, K kernel, int64_t nw, bool fixed) {
   int dev = 0, nsm = 1;
   cudaGetDevice(&dev);
-  GradShape best = grad_shape(d, 1, 2, jc, true);
+  GradShape best = grad_shape(d, 1, 2, jc, true, fixed);
   const PlanKey key = plan_key((const void*)kernel, dev, nw, d, best.smem);
   PlanChoice got;
-  if (plan_find(key, &got)) return grad_shape(d, got.nwb, got.nslot, jc, got.in_smem);
+  if (plan_find(key, &got)) return grad_shape(d, got.nwb, got.nslot, jc, got.in_smem, fixed);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   best.smem = -1;
   double best_cost = 0.0;
@@ -692,7 +703,7 @@ inline GradShape grad_plan(const qmc_wf_desc& d, int jc, K kernel, int64_t nw) {
       for (int per = 1; per <= 8; ++per) {
         const int nslot = (d.nelec + per - 1) / per;
         if (per > 1 && nslot == (d.nelec + per - 2) / (per - 1)) continue;
-        const GradShape s = grad_shape(d, nwb, nslot, jc, in_smem == 1);
+        const GradShape s = grad_shape(d, nwb, nslot, jc, in_smem == 1, fixed);
         if (s.nthreads > kGradThreads || s.smem > 227 * 1024) continue;
         if (prepare_smem(kernel, s.smem) != QMC_OK) continue;
         int occ = 0;
@@ -716,7 +727,7 @@ inline GradShape grad_plan(const qmc_wf_desc& d, int jc, K kernel, int64_t nw) {
           best_cost = cost;
         }
       }
-  if (best.smem >= 0) plan_keep(key, {best.nwb, best.nslot, best.o_work >= 0, 0});
+  if (best.smem >= 0) plan_keep(key, {best.nwb, best.nslot, best.o_work >= 0, 0, false});
   return best;
 }
 

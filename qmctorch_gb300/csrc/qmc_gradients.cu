@@ -10,13 +10,13 @@
 
 namespace qmc {
 
-template <int JC>
+template <int JC, bool FIXED>
 __global__ void __launch_bounds__(kGradThreads)
     gradients_kernel(const __grid_constant__ qmc_wf_desc d, const double* __restrict__ pos,
                      int64_t nw, int pdf, double* __restrict__ out, double* __restrict__ scr,
                      int64_t ss, const __grid_constant__ GradShape S) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const GradTables t = grad_tables(d, S, smem);
+  const GradTables t = grad_tables<FIXED>(d, S, smem);
   const GradBlock b(S, smem, scr, ss, nw);
   const GradWork& k = b.k;
   const int ne = d.nelec;
@@ -25,7 +25,7 @@ __global__ void __launch_bounds__(kGradThreads)
     for (int e = b.slot; e < ne; e += S.nslot)
       for (int q = 0; q < 3; ++q) k.at(S.pos + 3 * e + q) = x[3 * e + q];
   __syncthreads();
-  grad_evaluate(d, t, S, b);
+  grad_evaluate<FIXED>(d, t, S, b);
   if (!b.live) return;
   double logj = 0.0;
   for (int e = 0; e < ne; ++e) logj += k.at(S.ju + e);
@@ -33,20 +33,20 @@ __global__ void __launch_bounds__(kGradThreads)
   const double scale = pdf ? 2.0 * J * J * (dd * sigma) * dd : J * dd;
   for (int e = b.slot; e < ne; e += S.nslot) {
     double g[3];
-    grad_backward<JC>(d, t, S, k, e, g);
+    grad_backward<JC, FIXED>(d, t, S, k, e, g);
     for (int q = 0; q < 3; ++q)
       out[b.w * 3 * ne + 3 * e + q] = scale * fma(sigma, k.at(S.jg + 3 * e + q), g[q]);
   }
 }
 
-template <int JC>
+template <int JC, bool FIXED = true>
 static int launch_gradients(const qmc_wf_desc& d, const double* pos, int64_t nw, int pdf,
                             double* out, double* scr, cudaStream_t s) {
-  const GradShape S = grad_plan(d, JC, gradients_kernel<JC>, nw);
+  const GradShape S = grad_plan(d, JC, gradients_kernel<JC, FIXED>, nw, FIXED);
   if (S.smem < 0) return QMC_ERR_SHAPE;
-  const int st = prepare_smem(gradients_kernel<JC>, S.smem);
+  const int st = prepare_smem(gradients_kernel<JC, FIXED>, S.smem);
   if (st) return st;
-  gradients_kernel<JC><<<(unsigned)((nw + S.nwb - 1) / S.nwb), S.nthreads, S.smem, s>>>(
+  gradients_kernel<JC, FIXED><<<(unsigned)((nw + S.nwb - 1) / S.nwb), S.nthreads, S.smem, s>>>(
       d, pos, nw, pdf, out, scr, pad_walkers(nw), S);
   return launch_status();
 }
@@ -76,9 +76,13 @@ int qmc_wf_gradients(const qmc_wf_desc* d0, const double* pos, int64_t nw, int32
   if (scratch_bytes < qmc_grad_scratch_bytes(d, nw)) return QMC_ERR_SCRATCH;
   cudaStream_t cs = (cudaStream_t)stream;
   double* scr = (double*)scratch;
-  if (d->nmo_used <= 8) return launch_gradients<8>(dd, pos, nw, pdf ? 1 : 0, grad, scr, cs);
-  if (d->nmo_used <= 16) return launch_gradients<16>(dd, pos, nw, pdf ? 1 : 0, grad, scr, cs);
-  return launch_gradients<24>(dd, pos, nw, pdf ? 1 : 0, grad, scr, cs);
+  const int p = pdf ? 1 : 0;
+  st = QMC_ERR_SHAPE;
+  if (d->nmo_used > 16) st = launch_gradients<24>(dd, pos, nw, p, grad, scr, cs);
+  else if (d->nmo_used > 8) st = launch_gradients<16>(dd, pos, nw, p, grad, scr, cs);
+  if (st == QMC_ERR_SHAPE) st = launch_gradients<8>(dd, pos, nw, p, grad, scr, cs);
+  if (st == QMC_ERR_SHAPE) st = launch_gradients<8, false>(dd, pos, nw, p, grad, scr, cs);
+  return st;
 }
 
 }  // extern "C"

@@ -1,9 +1,14 @@
 // Hamiltonian Monte Carlo on the device, FP64 (hamiltonian.py:75-201): all
 // trajectories of a call in one launch, blocks of walkers with a thread per
 // electron (qmc_grad.cuh). One translation unit per MO column chunk: compiled
-// with -DQMC_INST_JC=<8|16|24>; the instance 8 holds the C entry points.
+// with -DQMC_INST_JC=<8|16|24> and, for the instance without limbs, 8 and
+// -DQMC_INST_FIXED=0; the instance 8 with limbs holds the C entry points.
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#ifndef QMC_INST_FIXED
+#define QMC_INST_FIXED 1
+#endif
 
 #include "qmc_grad.cuh"
 #include "qmc_host.cuh"
@@ -22,13 +27,13 @@ namespace qmc {
 // p negated, and the end point rejected when exp(H_start - H_end) < u. The
 // trajectory's positions, momenta and forces live in the walker's work
 // arrays (xi, dri, drf); pos holds the chain's current positions.
-template <int JC>
+template <int JC, bool FIXED>
 __global__ void __launch_bounds__(kGradThreads) hmc_kernel(const __grid_constant__ qmc_wf_desc d,
                                                            const __grid_constant__ qmc_hmc_args a,
                                                            double* __restrict__ scr, int64_t ss,
                                                            const __grid_constant__ GradShape S) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const GradTables t = grad_tables(d, S, smem);
+  const GradTables t = grad_tables<FIXED>(d, S, smem);
   const GradBlock b(S, smem, scr, ss, a.nwalkers);
   const GradWork& k = b.k;
   const int ne = d.nelec, nc = 3 * ne, tid = threadIdx.x;
@@ -85,13 +90,13 @@ __global__ void __launch_bounds__(kGradThreads) hmc_kernel(const __grid_constant
     // then a full step of each, the last momentum step a half one again:
     // p -= f grad U with grad U = -2 grad log psi
     for (int l = 0; l <= a.traj_length; ++l) {
-      grad_evaluate(d, t, S, b);
+      grad_evaluate<FIXED>(d, t, S, b);
       if (l == 0 && tid < S.nwb) h0 = energy(psq0);
       const double f = (l == 0 || l == a.traj_length) ? heps : eps;
       if (b.on)
         for (int e = b.slot; e < ne; e += S.nslot) {
           double g[3];
-          grad_backward<JC>(d, t, S, k, e, g);
+          grad_backward<JC, FIXED>(d, t, S, k, e, g);
           const double is = k.at(S.val + GV_INV);
           for (int q = 0; q < 3; ++q) {
             const double gl = fma(g[q], is, k.at(S.jg + 3 * e + q));
@@ -138,25 +143,30 @@ __global__ void __launch_bounds__(kGradThreads) hmc_kernel(const __grid_constant
   if (tid < S.nwb && b.w < a.nwalkers && a.accepted) a.accepted[b.w] += nacc;
 }
 
-template <int JC>
+template <int JC, bool FIXED>
 int launch_hmc(const qmc_wf_desc& d, const qmc_hmc_args& a, double* scr, cudaStream_t s) {
-  const GradShape S = grad_plan(d, JC, hmc_kernel<JC>, a.nwalkers);
+  const GradShape S = grad_plan(d, JC, hmc_kernel<JC, FIXED>, a.nwalkers, FIXED);
   if (S.smem < 0) return QMC_ERR_SHAPE;
-  const int st = prepare_smem(hmc_kernel<JC>, S.smem);
+  const int st = prepare_smem(hmc_kernel<JC, FIXED>, S.smem);
   if (st) return st;
-  hmc_kernel<JC><<<(unsigned)((a.nwalkers + S.nwb - 1) / S.nwb), S.nthreads, S.smem, s>>>(
+  hmc_kernel<JC, FIXED><<<(unsigned)((a.nwalkers + S.nwb - 1) / S.nwb), S.nthreads, S.smem, s>>>(
       d, a, scr, pad_walkers(a.nwalkers), S);
   return launch_status();
 }
 
-template int launch_hmc<QMC_INST_JC>(const qmc_wf_desc&, const qmc_hmc_args&, double*,
-                                     cudaStream_t);
+template int launch_hmc<QMC_INST_JC, QMC_INST_FIXED != 0>(const qmc_wf_desc&, const qmc_hmc_args&,
+                                                          double*, cudaStream_t);
 }  // namespace qmc
 
-#if QMC_INST_JC == 8
+#if QMC_INST_JC == 8 && QMC_INST_FIXED
 namespace qmc {
-extern template int launch_hmc<16>(const qmc_wf_desc&, const qmc_hmc_args&, double*, cudaStream_t);
-extern template int launch_hmc<24>(const qmc_wf_desc&, const qmc_hmc_args&, double*, cudaStream_t);
+#define QMC_HMC_EXTERN(JC, FIXED)                                                      \
+  extern template int launch_hmc<JC, FIXED>(const qmc_wf_desc&, const qmc_hmc_args&, \
+                                            double*, cudaStream_t);
+QMC_HMC_EXTERN(16, true)
+QMC_HMC_EXTERN(24, true)
+QMC_HMC_EXTERN(8, false)
+#undef QMC_HMC_EXTERN
 }  // namespace qmc
 
 using namespace qmc;
@@ -184,9 +194,13 @@ int qmc_hmc_run(const qmc_wf_desc* d0, const qmc_hmc_args* a, void* scratch,
   if (a->nsnap > 0 && !a->samples) return QMC_ERR_ARG;
   if (scratch_bytes < qmc_hmc_scratch_bytes(d, a->nwalkers)) return QMC_ERR_SCRATCH;
   cudaStream_t cs = (cudaStream_t)stream;
-  if (d->nmo_used <= 8) return qmc::launch_hmc<8>(dd, *a, (double*)scratch, cs);
-  if (d->nmo_used <= 16) return qmc::launch_hmc<16>(dd, *a, (double*)scratch, cs);
-  return qmc::launch_hmc<24>(dd, *a, (double*)scratch, cs);
+  double* const scr = (double*)scratch;
+  st = QMC_ERR_SHAPE;
+  if (d->nmo_used > 16) st = qmc::launch_hmc<24, true>(dd, *a, scr, cs);
+  else if (d->nmo_used > 8) st = qmc::launch_hmc<16, true>(dd, *a, scr, cs);
+  if (st == QMC_ERR_SHAPE) st = qmc::launch_hmc<8, true>(dd, *a, scr, cs);
+  if (st == QMC_ERR_SHAPE) st = qmc::launch_hmc<8, false>(dd, *a, scr, cs);
+  return st;
 }
 
 }  // extern "C"
