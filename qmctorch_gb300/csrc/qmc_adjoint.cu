@@ -70,10 +70,11 @@ __host__ __device__ inline int adj_parts(const qmc_wf_desc& d) {
   return n >= 128 ? 1 : (n >= 64 ? 2 : (n >= 32 ? 4 : 8));
 }
 
-// The E_L adjoint's terms cancel by about the ratio's square: with a line at 4096 the
-// H2O gradients of 4000 walkers were within 5e-11 of the explicit sums' (2-norm), at
-// 256 within 7e-12 (eight sets of walkers; most within 2e-13).
-constexpr double kAdjRatio = 256.0;
+// The E_L adjoint's line, by the same rule: parameter gradients of 2000 H2O walkers (2-norm,
+// the largest of 25) differ from the explicit sums' by 3.2e-14 at 64 and below, which is
+// their rounding, by 1.5e-13 at 256 and by 9e-12 at 1024. A step of 4000 walkers takes 1.85 ms
+// at 32, 1.80 at 256.
+constexpr double kAdjRatio = 32.0;
 
 struct AdjShape {
   GradShape g;  // per-walker arrays of the psi adjoint and the block's layout
