@@ -1135,7 +1135,8 @@ static int run_adjoint(const qmc_wf_desc* d0, const double* pos, int64_t nw, con
   const AdjArgs a{pos, gout, nw, weight_entry, nentries, ldw, grad_exp, grad_W, grad_jastrow_w,
                   grad_ci, (double*)scratch};
   // wider columns would not leave registers for the AO pass
-  st = launch_adjoint<EL, 8, true>(dd, a, (cudaStream_t)stream);
+  st = QMC_ERR_SHAPE;
+  if (fix_applies(dd)) st = launch_adjoint<EL, 8, true>(dd, a, (cudaStream_t)stream);
   if (st == QMC_ERR_SHAPE) st = launch_adjoint<EL, 8, false>(dd, a, (cudaStream_t)stream);
   return st;
 }

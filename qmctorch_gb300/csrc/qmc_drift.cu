@@ -1084,8 +1084,9 @@ int qmc_drift_run(const qmc_wf_desc* d0, const qmc_drift_args* a, void* scratch,
   if (!a->pos || !scratch) return QMC_ERR_ARG;
   if (a->nsnap > 0 && !a->samples) return QMC_ERR_ARG;
   if (scratch_bytes < qmc_drift_scratch_bytes(d, a->nwalkers)) return QMC_ERR_SCRATCH;
-  st = launch_drift<true>(dd, *a, (double*)scratch, (cudaStream_t)stream);
-  // without limbs where W and the AO slots do not fit (grad_plan)
+  st = QMC_ERR_SHAPE;
+  if (fix_applies(dd)) st = launch_drift<true>(dd, *a, (double*)scratch, (cudaStream_t)stream);
+  // and without limbs where W and the AO slots do not fit (grad_plan)
   if (st == QMC_ERR_SHAPE) st = launch_drift<false>(dd, *a, (double*)scratch, (cudaStream_t)stream);
   return st;
 }

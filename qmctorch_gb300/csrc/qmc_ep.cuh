@@ -194,7 +194,7 @@ __host__ __device__ inline EPShape ep_shape(const qmc_wf_desc& d, int kind, int 
     s.o_lu = o;
     o += align8(2 * nmax * nmax * nwb * (int64_t)sizeof(R));
   }
-  const bool fixed = !kMixed<R> && level < 2;
+  const bool fixed = !kMixed<R> && level < 2 && fix_applies(d);
   s.o_fix = o;
   if (fixed || s.o_bd >= 0)
     o += align8((int64_t)s.nthreads * (kind == 1 ? (kMixed<R> ? 3 : 2) * kFixElAOs : kFixAOs) *
@@ -550,7 +550,8 @@ __device__ inline void ep_fixed_rows(const Tables<double>& t, const int* ecol, i
     for (int j = 0; j < nmu; ++j) bk[j * rs] = -0.5 * fma(jl, mo[j * rs], bk[j * rs]);
 }
 
-// The same rows by FP64 multiply-adds with W itself, a pass over the AOs per eight columns.
+// The same rows by FP64 multiply-adds with W itself, a pass over the AOs per eight columns
+// (molecules with one electron of a spin, and shapes that do not fit: ep_shape).
 template <bool KIN, bool CUT>
 __device__ __noinline__ inline void ep_plain_rows(const Tables<double>& t, int nmu, double x,
                                                   double y, double z, double gx, double gy,

@@ -18,6 +18,18 @@
 
 namespace qmc {
 
+// The error is relative to the largest AO value of a chunk times the column's largest entry,
+// not to the sum: where an electron lies close to a column's nodal plane, so that the AOs
+// that the column has are small against others, multiply-adds keep the entry's own relative
+// error and limbs do not (six bits in hand, then a bit lost for every halving). In a
+// determinant of several electrons the column's other entries carry the value; the
+// determinant of a single electron is that entry. So molecules with one electron of a spin
+// take the sums of multiply-adds (ep_plain_rows, PlainG); the AO -> MO layer, whose entries
+// are the result, forms such an entry again (mo_kernel).
+__host__ __device__ inline bool fix_applies(const qmc_wf_desc& d) {
+  return d.nup != 1 && d.ndown != 1;
+}
+
 constexpr int kFixAOs = 15;  // AOs per chunk: 15 x 2 x 2^58 < 2^63
 
 // x 2^(59 - e) (e: |x| < 2^e; biased exponent of the bound E = e + 1022) as limbs

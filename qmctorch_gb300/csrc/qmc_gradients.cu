@@ -78,6 +78,7 @@ int qmc_wf_gradients(const qmc_wf_desc* d0, const double* pos, int64_t nw, int32
   double* scr = (double*)scratch;
   const int p = pdf ? 1 : 0;
   st = QMC_ERR_SHAPE;
+  if (!fix_applies(dd)) return launch_gradients<8, false>(dd, pos, nw, p, grad, scr, cs);
   if (d->nmo_used > 16) st = launch_gradients<24>(dd, pos, nw, p, grad, scr, cs);
   else if (d->nmo_used > 8) st = launch_gradients<16>(dd, pos, nw, p, grad, scr, cs);
   if (st == QMC_ERR_SHAPE) st = launch_gradients<8>(dd, pos, nw, p, grad, scr, cs);

@@ -196,6 +196,7 @@ int qmc_hmc_run(const qmc_wf_desc* d0, const qmc_hmc_args* a, void* scratch,
   cudaStream_t cs = (cudaStream_t)stream;
   double* const scr = (double*)scratch;
   st = QMC_ERR_SHAPE;
+  if (!fix_applies(dd)) return qmc::launch_hmc<8, false>(dd, *a, scr, cs);
   if (d->nmo_used > 16) st = qmc::launch_hmc<24, true>(dd, *a, scr, cs);
   else if (d->nmo_used > 8) st = qmc::launch_hmc<16, true>(dd, *a, scr, cs);
   if (st == QMC_ERR_SHAPE) st = qmc::launch_hmc<8, true>(dd, *a, scr, cs);
