@@ -595,7 +595,7 @@ __device__ inline void adj_ao_pass(const qmc_wf_desc& d, const GradTables& tb,
         double* const er = rt + (row + ao_rows(gi)) * ts + tid;      // the first of them
         auto prim = [&](int p) {  // exponential of group primitive p
           const double ar = t.alpha[t.group_prim[gi] + p] * r2;
-          return above_cut(ar) ? 0.0 : rexp(-ar);
+          return above_zero(ar) ? 0.0 : rexp(-ar);
         };
         if (!own)
           for (int p = e0; p < e0 + en; ++p) er[(p - e0) * ts] = prim(p);
@@ -644,7 +644,7 @@ __device__ inline void adj_ao_pass(const qmc_wf_desc& d, const GradTables& tb,
                 double ev;
                 if (own) {
                   const double ar = al * r2;
-                  ev = above_cut(ar) ? 0.0 : rexp(-ar);
+                  ev = above_zero(ar) ? 0.0 : rexp(-ar);
                 } else {
                   ev = (p >= e0 && p < e0 + en) ? er[(p - e0) * ts] : prim(p);
                 }
@@ -701,7 +701,7 @@ __device__ inline void adj_ao_pass(const qmc_wf_desc& d, const GradTables& tb,
                 if (EL)
                   v -= hb * (0.5 * vs * sd.lap + el.gu[0] * sd.gx + el.gu[1] * sd.gy + el.gu[2] * sd.gz);
               } else {
-                const double z = al * r2, ev = above_cut(z) ? 0.0 : rexp(-z);
+                const double z = al * r2, ev = above_zero(z) ? 0.0 : rexp(-z);
                 // the value and Laplacian carry vs, the gradient does not
                 v = -vs * ha * P * r2;
                 if (EL) {
@@ -843,7 +843,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
         for (int e = slot; e < ne; e += S.nslot) {
           adj_jastrow(d, S, k, A.jt, e);
           const int j = A.jt + 8 * e;
-          ep_rows<FIXED, true, true>(t, tb.ecol, nmu, k.at(S.pos + 3 * e), k.at(S.pos + 3 * e + 1),
+          ep_rows<FIXED, true, false>(t, tb.ecol, nmu, k.at(S.pos + 3 * e), k.at(S.pos + 3 * e + 1),
                                      k.at(S.pos + 3 * e + 2), k.at(j), k.at(j + 1), k.at(j + 2),
                                      k.at(j + 3), tb.fix, S.nthreads, &k.at(S.mo + e * nmu),
                                      &k.at(A.bk + e * nmu), k.ws, 0, t.ngroup);
@@ -874,7 +874,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
         for (int e = slot; e < ne; e += S.nslot) {
           // log J, and its derivatives with respect to the weights (in `mom`)
           grad_jastrow<true>(d, S, k, e);
-          ep_rows<FIXED, false, true>(t, tb.ecol, nmu, k.at(S.pos + 3 * e), k.at(S.pos + 3 * e + 1),
+          ep_rows<FIXED, false, false>(t, tb.ecol, nmu, k.at(S.pos + 3 * e), k.at(S.pos + 3 * e + 1),
                                       k.at(S.pos + 3 * e + 2), 0.0, 0.0, 0.0, 0.0, tb.fix, S.nthreads,
                                       &k.at(S.mo + e * nmu), nullptr, k.ws, 0, t.ngroup);
         }
