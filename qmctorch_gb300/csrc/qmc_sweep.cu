@@ -500,26 +500,49 @@ __global__ void __launch_bounds__(32 * kSweepWarps<R>, 1)
 
 // Walkers per block: the fewest rounds of resident warps over the walkers that fall
 // to an SM, then the fewest walkers on the busiest SM, then the larger block (one
-// copy of the tables for more warps).
+// copy of the tables for more warps). What a block of each size would take of an SM is
+// asked once per device and shape (two sizes that the shared memory is linear in) and
+// kept: the 24 questions take some 20 us, as long as a small call's other host work.
 template <typename R, int JC>
 static int launch_sweep(const qmc_wf_desc* d, const qmc_metropolis_args* a, cudaStream_t st) {
+  struct Resident {
+    int dev;
+    int64_t base, per_warp;
+    int nsm, occ[kSweepWarps<R> + 1];  // 0: does not fit
+  };
+  static std::mutex mu;
+  static std::vector<Resident> cache;  // at most 64
   SweepShape best = sweep_shape<R>(*d, 1, JC);
-  int best_warps = 0, dev = 0, nsm = 1;
+  int best_warps = 0, dev = 0;
   int64_t best_rounds = 0, best_load = 0;
   cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  for (int nww = kSweepWarps<R>; nww >= 1; --nww) {
-    const SweepShape s = sweep_shape<R>(*d, nww, JC);
-    if (s.smem > 227 * 1024) continue;
-    if (prepare_smem(sweep_kernel<R, JC>, s.smem) != QMC_OK) continue;
-    int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sweep_kernel<R, JC>, s.nthreads, s.smem) !=
-            cudaSuccess ||
-        occ < 1) {
-      cudaGetLastError();
-      continue;
+  Resident r{dev, best.o_warp, best.warp_bytes, 0, {}};
+  {
+    std::lock_guard<std::mutex> g(mu);
+    for (const Resident& c : cache)
+      if (c.dev == r.dev && c.base == r.base && c.per_warp == r.per_warp) r = c;
+  }
+  if (r.nsm == 0) {
+    r.nsm = 1;
+    cudaDeviceGetAttribute(&r.nsm, cudaDevAttrMultiProcessorCount, dev);
+    for (int nww = kSweepWarps<R>; nww >= 1; --nww) {
+      const int64_t smem = r.base + nww * r.per_warp;
+      if (smem > 227 * 1024 || prepare_smem(sweep_kernel<R, JC>, smem) != QMC_OK) continue;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r.occ[nww], sweep_kernel<R, JC>, 32 * nww,
+                                                        smem) != cudaSuccess) {
+        cudaGetLastError();
+        r.occ[nww] = 0;
+      }
     }
-    const int64_t blocks = (a->nwalkers + nww - 1) / nww, on_sm = (blocks + nsm - 1) / nsm;
+    std::lock_guard<std::mutex> g(mu);
+    if (cache.size() >= 64) cache.clear();
+    cache.push_back(r);
+  }
+  for (int nww = kSweepWarps<R>; nww >= 1; --nww) {
+    const int occ = r.occ[nww];
+    if (occ < 1) continue;
+    const SweepShape s = sweep_shape<R>(*d, nww, JC);
+    const int64_t blocks = (a->nwalkers + nww - 1) / nww, on_sm = (blocks + r.nsm - 1) / r.nsm;
     const int64_t rounds = (on_sm + occ - 1) / occ, load = on_sm * nww;
     if (best_warps == 0 || rounds < best_rounds || (rounds == best_rounds && load < best_load)) {
       best_warps = occ * nww;
