@@ -265,7 +265,20 @@ template <typename R, bool DERIV, int NC, bool CUT = false>
 __device__ __forceinline__ void group_radial(const Tables<R>& t, int g, R r2, R (&G0)[NC],
                                              R (&G1)[NC], R (&G2)[NC]) {
   const int p0 = t.group_prim[g], np = t.group_prim[g + 1] - p0;
-  const int wb = t.ao_wofs[t.group_ao[g]];  // weights of component c at wb + c * np
+  // Weights of component c from ofs(c): the fused kernels take them to follow one another
+  // (an offset per component costs the FP32 ones registers that they do not have), the
+  // others read each one's.
+  constexpr bool OWN = !kMixed<R> && !CUT;
+  const int wb = t.ao_wofs[t.group_ao[g]];
+  int own[OWN ? NC : 1];
+  if constexpr (OWN) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) own[c] = t.ao_wofs[t.group_ao[g] + c];
+  }
+  auto ofs = [&](int c) {
+    if constexpr (OWN) return own[c];
+    else return wb + c * np;
+  };
 #pragma unroll
   for (int c = 0; c < NC; ++c) G0[c] = G1[c] = G2[c] = (R)0;
   if (!t.group_split[g]) {
@@ -276,7 +289,7 @@ __device__ __forceinline__ void group_radial(const Tables<R>& t, int g, R r2, R 
       const R e1 = al * e0, e2 = al * e1;
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
-        const R w = t.wd[wb + c * np + p];
+        const R w = t.wd[ofs(c) + p];
         G0[c] = fma(w, e0, G0[c]);
         if (DERIV) {
           G1[c] = fma(w, e1, G1[c]);
@@ -289,7 +302,7 @@ __device__ __forceinline__ void group_radial(const Tables<R>& t, int g, R r2, R 
     for (int p = 0; p < np; ++p) {
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
-        const int wi = wb + c * np + p;
+        const int wi = ofs(c) + p;
         const R al = t.walpha[wi], ar = al * r2;
         if (CUT ? above_cut(ar) : above_zero(ar)) continue;
         const R e0 = rexp(-ar);
