@@ -54,7 +54,8 @@ __device__ __forceinline__ double fix_value(int64_t hh, int64_t mid, int64_t ll,
   const int z = mh ? __clzll((long long)mh) : 64 + __clzll((long long)ml);
   const uint64_t top = (uint64_t)((m << z) >> 64);
   const int ex = 1022 + 127 - z + u - 118;  // exponent field less the implicit bit
-  if (ex < 0) return 0.0;                   // below FP64's normal range
+  if ((unsigned)ex >= 2046u)  // below FP64's normal range, or beyond it
+    return ex < 0 ? 0.0 : (neg ? -INFINITY : INFINITY);
   return __longlong_as_double(
       (long long)(((uint64_t)neg << 63) | (((uint64_t)ex << 52) + (top >> 11) + ((top >> 10) & 1))));
 }
