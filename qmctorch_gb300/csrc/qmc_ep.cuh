@@ -431,7 +431,8 @@ __device__ __forceinline__ void ao_group(const Tables<R>& t, int g, R dx, R dy, 
   switch (t.group_kind[g]) {
     case GK_S:
       if (nc == 1) group_s<R, DERIV, 1, F, CUT>(t, g, dx, dy, dz, r2, f);
-      else group_s<R, DERIV, 2, F, CUT>(t, g, dx, dy, dz, r2, f);
+      else if (!kMixed<R> || nc == 2) group_s<R, DERIV, 2, F, CUT>(t, g, dx, dy, dz, r2, f);
+      else group_generic<R, DERIV, QMC_MAX_COMP, F, CUT>(t, g, dx, dy, dz, r2, f);
       break;
     case GK_P: group_p<R, DERIV, F, CUT>(t, g, dx, dy, dz, r2, f); break;
     case GK_D: group_d<R, DERIV, F, CUT>(t, g, dx, dy, dz, r2, f); break;
