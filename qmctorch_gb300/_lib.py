@@ -28,11 +28,13 @@ SOURCES = ["qmc_wf_kernels.cu", "qmc_staged.cu", "qmc_metropolis.cu", "qmc_capi_
 # translation units compiled more than once, with defines: (source, object, flags)
 INSTANCES = [("qmc_metropolis_inst.cu", "qmc_metropolis_%s_%d" % (r, jc),
               ["-DQMC_INST_R=%s" % r, "-DQMC_INST_JC=%d" % jc])
-             for r, jc in (("float", 8), ("float", 16), ("float", 24), ("double", 8))]
+             for r, jc in (("float", 8), ("float", 16), ("float", 24), ("double", 8),
+                           ("double", 16))]
 INSTANCES += [("qmc_hmc_inst.cu", "qmc_hmc_%d" % jc, ["-DQMC_INST_JC=%d" % jc])
               for jc in (8, 16, 24)]
 INSTANCES += [("qmc_hmc_inst.cu", "qmc_hmc_plain", ["-DQMC_INST_JC=8", "-DQMC_INST_FIXED=0"]),
-              ("qmc_adjoint.cu", "qmc_adjoint_plain", ["-DQMC_INST_FIXED=0"])]
+              ("qmc_adjoint.cu", "qmc_adjoint_plain", ["-DQMC_INST_FIXED=0"]),
+              ("qmc_wf_kernels.cu", "qmc_wf_kernels_plain", ["-DQMC_INST_FIXED=0"])]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I" + INCLUDE]
 

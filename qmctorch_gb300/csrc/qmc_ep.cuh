@@ -133,11 +133,20 @@ struct EPShape {
   int64_t o_det;  // determinant-phase work arrays of the block's walkers, or -1: HBM scratch
 };
 
-// level 0: everything that helps; 1: el_diagonal's factors in the work arrays; 2: the least
-// shared memory, without the threads' AO slots (FP64: sums of FP64 multiply-adds; FP32 local
-// energy: columns in registers, a pass over the AOs per eight). The plan search takes the first level at
-// which a block of one walker fits.
-constexpr int kEPLevels = 3;
+// level 0: everything that helps; 1: el_diagonal's factors in the work arrays; 2 (FP32 local
+// energy): columns in registers, a pass over the AOs per eight, without the threads' AO slots. The
+// plan search takes the first level at which a block of one walker fits.
+template <typename R>
+constexpr int kEPLevels = kMixed<R> ? 3 : 2;
+
+// The column chunk JC of a kernel instance. FP32 kernels have one for 8, 16 and 24 columns.
+// FP64 kernels sum all columns in one pass over the AOs, by limbs (kFixJC), or eight in a pass
+// by multiply-adds with W itself (kPlainJC: molecules with one electron of a spin, and those whose
+// limbs' slots fit no block). Two instances, not a branch in one: with both loops in it the Metropolis
+// kernel was 7 to 19 % slower where many blocks share an SM (H2O, 32768 walkers x 25 steps,
+// 8.9 against 10.6 ms).
+constexpr int kFixJC = 8, kPlainJC = 16;
+
 template <typename R>
 __host__ __device__ inline EPShape ep_shape(const qmc_wf_desc& d, int kind, int nwb, int jc,
                                            int nslot, bool pos_global = false, int level = 0) {
@@ -149,7 +158,7 @@ __host__ __device__ inline EPShape ep_shape(const qmc_wf_desc& d, int kind, int 
   int nt = nwb * nslot;
   if (nt < 2 * nwb) nt = 2 * nwb;
   s.nthreads = ((nt + 31) / 32) * 32;
-  s.ncol = round_up(d.nmo_used, jc);
+  s.ncol = round_up(d.nmo_used, kMixed<R> ? jc : 8);
   const int64_t nc = 3 * (int64_t)d.nelec, nmu = d.nmo_used;
   const int64_t xps = 2 * (int64_t)sizeof(R);  // bytes of one split coordinate
   int64_t o = 0;
@@ -194,7 +203,7 @@ __host__ __device__ inline EPShape ep_shape(const qmc_wf_desc& d, int kind, int 
     s.o_lu = o;
     o += align8(2 * nmax * nmax * nwb * (int64_t)sizeof(R));
   }
-  const bool fixed = !kMixed<R> && level < 2 && fix_applies(d);
+  const bool fixed = !kMixed<R> && jc == kFixJC;
   s.o_fix = o;
   if (fixed || s.o_bd >= 0)
     o += align8((int64_t)s.nthreads * (kind == 1 ? (kMixed<R> ? 3 : 2) * kFixElAOs : kFixAOs) *
@@ -565,7 +574,7 @@ __device__ inline void ep_fixed_rows(const Tables<double>& t, const int* ecol, i
 }
 
 // The same rows by FP64 multiply-adds with W itself, a pass over the AOs per eight columns
-// (molecules with one electron of a spin, and shapes that do not fit: ep_shape).
+// (kPlainJC).
 template <bool KIN, bool CUT>
 __device__ __noinline__ inline void ep_plain_rows(const Tables<double>& t, int nmu, double x,
                                                   double y, double z, double gx, double gy,
@@ -790,13 +799,9 @@ __device__ inline void ep_electron(const qmc_wf_desc& d, const Tables<R>& t, con
   R* mrow = mo + (int64_t)e * nmu * cs;
   R* brow = KIN ? bk + (int64_t)e * nmu * cs : nullptr;
   if constexpr (!kMixed<R>) {
-    if (ecol)
-      ep_fixed_rows<KIN, true>(t, ecol, nmu, ex.h, ey.h, ez.h, gx, gy, gz, jl,
-                               reinterpret_cast<int2*>(fix), fix_stride, mrow,
-                               brow, cs, 0, t.ngroup);
-    else
-      ep_plain_rows<KIN, true>(t, nmu, ex.h, ey.h, ez.h, gx, gy, gz, jl, mrow, brow, cs, 0,
-                               t.ngroup);
+    ep_rows<JC == kFixJC, KIN, true>(t, ecol, nmu, ex.h, ey.h, ez.h, gx, gy, gz, jl,
+                                     reinterpret_cast<int2*>(fix), fix_stride, mrow, brow, cs, 0,
+                                     t.ngroup);
   } else if constexpr (KIN) {
     if (bd) {
       ep_float_rows(t, nmu, ex, ey, ez, gx, gy, gz, jl, fix, fix_stride, mrow, brow,
@@ -1508,8 +1513,7 @@ struct EPPtrs {
   EPShape S;
 };
 
-// The block's tables for the electron-parallel kernels (FP64: W as limbs, unless the
-// shape goes without).
+// The block's tables for the electron-parallel kernels (FP64: W as limbs, or itself).
 template <typename R>
 __device__ inline Tables<R> ep_tables(const qmc_wf_desc& d, const EPShape& S, unsigned char* smem) {
   const Tables<R> t = load_tables<R>(d, d.nmo_used, S.ncol, smem + S.o_tab);
@@ -1658,7 +1662,7 @@ __device__ inline void ep_eval(const qmc_wf_desc& d, const Tables<R>& t, const E
         ep_electron<R, JC, KIN>(d, t, pbuf + wl * S.pstride, e, MO + wl, BK + wl, nwb,
                                 &JR[e * nwb + wl], &VR[e * nwb + wl],
                                 reinterpret_cast<R*>(p.smem + S.o_fix) + tid, S.nthreads,
-                                S.o_ecol >= 0 ? reinterpret_cast<const int*>(p.smem + S.o_ecol) : nullptr,
+                                reinterpret_cast<const int*>(p.smem + S.o_ecol),
                                 S.o_bd >= 0 ? reinterpret_cast<R*>(p.smem + S.o_bd) + wl : nullptr);
     }
   }

@@ -142,7 +142,7 @@ static inline EPShape ep_plan(const qmc_wf_desc& d, int kind, int jc, K kernel, 
   // no plan gives one wave that way, a second pass moves them to the
   // (L2-resident) scratch, read once per step by the proposal and written on
   // acceptance, which frees a position row per walker of shared memory.
-  for (int level = 0; level < kEPLevels && best.smem < 0; ++level)
+  for (int level = 0; level < kEPLevels<R> && best.smem < 0; ++level)
   for (int pg = 0; pg < (kind == 2 ? 2 : 1) && !one_wave; ++pg)
   for (int nwb = nwb0; nwb >= 1 && !one_wave; nwb /= 2) {
     // the first block size that fits is kept, except by the persistent

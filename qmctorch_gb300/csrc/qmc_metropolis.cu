@@ -11,12 +11,13 @@ namespace qmc {
                                                unsigned char*, cudaStream_t);                  \
   extern template int launch_metropolis_batch<R, JC>(const qmc_wf_desc*,                       \
                                                      const qmc_metropolis_args*, void* const*, \
-                                                     int, cudaStream_t);                  \
+                                                     const int*, int, cudaStream_t);           \
   extern template int plan_metropolis<R, JC>(const qmc_wf_desc*, int64_t, int32_t*);
 QMC_MET_EXTERN(float, 8)
 QMC_MET_EXTERN(float, 16)
 QMC_MET_EXTERN(float, 24)
-QMC_MET_EXTERN(double, 8)
+QMC_MET_EXTERN(double, kFixJC)
+QMC_MET_EXTERN(double, kPlainJC)
 #undef QMC_MET_EXTERN
 }  // namespace qmc
 
@@ -27,8 +28,8 @@ using namespace qmc;
 int qmc_sweep_run(const qmc_wf_desc* d, const qmc_metropolis_args* a, void* stream);
 bool qmc_sweep_eligible(const qmc_wf_desc* d, const qmc_metropolis_args* a);
 
-// column-chunk class of the electron-parallel kernels (FP32: JC = 8, 16, 24; FP64 has one
-// instance, whose batches keep to the classes)
+// column-chunk class of the electron-parallel kernels (FP32: JC = 8, 16, 24; FP64 batches
+// keep to the classes as well)
 static inline int mo_chunk_class(int nmo_used) { return nmo_used <= 8 ? 0 : (nmo_used <= 16 ? 1 : 2); }
 
 extern "C" {
@@ -53,7 +54,11 @@ int qmc_metropolis_run(const qmc_wf_desc* d, const qmc_metropolis_args* a, void*
     if (d->nmo_used <= 16) return launch_metropolis<float, 16>(d, a, scr, s);
     return launch_metropolis<float, 24>(d, a, scr, s);
   }
-  return launch_metropolis<double, 8>(d, a, scr, s);
+  if (fix_applies(*d)) {
+    st = launch_metropolis<double, kFixJC>(d, a, scr, s);
+    if (st != QMC_ERR_SHAPE) return st;  // else: the limbs' slots fit no block
+  }
+  return launch_metropolis<double, kPlainJC>(d, a, scr, s);
 }
 
 int qmc_metropolis_plan(const qmc_wf_desc* d, int64_t nwalkers, int32_t* plan) {
@@ -65,7 +70,11 @@ int qmc_metropolis_plan(const qmc_wf_desc* d, int64_t nwalkers, int32_t* plan) {
     if (d->nmo_used <= 16) return plan_metropolis<float, 16>(d, nwalkers, plan);
     return plan_metropolis<float, 24>(d, nwalkers, plan);
   }
-  return plan_metropolis<double, 8>(d, nwalkers, plan);
+  if (fix_applies(*d)) {
+    st = plan_metropolis<double, kFixJC>(d, nwalkers, plan);
+    if (st != QMC_ERR_SHAPE) return st;
+  }
+  return plan_metropolis<double, kPlainJC>(d, nwalkers, plan);
 }
 
 int qmc_metropolis_run_batch(const qmc_wf_desc* descs, const qmc_metropolis_args* args,
@@ -93,11 +102,30 @@ int qmc_metropolis_run_batch(const qmc_wf_desc* descs, const qmc_metropolis_args
   cudaStream_t s = (cudaStream_t)stream;
   const qmc_wf_desc* d = descs;
   if (d->precision == QMC_PREC_MIXED) {
-    if (d->nmo_used <= 8) return launch_metropolis_batch<float, 8>(descs, args, scratch, njobs, s);
-    if (d->nmo_used <= 16) return launch_metropolis_batch<float, 16>(descs, args, scratch, njobs, s);
-    return launch_metropolis_batch<float, 24>(descs, args, scratch, njobs, s);
+    int all[QMC_MAX_BATCH];
+    for (int j = 0; j < njobs; ++j) all[j] = j;
+    if (d->nmo_used <= 8)
+      return launch_metropolis_batch<float, 8>(descs, args, scratch, all, njobs, s);
+    if (d->nmo_used <= 16)
+      return launch_metropolis_batch<float, 16>(descs, args, scratch, all, njobs, s);
+    return launch_metropolis_batch<float, 24>(descs, args, scratch, all, njobs, s);
   }
-  return launch_metropolis_batch<double, 8>(descs, args, scratch, njobs, s);
+  // the jobs of each of the two FP64 instances, in a launch of their own; all are known to fit
+  // before the first starts
+  int jobs[2][QMC_MAX_BATCH], n[2] = {0, 0};
+  for (int j = 0; j < njobs; ++j) {
+    const int64_t nw = args[j].nwalkers > 0 ? args[j].nwalkers : 1;
+    int32_t plan[5];
+    const bool fix =
+        fix_applies(descs[j]) && plan_metropolis<double, kFixJC>(descs + j, nw, plan) == QMC_OK;
+    if (!fix && plan_metropolis<double, kPlainJC>(descs + j, nw, plan) != QMC_OK)
+      return QMC_ERR_SHAPE;
+    jobs[fix ? 0 : 1][n[fix ? 0 : 1]++] = j;
+  }
+  int st = launch_metropolis_batch<double, kFixJC>(descs, args, scratch, jobs[0], n[0], s);
+  if (st == QMC_OK)
+    st = launch_metropolis_batch<double, kPlainJC>(descs, args, scratch, jobs[1], n[1], s);
+  return st;
 }
 
 }  // extern "C"

@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(EPBound<R>::kThreads)
   metropolis_block<R, JC>(d, a, scr, ss, S, blockIdx.x, smem);
 }
 
-// Several independent jobs in one launch: molecules of any size whose MO
+// Several independent jobs in one launch (jobs: their indices in the caller's arrays): molecules of any size whose MO
 // column count falls in this kernel's chunk class (JC), in one precision. The
 // job table travels in the kernel parameters with each job's own launch plan
 // (walkers per block, electron slots, shared-memory offsets: the plan the job
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(EPBound<R>::kThreads)
 
 template <typename R, int JC>
 int launch_metropolis_batch(const qmc_wf_desc* descs, const qmc_metropolis_args* args,
-                            void* const* scratch, int njobs, cudaStream_t s) {
+                            void* const* scratch, const int* jobs, int njobs, cudaStream_t s) {
   static MetBatch b;  // host staging of the parameter block (copied at launch)
   static std::mutex mu;
   std::lock_guard<std::mutex> g(mu);
@@ -225,18 +225,19 @@ int launch_metropolis_batch(const qmc_wf_desc* descs, const qmc_metropolis_args*
   b.njobs = njobs;
   b.block0[0] = 0;
   for (int j = 0; j < njobs; ++j) {
-    const int64_t nw = args[j].nwalkers > 0 ? args[j].nwalkers : 1;
-    const EPShape S = ep_plan<R>(descs[j], 2, JC, metropolis_batch_kernel<R, JC>, nw);
+    const int q = jobs[j];
+    const int64_t nw = args[q].nwalkers > 0 ? args[q].nwalkers : 1;
+    const EPShape S = ep_plan<R>(descs[q], 2, JC, metropolis_batch_kernel<R, JC>, nw);
     if (S.smem < 0 || S.smem > 227 * 1024 || S.nthreads > EPBound<R>::kThreads)
       return QMC_ERR_SHAPE;
     if (S.smem > smem) smem = S.smem;
     if (S.nthreads > nthreads) nthreads = S.nthreads;
-    b.job[j].d = descs[j];
-    b.job[j].a = args[j];
-    b.job[j].scr = (unsigned char*)scratch[j];
-    b.job[j].ss = pad_walkers(args[j].nwalkers);
+    b.job[j].d = descs[q];
+    b.job[j].a = args[q];
+    b.job[j].scr = (unsigned char*)scratch[q];
+    b.job[j].ss = pad_walkers(args[q].nwalkers);
     b.job[j].S = S;
-    b.block0[j + 1] = b.block0[j] + (args[j].nwalkers + S.nwb - 1) / S.nwb;
+    b.block0[j + 1] = b.block0[j] + (args[q].nwalkers + S.nwb - 1) / S.nwb;
   }
   if (b.block0[njobs] == 0) return QMC_OK;
   int st = prepare_smem(metropolis_batch_kernel<R, JC>, smem);

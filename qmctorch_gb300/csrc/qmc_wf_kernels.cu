@@ -1,8 +1,14 @@
-// Fused psi and local-energy kernels (plain FP64 and mixed methods).
+// Fused psi and local-energy kernels (plain FP64 and mixed methods). Compiled twice: with the C
+// entry points, and with -DQMC_INST_FIXED=0 for the FP64 instances that sum by multiply-adds
+// (kPlainJC).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <mutex>
+
+#ifndef QMC_INST_FIXED
+#define QMC_INST_FIXED 1
+#endif
 
 #include "qmc_ep.cuh"
 #include "qmc_host.cuh"
@@ -59,25 +65,14 @@ static int launch_prepare(K kernel, const EPShape& S, int kind) {
 }
 
 template <typename R, int JC>
-static int launch_psi(const qmc_wf_desc* d, const double* pos, int64_t nw, double* psi,
-                      unsigned char* scr, cudaStream_t s) {
+int launch_psi(const qmc_wf_desc* d, const double* pos, int64_t nw, double* psi,
+               unsigned char* scr, cudaStream_t s) {
   const EPShape S = ep_plan<R>(*d, 0, JC, ep_psi_kernel<R, JC>, nw);
   int st = launch_prepare<R>(ep_psi_kernel<R, JC>, S, 0);
   if (st) return st;
   const dim3 grid((unsigned)((nw + S.nwb - 1) / S.nwb));
   ep_psi_kernel<R, JC><<<grid, S.nthreads, S.smem, s>>>(*d, pos, nw, psi, scr, pad_walkers(nw), S);
   return launch_status();
-}
-
-template <typename R>
-static int dispatch_psi(const qmc_wf_desc* d, const double* pos, int64_t nw, double* psi,
-                        unsigned char* scr, cudaStream_t s) {
-  // the columns per pass over the AOs; FP64 sums all of them in one (ep_fixed_rows)
-  if constexpr (kMixed<R>) {
-    if (d->nmo_used > 16) return launch_psi<R, 24>(d, pos, nw, psi, scr, s);
-    if (d->nmo_used > 8) return launch_psi<R, 16>(d, pos, nw, psi, scr, s);
-  }
-  return launch_psi<R, 8>(d, pos, nw, psi, scr, s);
 }
 
 template <typename R, int JC, bool ELCOOP>
@@ -95,11 +90,49 @@ static int launch_eloc_k(const qmc_wf_desc* d, const double* pos, int64_t nw, do
 // Molecules with large excitation-mode channels (beyond the register path)
 // run the instance with the cooperative determinant phase.
 template <typename R, int JC>
-static int launch_eloc(const qmc_wf_desc* d, const double* pos, int64_t nw, double* eloc,
-                       double* kin, double* psi, unsigned char* scr, cudaStream_t s) {
+int launch_eloc(const qmc_wf_desc* d, const double* pos, int64_t nw, double* eloc, double* kin,
+                double* psi, unsigned char* scr, cudaStream_t s) {
   if (coop_el_applies<R>(*d, 4))
     return launch_eloc_k<R, JC, true>(d, pos, nw, eloc, kin, psi, scr, s);
   return launch_eloc_k<R, JC, false>(d, pos, nw, eloc, kin, psi, scr, s);
+}
+
+#if !QMC_INST_FIXED
+template int launch_psi<double, kPlainJC>(const qmc_wf_desc*, const double*, int64_t, double*,
+                                          unsigned char*, cudaStream_t);
+template int launch_eloc<double, kPlainJC>(const qmc_wf_desc*, const double*, int64_t, double*,
+                                           double*, double*, unsigned char*, cudaStream_t);
+}  // namespace qmc
+#else
+extern template int launch_psi<double, kPlainJC>(const qmc_wf_desc*, const double*, int64_t,
+                                                 double*, unsigned char*, cudaStream_t);
+extern template int launch_eloc<double, kPlainJC>(const qmc_wf_desc*, const double*, int64_t,
+                                                  double*, double*, double*, unsigned char*,
+                                                  cudaStream_t);
+
+static int dispatch_psi(const qmc_wf_desc* d, const double* pos, int64_t nw, double* psi,
+                        unsigned char* scr, cudaStream_t s) {
+  if (d->precision == QMC_PREC_MIXED) {  // the columns per pass over the AOs
+    if (d->nmo_used > 16) return launch_psi<float, 24>(d, pos, nw, psi, scr, s);
+    if (d->nmo_used > 8) return launch_psi<float, 16>(d, pos, nw, psi, scr, s);
+    return launch_psi<float, 8>(d, pos, nw, psi, scr, s);
+  }
+  if (fix_applies(*d)) {
+    const int st = launch_psi<double, kFixJC>(d, pos, nw, psi, scr, s);
+    if (st != QMC_ERR_SHAPE) return st;  // else: the limbs' slots fit no block
+  }
+  return launch_psi<double, kPlainJC>(d, pos, nw, psi, scr, s);
+}
+
+static int dispatch_eloc(const qmc_wf_desc* d, const double* pos, int64_t nw, double* eloc,
+                         double* kin, double* psi, unsigned char* scr, cudaStream_t s) {
+  if (d->precision == QMC_PREC_MIXED)
+    return launch_eloc<float, 8>(d, pos, nw, eloc, kin, psi, scr, s);
+  if (fix_applies(*d)) {
+    const int st = launch_eloc<double, kFixJC>(d, pos, nw, eloc, kin, psi, scr, s);
+    if (st != QMC_ERR_SHAPE) return st;
+  }
+  return launch_eloc<double, kPlainJC>(d, pos, nw, eloc, kin, psi, scr, s);
 }
 
 }  // namespace qmc
@@ -117,8 +150,7 @@ int qmc_wf_psi(const qmc_wf_desc* d, const double* pos, int64_t nw, double* psi,
   if (scratch_bytes < qmc_scratch_bytes(d, nw, 0)) return QMC_ERR_SCRATCH;
   unsigned char* scr = (unsigned char*)scratch;
   cudaStream_t s = (cudaStream_t)stream;
-  if (d->precision == QMC_PREC_MIXED) return dispatch_psi<float>(d, pos, nw, psi, scr, s);
-  return dispatch_psi<double>(d, pos, nw, psi, scr, s);
+  return dispatch_psi(d, pos, nw, psi, scr, s);
 }
 
 int qmc_wf_local_energy(const qmc_wf_desc* d, const double* pos, int64_t nw, double* eloc,
@@ -131,9 +163,7 @@ int qmc_wf_local_energy(const qmc_wf_desc* d, const double* pos, int64_t nw, dou
   if (scratch_bytes < qmc_scratch_bytes(d, nw, 1)) return QMC_ERR_SCRATCH;
   unsigned char* scr = (unsigned char*)scratch;
   cudaStream_t s = (cudaStream_t)stream;
-  if (d->precision == QMC_PREC_MIXED)
-    return launch_eloc<float, 8>(d, pos, nw, eloc, kinetic, psi, scr, s);
-  return launch_eloc<double, 8>(d, pos, nw, eloc, kinetic, psi, scr, s);
+  return dispatch_eloc(d, pos, nw, eloc, kinetic, psi, scr, s);
 }
 
 }  // extern "C"
@@ -187,3 +217,4 @@ extern "C" int qmc_wf_psi_static(const qmc_wf_desc* d, const double* pos, int64_
   if ((st = static_scratch_address(&scr))) return st;
   return qmc_wf_psi(d, pos, nw, psi, scr, need, stream);
 }
+#endif  // QMC_INST_FIXED
