@@ -72,8 +72,8 @@ __host__ __device__ inline int adj_parts(const qmc_wf_desc& d) {
 
 // The E_L adjoint's line, by the same rule: parameter gradients of 2000 H2O walkers (2-norm,
 // the largest of 25) differ from the explicit sums' by 3.2e-14 at 64 and below, which is
-// their rounding, by 1.5e-13 at 256 and by 9e-12 at 1024. A step of 4000 walkers takes 1.85 ms
-// at 32, 1.80 at 256.
+// their rounding, by 1.5e-13 at 256 and by 9e-12 at 1024. A step of 4000 walkers takes the
+// same at 32 and at 256, 1.82 ms.
 constexpr double kAdjRatio = 32.0;
 
 struct AdjShape {

@@ -212,8 +212,8 @@ __device__ __noinline__ void drift_explicit(const qmc_wf_desc& d, const DriftSha
 // A lane's determinant for the sums of a few walkers' spins (start_sums and below). Rolled,
 // in local memory, where sum_warp's is unrolled in registers: a walker in some hundred
 // sums, so what counts here is what the code costs the others (registers around the call,
-// instruction cache: H2O without any sum 5.05 -> 4.71 ms for 50 steps), and the time of one sum is the
-// same (it waits for the FP64 pipe, which the block's other warps and the SM's other block hold).
+// instruction cache: H2O, 8192 walkers x 50 steps without any sum, 5.05 -> 4.71 ms), and the time of one
+// sum is the same (it waits for the FP64 pipe, which the block's other warps and the SM's other block hold).
 struct DetSum {
   double a[kSumN * kSumN], det;    // factors, 1 / U_kk on the diagonal
   int perm[kSumN], cols[kSumN];    // the row of A that row k of the factors came from

@@ -108,8 +108,8 @@ constexpr int kFixElAOs = 8;
 // FP32 local energy: up to this many columns are summed in registers, in one pass over
 // the AOs; more go through the threads' slots in shared memory (ep_float_rows), where
 // the registers would take a pass per eight. H2O (7 columns) through the slots: 1.09e8
-// E_L/s, in registers 1.55e8; C6H6 (21 columns) in registers 4.57 ms, through the
-// slots 2.83.
+// E_L/s, in registers 1.55e8; 16384 walkers of H18 (9 columns) in registers, two passes, 441 us,
+// through the slots 386, H32 (16) 1507 and 1205; C6H6 (21) 4.57 and 2.83 ms.
 constexpr int kFloatRegCols = 8;
 static_assert(kFixElAOs >= QMC_MAX_COMP && kFixElAOs <= kFixAOs, "a chunk holds an AO group");
 

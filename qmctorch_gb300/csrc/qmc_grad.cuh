@@ -52,8 +52,9 @@ enum { GV_SIGMA = 0, GV_INV = 1, GV_DD = 2, GV_DET = 3, GV_ACC = 5, GV_G = 6, GV
 // where that stays within the rounding that the explicit sums have as well. Position
 // gradients of 10,000 H2O walkers, difference from the explicit sums (their own error: 99.9 %
 // below 9e-15, largest 1.4e-14): at 32, where one walker in 22 has such a spin, 99.9 % below
-// 4.7e-15 and largest 1.2e-14; at 64 8.4e-15 and 3.7e-14; at 4096 7e-13 and 1e-11. HMC, 8192
-// walkers: 4.41 ms at 32, 4.09 at 4096.
+// 4.7e-15 and largest 1.2e-14; at 64 8.4e-15 and 3.7e-14; at 4096 7e-13 and 1e-11. H2O,
+// 8192 walkers: two HMC trajectories take 4.22 ms at 32, 4.05 at 4096, 50 drift steps 8.21, 5.73
+// and without any sum 4.78.
 constexpr double kGradRatio = 32.0;
 
 // fixed: W as limbs (in the tables' place) and slots for the AOs'; else W itself, the least
